@@ -22,127 +22,214 @@
 // run to run.  Non-finite inputs give all-NaN outputs per member, as the
 // reference's lax.cond guards do.
 #include <cmath>
+#include <cooperative_groups.h>
 #include "swp_internal.h"
 
 namespace swp {
 namespace {
 
-constexpr int EM_THREADS = 256;
+namespace cg = cooperative_groups;
 
-// FP64 block sum of one value per thread (fixed order: warp shuffles, then
-// warp 0 over the 8 warp slots); every thread gets the total.
-__device__ double block_sum(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();  // red may still be read from the previous call
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  if (warp == 0) {
-    double s = lane < EM_THREADS / 32 ? red[lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) red[EM_THREADS / 32] = s;
-  }
-  __syncthreads();
-  return red[EM_THREADS / 32];
+constexpr int EM_THREADS = 256;
+constexpr int EM_WARPS = EM_THREADS / 32;
+// The map and the simple phase curve run one cluster of EM_CL CTAs per member,
+// whatever the ensemble's size: a member's FP64 work (two divisions, expm1 and
+// a reciprocal per pixel; GB300 retires 1.7 FP64 instructions per cycle and SM)
+// then spreads over 8 SMs, and its sums run in one fixed order (lanes, warps,
+// ranks), so that ensembles equal single-member calls bit for bit.
+constexpr int EM_CL = 8;
+
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
-__device__ bool block_all(bool v) { return __syncthreads_and(v ? 1 : 0) != 0; }
+
+// Sums of two values and the conjunction of a flag over the cluster's threads.
+// Warp sums go to this CTA's slots; each warp slot of each rank is then added
+// in rank and warp order by every thread.  `slot` is 3 * EM_WARPS doubles of
+// shared memory per call (a slot is not reused: no barrier after the reads).
+struct ClusterSum {
+  double a, b;
+  bool all;
+};
+__device__ ClusterSum cluster_sum(double a, double b, bool ok, double* slot) {
+  cg::cluster_group cl = cg::this_cluster();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  a = warp_sum(a);
+  b = warp_sum(b);
+  const bool wok = __all_sync(0xffffffffu, ok) != 0;
+  if (lane == 0) {
+    slot[warp] = a;
+    slot[EM_WARPS + warp] = b;
+    slot[2 * EM_WARPS + warp] = wok ? 0.0 : 1.0;
+  }
+  cl.sync();
+  // lane l reads warp slots l and l + 32 of the 64 (8 ranks x 8 warps)
+  double va = 0.0, vb = 0.0, bad = 0.0;
+#pragma unroll
+  for (int h = 0; h < EM_CL * EM_WARPS / 32; ++h) {
+    const int s = lane + 32 * h;
+    const double* r = cl.map_shared_rank(slot, s / EM_WARPS);
+    va += r[s % EM_WARPS];
+    vb += r[EM_WARPS + s % EM_WARPS];
+    bad += r[2 * EM_WARPS + s % EM_WARPS];
+  }
+  ClusterSum t;
+  t.a = warp_sum(va);
+  t.b = warp_sum(vb);
+  t.all = __all_sync(0xffffffffu, bad == 0.0) != 0;
+  return t;
+}
+
+constexpr int EXP_N = 64;  // steps of 2^(j / 64) in the table of planck_rel
 
 struct EmCfg {
   int temp_mode, model, nbands, input;  // input: 0 = Phi, 1 = T, 2 = intensity
   double R_d, T_ref, phi_to_T_scale, Tmin, x_clip;
-  double wl[SWP_EMISSION_MAX_BANDS], bw[SWP_EMISSION_MAX_BANDS];
+  // Planck bands: x = pl[k] / max(p0 + v, pmin), the argument h c / (lambda kB T)
+  // with the scale of T folded into pl, p0 and pmin (p0 null for Phibar); see
+  // planck_bands
+  double pl[SWP_EMISSION_MAX_BANDS], bw[SWP_EMISSION_MAX_BANDS];
+  double p0, pmin;
+  int folded;  // scale >= 1: T need not be formed
+  double tm1[EXP_N];  // 2^(j / 64) - 1
 };
+
+__device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
 
 __device__ __forceinline__ double temperature(const EmCfg& c, double phi, double Phibar) {
   const double T = c.temp_mode == 0 ? (Phibar + phi) / c.R_d : c.T_ref + phi / c.phi_to_T_scale;
   return fmax(T, c.Tmin);
 }
-// relative Planck intensity 1 / (expm1(x) + tiny), x = h c / (lambda kB T)
-// clipped to [0, x_clip] (pipeline.py:716-735)
-__device__ __forceinline__ double planck_rel(double T, double lam, double x_clip) {
-  const double h = 6.62607015e-34, c = 299792458.0, kB = 1.380649e-23;
-  double x = (h * c) / (lam * kB * T);
-  x = fmin(fmax(x, 0.0), x_clip);
-  return 1.0 / (expm1(x) + 1.0e-30);
+// relative Planck intensity 1 / (expm1(x) + tiny) at x in [0, 700]
+// (pipeline.py:716-735).  expm1 by table-driven reduction (Tang, ACM TOMS 15,
+// 1989): x = n ln2 / 64 + r, 2^(n/64) = 2^e (1 + tm1[j]),
+//   expm1(x) = 2^e (1 + tm1) p + (2^e tm1 + (2^e - 1)),  p = expm1(r), |r| <= ln2 / 128,
+// with p's Taylor polynomial to r^5 (the next term is below 2^-54 p).  12 FP64
+// instructions, where the library call took about 40 of the map's 100 a pixel.
+__device__ __forceinline__ double planck_rel(double x, const double* __restrict__ tm1) {
+  const double magic = 6755399441055744.0;  // 1.5 * 2^52: rounds to an integer in the low word
+  const double t = fma(x, 92.332482616893656877, magic);  // 64 / ln 2
+  const int n = __double2loint(t);
+  const double fn = t - magic;
+  // ln2 / 64 as a 33-bit head (n < 2^17: the products are exact) and a tail
+  double r = fma(fn, -0x1.62e42feep-7, x);
+  r = fma(fn, -0x1.a39ef35793c76p-39, r);
+  double p = fma(r, 1.0 / 120.0, 1.0 / 24.0);
+  p = fma(p, r, 1.0 / 6.0);
+  p = fma(p, r, 0.5);
+  p = fma(p, r, 1.0) * r;
+  const double e2 = __hiloint2double((1023 + (n >> 6)) << 20, 0);
+  const double t1 = tm1[n & (EXP_N - 1)];
+  const double q = fma(e2, t1, e2 - 1.0);
+  return 1.0 / (fma(q + 1.0, p, q) + 1.0e-30);
 }
-__device__ __forceinline__ double intensity(const EmCfg& c, double T) {
-  if (c.model == 0) {
-    const double t2 = T * T;
-    return t2 * t2;
-  }
+// v: Phi, or T (c.input 1)
+__device__ __forceinline__ double planck_bands(const EmCfg& c, double v, double Phibar,
+                                               const double* __restrict__ tm1) {
+  const double p0 = c.input == 0 && c.temp_mode == 0 ? Phibar : c.p0;
+  const double u = c.input != 0 ? v : c.folded ? fmax(p0 + v, c.pmin) : temperature(c, v, Phibar);
   double out = 0.0;
-  for (int k = 0; k < c.nbands; ++k) out += c.bw[k] * planck_rel(T, c.wl[k], c.x_clip);
+  for (int k = 0; k < c.nbands; ++k)
+    out += c.bw[k] * planck_rel(fmin(fmax(c.pl[k] / u, 0.0), c.x_clip), tm1);
   return out;
 }
 
-// One CTA per member.  stage 0 writes T, 1 the intensity map, 2 the weighted
-// relative intensity w_sqrt I / I_mean that the projector multiplies (and
-// ok[b] = the map's guards passed).  The passes follow the reference's guards:
-// a non-finite Phi makes T all NaN; a non-finite T makes the Planck intensity
-// all NaN; the relative map needs a finite, nonzero weighted mean.
-__global__ void __launch_bounds__(EM_THREADS) k_emission_map(const double* __restrict__ in,
-                                                             const double* __restrict__ Phibar, int J, int I,
-                                                             const double* __restrict__ w_lat, EmCfg c, int stage,
-                                                             double* __restrict__ out, int* __restrict__ ok) {
-  __shared__ double red[EM_THREADS / 32 + 1];
-  const int b = blockIdx.x;
+// One cluster per member, a warp per latitude row.  stage 0 writes T, 1 the
+// intensity map, 2 the weighted relative intensity w_sqrt I / I_mean that the
+// projector multiplies (and ok[b] = the map's guards passed).  The passes
+// follow the reference's guards: a non-finite Phi makes T all NaN; a non-finite
+// T makes the Planck intensity all NaN; the relative map needs a finite,
+// nonzero weighted mean.
+//
+// FP64-bound (see EM_CL).  The Planck argument takes one division (T itself is
+// not formed), finiteness is tested on the exponent bits, the square root of a
+// weight is taken once per row, with the quotient by the mean folded into it.
+__global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS)
+    k_emission_map(const double* __restrict__ in, const double* __restrict__ Phibar, int J, int I,
+                   const double* __restrict__ w_lat, const __grid_constant__ EmCfg c, int stage,
+                   double* __restrict__ out, int* __restrict__ ok) {
+  __shared__ double slots[2][3 * EM_WARPS];
+  __shared__ double tm1[EXP_N];
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), b = blockIdx.x / EM_CL;
+  const int lane = threadIdx.x & 31;
+  const int row0 = rank * EM_WARPS + (threadIdx.x >> 5);
+  constexpr int ROWS = EM_CL * EM_WARPS;
   const size_t npix = (size_t)J * I;
   const double* x = in + (size_t)b * npix;
   double* y = out + (size_t)b * npix;
   const double pb = Phibar ? Phibar[b] : 0.0;
   const double qnan = __longlong_as_double(0x7ff8000000000000ll);
-  // pass 1: all of the input finite (Phi -> T guard; a T or intensity input
-  // enters the guard of its own stage below)
-  bool fin = true;
-  for (size_t p = threadIdx.x; p < npix; p += EM_THREADS) fin &= isfinite(x[p]) != 0;
-  const bool in_ok = block_all(fin);
-  auto T_at = [&](size_t p) { return c.input == 0 ? (in_ok ? temperature(c, x[p], pb) : qnan) : x[p]; };
-  if (stage == 0) {
-    for (size_t p = threadIdx.x; p < npix; p += EM_THREADS) y[p] = T_at(p);
-    return;
+  if (threadIdx.x < EXP_N) tm1[threadIdx.x] = c.tm1[threadIdx.x];
+  // pass 1: all of the input finite (Phi -> T guard) and, with the Planck
+  // model, all of T finite
+  bool nan_map = false;
+  if (c.input == 0 || (c.input == 1 && c.model == 1)) {
+    bool fin = true;
+    const double p0 = c.temp_mode == 0 ? pb : c.p0;
+    for (int j = row0; j < J; j += ROWS)
+      for (int i = lane; i < I; i += 32) {
+        const double v = x[(size_t)j * I + i];
+        fin &= finite_bits(v);
+        if (c.input == 0 && c.model == 1 && stage > 0) fin &= finite_bits(c.folded ? p0 + v : temperature(c, v, pb));
+      }
+    nan_map = !cluster_sum(0.0, 0.0, fin, slots[0]).all;
+  } else {
+    cl.sync();  // tm1, and every rank running before the remote reads below
   }
-  // pass 2: the Planck guard needs every T finite
-  bool t_ok = true;
-  if (c.input <= 1 && c.model == 1) {
-    bool ft = true;
-    for (size_t p = threadIdx.x; p < npix; p += EM_THREADS) ft &= isfinite(T_at(p)) != 0;
-    t_ok = block_all(ft);
-  }
-  auto I_at = [&](size_t p) {
-    if (c.input == 2) return x[p];
-    const double T = T_at(p);
-    return (c.model == 1 && !t_ok) ? qnan : intensity(c, T);
-  };
-  if (stage == 1) {
-    for (size_t p = threadIdx.x; p < npix; p += EM_THREADS) y[p] = I_at(p);
-    return;
-  }
-  // pass 3: the weighted mean over the finite pixels (pipeline.py:821-837)
+  // pass 2: T, or the intensity and, for stage 2, its weighted mean over the
+  // finite pixels (pipeline.py:821-837)
   double sw = 0.0, swi = 0.0;
   bool fi = true;
-  for (size_t p = threadIdx.x; p < npix; p += EM_THREADS) {
-    const double v = I_at(p);
-    const double w = w_lat[p / I];
-    const bool f = isfinite(v) != 0;
-    fi &= f;
-    if (f) {
-      sw += w;
-      swi += w * v;
+  for (int j = row0; j < J; j += ROWS) {
+    const double w = stage == 2 ? w_lat[j] : 0.0;
+    for (int i = lane; i < I; i += 32) {
+      const size_t p = (size_t)j * I + i;
+      double v = x[p];
+      if (nan_map) {
+        v = qnan;
+      } else if (c.input < 2) {
+        if (stage > 0 && c.model == 1) {
+          v = planck_bands(c, v, pb, tm1);
+        } else {
+          if (c.input == 0) v = temperature(c, v, pb);
+          if (stage > 0) {
+            v *= v;
+            v *= v;
+          }
+        }
+      }
+      y[p] = v;
+      if (stage == 2) {
+        const bool f = finite_bits(v);
+        fi &= f;
+        if (f) {
+          sw += w;
+          swi += w * v;
+        }
+      }
     }
-    y[p] = v;  // kept for pass 4
   }
-  const bool all_fin = block_all(fi);
-  const double w_sum = block_sum(sw, red);
-  const double wi_sum = block_sum(swi, red);
-  const double mean = w_sum > 0.0 ? wi_sum / w_sum : qnan;
+  if (stage < 2) {
+    cl.sync();  // a peer may still read this CTA's slots
+    return;
+  }
+  const ClusterSum s = cluster_sum(sw, swi, fi, slots[1]);
+  const double mean = s.a > 0.0 ? s.b / s.a : qnan;
   const bool mean_ok = isfinite(mean) && fabs(mean) > 1.0e-30;
-  // pass 4: rhs = sqrt(w) * I_rel, I_rel = I / mean (NaN where I is not finite or the mean fails)
-  for (size_t p = threadIdx.x; p < npix; p += EM_THREADS) {
-    const double v = y[p];
-    const double safe = isfinite(v) ? v : 0.0;
-    y[p] = sqrt(w_lat[p / I]) * (mean_ok ? safe / mean : qnan);
+  // pass 3: rhs = sqrt(w) * I_rel, I_rel = I / mean (NaN where the mean fails, 0 where I is not finite)
+  for (int j = row0; j < J; j += ROWS) {
+    const double q = mean_ok ? sqrt(w_lat[j]) / mean : qnan;
+    for (int i = lane; i < I; i += 32) {
+      const size_t p = (size_t)j * I + i;
+      const double v = y[p];
+      y[p] = finite_bits(v) ? q * v : q * 0.0;
+    }
   }
-  if (threadIdx.x == 0 && ok) ok[b] = (all_fin && mean_ok) ? 1 : 0;
+  if (rank == 0 && threadIdx.x == 0 && ok) ok[b] = (s.all && mean_ok) ? 1 : 0;
+  cl.sync();
 }
 
 // Y[b][c] = sum_p P[c][p] rhs[b][p]: one CTA per (member, 32 coefficients),
@@ -200,36 +287,86 @@ __global__ void k_phase_curve_linear(const double* __restrict__ y, const double*
 }
 
 // flux[b][k] = sum_{j,i} Phi max(cos(lambda_i - phase_k), 0) sqrt(1 - mu_j^2),
-// then divided by mean_k |flux| when that is positive: one CTA per member.
-__global__ void __launch_bounds__(EM_THREADS) k_phase_curve_simple(const double* __restrict__ phi, int J, int I,
-                                                                   const double* __restrict__ mus,
-                                                                   const double* __restrict__ phases, int nph,
-                                                                   double* __restrict__ flux) {
-  __shared__ double red[EM_THREADS / 32 + 1];
-  const int b = blockIdx.x;
-  const size_t npix = (size_t)J * I;
-  const double* x = phi + (size_t)b * npix;
+// then divided by mean_k |flux| when that is positive: one cluster per member.
+// The sum over latitudes does not depend on the phase, so each rank first forms
+// the columns s_i = sum_j Phi_ij sqrt(1 - mu_j^2) of its share of a block of
+// PC_BLOCK longitudes, with cos and sin of those longitudes, and hands them to
+// every rank; a warp then takes a phase and its lanes the longitudes, with
+// cos(lambda - phase) by the addition theorem.  One cosine per longitude and
+// per phase in the place of one per (pixel, phase): 8.0 ms before for one M = 42
+// map and 100 phases, FP64-bound on one SM.
+constexpr int PC_BLOCK = 512;
+__global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS)
+    k_phase_curve_simple(const double* __restrict__ phi, int J, int I, const double* __restrict__ mus,
+                         const double* __restrict__ phases, int nph, double* __restrict__ flux) {
+  __shared__ double col[3][PC_BLOCK];      // s_i, cos(lambda_i), sin(lambda_i) of the block
+  __shared__ double part[EM_THREADS];      // column partial sums of each row group
+  __shared__ double trig[2][32];           // cos, sin of this CTA's next 32 phases
+  __shared__ double slots[3 * EM_WARPS];
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), b = blockIdx.x / EM_CL;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const double* x = phi + (size_t)b * J * I;
   double* f = flux + (size_t)b * nph;
   const double pi = 3.141592653589793, step = (pi - (-pi)) / I;  // numpy linspace(-pi, pi, I, endpoint=False)
-  double asum = 0.0;
-  for (int k = 0; k < nph; ++k) {
-    const double ph = phases[k];
+  for (int i0 = 0; i0 < I; i0 += PC_BLOCK) {
+    const int nb = min(PC_BLOCK, I - i0), share = (nb + EM_CL - 1) / EM_CL;
+    const int c0 = rank * share, nc = max(0, min(share, nb - c0));
+    const int ng = EM_THREADS / share;  // row groups (share <= 64: at least 4)
+    const int g = threadIdx.x / share, cc = threadIdx.x % share;
     double s = 0.0;
-    for (size_t p = threadIdx.x; p < npix; p += EM_THREADS) {
-      const int j = (int)(p / I), i = (int)(p % I);
-      const double mu = mus[j];
-      const double aw = sqrt(fmax(1.0 - mu * mu, 0.0));
-      const double vis = fmax(cos((-pi + i * step) - ph), 0.0);
-      s += x[p] * vis * aw;
+    if (g < ng && cc < nc)
+      for (int j = g; j < J; j += ng) {
+        const double mu = mus[j];
+        s = fma(x[(size_t)j * I + i0 + c0 + cc], sqrt(fmax(1.0 - mu * mu, 0.0)), s);
+      }
+    part[threadIdx.x] = s;
+    double sl = 0.0, cs = 0.0;
+    if (threadIdx.x < nc) sincos(-pi + (i0 + c0 + (int)threadIdx.x) * step, &sl, &cs);
+    cl.sync();  // part is complete; every rank is done with the previous block's columns
+    if (threadIdx.x < nc) {
+      double t = 0.0;
+      for (int q = 0; q < ng; ++q) t += part[q * share + threadIdx.x];
+      for (int r = 0; r < EM_CL; ++r) {
+        double* dst = cl.map_shared_rank(&col[0][0], r) + c0 + threadIdx.x;
+        dst[0] = t;
+        dst[PC_BLOCK] = cs;
+        dst[2 * PC_BLOCK] = sl;
+      }
     }
-    const double tot = block_sum(s, red);
-    if (threadIdx.x == 0) f[k] = tot;
-    asum += fabs(tot);
+    cl.sync();
+    // this rank's phases k = rank + 8 q, 32 at a time: their sines and cosines
+    // by one warp, then a warp per phase
+    for (int q0 = 0; rank + EM_CL * q0 < nph; q0 += 32) {
+      __syncthreads();
+      if (warp == 0) {
+        const int k = rank + EM_CL * (q0 + lane);
+        double sp = 0.0, cp = 0.0;
+        if (k < nph) sincos(phases[k], &sp, &cp);
+        trig[0][lane] = cp;
+        trig[1][lane] = sp;
+      }
+      __syncthreads();
+      for (int q = warp; q < 32; q += EM_WARPS) {
+        const int k = rank + EM_CL * (q0 + q);
+        if (k >= nph) break;
+        const double cp = trig[0][q], sp = trig[1][q];
+        double t = 0.0;
+        for (int i = lane; i < nb; i += 32)
+          t = fma(col[0][i], fmax(fma(col[1][i], cp, col[2][i] * sp), 0.0), t);
+        t = warp_sum(t);
+        if (lane == 0) f[k] = i0 == 0 ? t : f[k] + t;
+      }
+    }
   }
-  const double norm = asum / nph;
-  __syncthreads();
-  if (norm > 0.0)
-    for (int k = threadIdx.x; k < nph; k += EM_THREADS) f[k] = f[k] / norm;
+  // the mean of |flux| and the division, by the thread that wrote each value
+  double asum = 0.0;
+  for (int q = warp; rank + EM_CL * q < nph; q += EM_WARPS)
+    if (lane == 0) asum += fabs(f[rank + EM_CL * q]);
+  const double norm = cluster_sum(asum, 0.0, true, slots).a / nph;
+  if (norm > 0.0 && lane == 0)
+    for (int q = warp; rank + EM_CL * q < nph; q += EM_WARPS) f[rank + EM_CL * q] /= norm;
+  cl.sync();  // a peer may still read this CTA's slots
 }
 
 int em_check(cudaError_t e) { return e == cudaSuccess ? SWP_OK : SWP_ERR_CUDA; }
@@ -258,12 +395,22 @@ extern "C" int swp_emission_map(const double* in, const double* Phibar, int B, i
   c.T_ref = cfg->T_ref;
   c.phi_to_T_scale = cfg->phi_to_T_scale;
   c.Tmin = cfg->Tmin;
-  c.x_clip = cfg->x_clip;
+  // T = (p0 + Phi) / scale: with scale >= 1 (so that T is finite where p0 + Phi
+  // is) the Planck argument needs no T of its own.  Formed in long double and
+  // rounded once.
+  const long double hck = 6.62607015e-34L * 299792458.0L / 1.380649e-23L;
+  const double div = cfg->temp_mode == 0 ? cfg->R_d : cfg->phi_to_T_scale;
+  c.folded = input == 0 && div >= 1.0;
+  const long double scale = c.folded ? div : 1.0L;
+  c.x_clip = cfg->x_clip < 700.0 ? cfg->x_clip : 700.0;
+  c.p0 = c.folded && cfg->temp_mode == 1 ? (double)(cfg->T_ref * scale) : 0.0;
+  c.pmin = (double)(cfg->Tmin * scale);
   for (int k = 0; k < SWP_EMISSION_MAX_BANDS; ++k) {
-    c.wl[k] = k < c.nbands ? cfg->wavelengths[k] : 1.0;
+    c.pl[k] = k < c.nbands ? (double)(hck * scale / cfg->wavelengths[k]) : 1.0;
     c.bw[k] = k < c.nbands ? cfg->band_weights[k] : 0.0;
   }
-  k_emission_map<<<B, EM_THREADS, 0, (cudaStream_t)stream>>>(in, Phibar, J, I, w_lat, c, stage, out, ok);
+  for (int j = 0; j < EXP_N; ++j) c.tm1[j] = (double)(exp2l((long double)j / EXP_N) - 1.0L);
+  k_emission_map<<<EM_CL * B, EM_THREADS, 0, (cudaStream_t)stream>>>(in, Phibar, J, I, w_lat, c, stage, out, ok);
   return em_check(cudaGetLastError());
 }
 
@@ -291,6 +438,6 @@ extern "C" int swp_phase_curve_linear(const double* y, const double* design, con
 extern "C" int swp_phase_curve_simple(const double* phi, int B, int J, int I, const double* mus,
                                       const double* phases, int nphase, double* flux, void* stream) {
   if (!phi || !mus || !phases || !flux || B < 1 || J < 1 || I < 1 || nphase < 1) return SWP_ERR_ARG;
-  k_phase_curve_simple<<<B, EM_THREADS, 0, (cudaStream_t)stream>>>(phi, J, I, mus, phases, nphase, flux);
+  k_phase_curve_simple<<<EM_CL * B, EM_THREADS, 0, (cudaStream_t)stream>>>(phi, J, I, mus, phases, nphase, flux);
   return em_check(cudaGetLastError());
 }

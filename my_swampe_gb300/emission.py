@@ -25,6 +25,7 @@ from __future__ import annotations
 
 import ctypes
 from dataclasses import dataclass
+from functools import lru_cache
 from typing import Optional, Sequence, Tuple
 
 import numpy as np
@@ -218,6 +219,13 @@ def phase_curve(y, design_lc, amplitude=1.0) -> torch.Tensor:
     return lc if batched else lc[0]
 
 
+@lru_cache(maxsize=8)
+def _gauss_nodes(J: int, dev: torch.device) -> torch.Tensor:
+    """numpy's Gauss-Legendre nodes of a J-latitude grid (constants: an
+    eigenvalue problem on the host, once per grid)."""
+    return torch.as_tensor(np.polynomial.legendre.leggauss(J)[0], dtype=torch.float64, device=dev)
+
+
 def simple_phase_curve(phi, phase_angles, mus=None) -> torch.Tensor:
     """The simplified phase-curve projection of the reference's parity test
     (``unit_tests/test_parity_reference_regression.py:67-82``): per phase, the
@@ -227,8 +235,8 @@ def simple_phase_curve(phi, phase_angles, mus=None) -> torch.Tensor:
     xs, batched = _ensemble(phi, "phi")
     B, J, I = xs.shape
     dev = xs.device
-    mu = np.polynomial.legendre.leggauss(J)[0] if mus is None else mus
-    mu = torch.as_tensor(mu, dtype=torch.float64, device=dev).reshape(-1).contiguous()
+    mu = _gauss_nodes(J, dev) if mus is None else torch.as_tensor(mus, dtype=torch.float64, device=dev)
+    mu = mu.reshape(-1).contiguous()
     ph = torch.as_tensor(phase_angles, dtype=torch.float64, device=dev).reshape(-1).contiguous()
     if mu.numel() != J:
         raise ValueError(f"mus must have {J} values")
