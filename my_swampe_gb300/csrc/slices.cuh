@@ -1,0 +1,166 @@
+// FP64 contractions on the FP16 tensor cores.
+//
+// GB300 retires 1.7 FP64 FMAs per cycle and SM (measured: one warp instruction
+// per 19 cycles and SM, per 64 cycles and sub-partition, whatever its active
+// lanes), and 1026 FP16 multiply-adds per cycle and SM through mma.sync.  So an
+// FP64 contraction is done on integer slices of its operands (Ozaki, Ogita,
+// Oishi, Rump, Numer. Algorithms 59, 2012):
+//
+//   * A row of an operand (its elements along the contraction) is put on one
+//     fixed-point scale: x = q 2^(er - 1076), er the largest exponent field of
+//     the row, |q| < 2^54, truncated: at most 2^-53 of the row's maximum off, 2^-54
+//     on average.  Basis matrices are put on it once, when the plan is made.
+//   * q is written in 7 balanced base-256 digits, each in [-128, 127] (the top
+//     one in [-65, 65]), which FP16 holds exactly.
+//   * Products of digits u and v (0 = top) go to level u + v.  Levels 0..7 are
+//     kept (34 digit products); what is dropped is below 2^-60 of the rows'
+//     maxima.  A level's sum over K = 32 stays below 2^22 and is therefore exact
+//     in the FP32 accumulator, which starts at 1.5 * 2^23, so that its bit
+//     pattern is the integer.
+//   * The levels are added up in 64-bit integers (hi: levels 0..3, lo: 4..7),
+//     over any number of K = 32 blocks, and converted once: 3 FP64 additions an
+//     output, whatever K.
+//
+// The result's error is that of the inputs on the row's scale and one final
+// rounding; a chain of FP64 FMAs rounds K times.  A row that holds an infinity or
+// a NaN gives NaN.
+#pragma once
+#include <cuda_fp16.h>
+#include <stdint.h>
+
+namespace swp {
+namespace slices {
+
+constexpr int ND = 7;                       // digits
+constexpr int NL = 8;                       // levels kept
+constexpr uint64_t BIAS = 0x0080808080808080ull;  // 128 in each digit
+constexpr float ACC0 = 12582912.0f;         // 1.5 * 2^23
+constexpr int ACC0_BITS = 0x4B400000;
+constexpr int ER_BAD = 4000;                // row exponent of a row with an infinity or a NaN
+constexpr int ER_ZERO = -8000;              // row exponent of a zero row
+constexpr int KFLUSH = 2;                   // mma k-steps (of 16) per flush of the accumulators
+
+__device__ __forceinline__ int expo(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+// A row's exponent from the maximum of expo over it; a row below 2^-959 counts as zero.
+__device__ __forceinline__ int row_exponent(int emax) { return emax == 0x7ff ? ER_BAD : emax < 64 ? ER_ZERO : emax; }
+
+// Biased fixed point of x on its row's scale, truncated: byte 6 - u is digit u
+// plus 128.  Elements below the scale's unit, and all of a zero or bad row, give 0.
+__device__ __forceinline__ uint64_t fixed(double x, int er) {
+  const uint32_t h = (uint32_t)__double2hiint(x), l = (uint32_t)__double2loint(x);
+  const uint32_t sh = min((uint32_t)(er - (int)((h >> 20) & 0x7ff)), 63u);
+  const uint32_t m1 = __funnelshift_l(l, (h & 0xfffffu) | 0x100000u, 1), m0 = l << 1;  // significand, 54 bits
+  const uint32_t a1 = __funnelshift_rc(m1, 0u, sh), a0 = __funnelshift_rc(m0, m1, sh);
+  const uint32_t b0 = __funnelshift_rc(m1, 0u, sh - 32u);
+  const uint64_t q = sh < 32u ? ((uint64_t)a1 << 32) | a0 : (uint64_t)b0;
+  return (h >> 31) ? BIAS - q : BIAS + q;
+}
+
+// Digit u of two elements as an FP16 pair.
+template <int U>
+__device__ __forceinline__ uint32_t digit_pair(uint64_t a, uint64_t b) {
+  constexpr int i = 6 - U;
+  const uint32_t wa = i < 4 ? (uint32_t)a : (uint32_t)(a >> 32), wb = i < 4 ? (uint32_t)b : (uint32_t)(b >> 32);
+  // bytes (a, any, b, any), then the upper byte of each half set to 0x64: 1024 + byte, exact in FP16
+  const uint32_t p = __byte_perm(wa, wb, (uint32_t)((i & 3) | ((4 + (i & 3)) << 8)));
+  const uint32_t h = (p & 0x00ff00ffu) | 0x64006400u;
+  const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&h), __floats2half2_rn(1152.0f, 1152.0f));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+// Digits of two elements adjacent along K: out[u * stride], u = 0..6.
+__device__ __forceinline__ void store_digits(uint32_t* out, int stride, uint64_t a, uint64_t b) {
+  out[0] = digit_pair<0>(a, b);
+  out[stride] = digit_pair<1>(a, b);
+  out[2 * stride] = digit_pair<2>(a, b);
+  out[3 * stride] = digit_pair<3>(a, b);
+  out[4 * stride] = digit_pair<4>(a, b);
+  out[5 * stride] = digit_pair<5>(a, b);
+  out[6 * stride] = digit_pair<6>(a, b);
+}
+
+__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// A 16 x 8 output tile of a warp.  Lane l holds rows l / 4 and l / 4 + 8,
+// columns 2 (l % 4) and + 1: element 2 r + c is (row r, column c).
+struct Tile {
+  float acc[NL][4];
+  long long hi[4], lo[4];
+
+  __device__ __forceinline__ void reset() {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) hi[e] = lo[e] = 0;
+    restart();
+  }
+  __device__ __forceinline__ void restart() {
+#pragma unroll
+    for (int l = 0; l < NL; ++l)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[l][e] = ACC0;
+  }
+  // one k-step: a[u] the A fragment of digit u, b[v] the B fragment of digit v
+  __device__ __forceinline__ void step(const uint32_t (&a)[ND][4], const uint32_t (&b)[ND][2]) {
+#pragma unroll
+    for (int u = 0; u < ND; ++u)
+#pragma unroll
+      for (int v = 0; v < ND; ++v)
+        if (u + v < NL) mma(acc[u + v], a[u], b[v]);
+  }
+  // add the accumulated levels (at most KFLUSH k-steps) to the integer sums
+  __device__ __forceinline__ void flush() {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      int i[NL];
+#pragma unroll
+      for (int l = 0; l < NL; ++l) i[l] = __float_as_int(acc[l][e]) - ACC0_BITS;
+      hi[e] += (long long)(i[0] * 256 + i[1]) * 65536 + (i[2] * 256 + i[3]);
+      lo[e] += (long long)(i[4] * 256 + i[5]) * 65536 + (i[6] * 256 + i[7]);
+    }
+    restart();
+  }
+};
+
+// The FP64 value of integer sums over at most 2^14 elements on the scales of an
+// A row and a B row.
+__device__ __forceinline__ double value(long long hi, long long lo, int era, int erb) {
+  const int s = era + erb;
+  hi += lo >> 32;  // a unit of hi is 2^32 units of lo
+  lo &= 0xffffffffll;
+  // 1.5 * 2^(52 + k) with unit 2^k: adding the integer to its bits adds integer * 2^k
+  const long long mh = ((long long)(s - 1005) << 52) | 0x8000000000000ll;
+  const long long ml = ((long long)(s - 1037) << 52) | 0x8000000000000ll;
+  const double h = __longlong_as_double(mh + hi) - __longlong_as_double(mh);
+  const double l = __longlong_as_double(ml + lo) - __longlong_as_double(ml);
+  if (s < 1038) return 0.0;                                       // a zero row, or below 2^-1000
+  if (s > 3051) return __longlong_as_double(0x7ff8000000000000ll);  // a bad row
+  return h + l;
+}
+
+// The B fragment of one k-step from digit planes in shared memory: `p` points
+// at (row of this lane's column, k) of digit 0, words of two elements.
+__device__ __forceinline__ void load_b(uint32_t (&b)[ND][2], const uint32_t* p, int plane) {
+#pragma unroll
+  for (int v = 0; v < ND; ++v) {
+    b[v][0] = p[v * plane];
+    b[v][1] = p[v * plane + 4];
+  }
+}
+// The A fragment of one k-step from a packed static operand (pack_a):
+// [k-step][digit][lane] of 16 bytes.
+__device__ __forceinline__ void load_a(uint32_t (&a)[ND][4], const uint4* __restrict__ p) {
+#pragma unroll
+  for (int u = 0; u < ND; ++u) {
+    const uint4 w = __ldg(p + u * 32);
+    a[u][0] = w.x;
+    a[u][1] = w.y;
+    a[u][2] = w.z;
+    a[u][3] = w.w;
+  }
+}
+
+}  // namespace slices
+}  // namespace swp

@@ -55,3 +55,47 @@ def test_planck_map_sizes(cuda, JI, mode, scale):
     assert np.max(np.abs(got / want - 1.0)) <= (4 * 81 + 8) * EPS
     again = temperature_to_intensity(torch.tensor(Tx, device="cuda"), EmissionConfig(**kw)).cpu().numpy()
     assert np.max(np.abs(again / want - 1.0)) <= (4 * 81 + 8) * EPS
+
+
+@pytest.mark.parametrize("npix,ncoef,B", [(1, 1, 1), (63, 5, 2), (65, 16, 16), (510, 17, 17), (8192, 121, 3),
+                                          (513, 129, 33), (70001, 3, 2)])
+@pytest.mark.parametrize("kind", ["noise", "constant", "range"])
+def test_projection_sizes(cuda, npix, ncoef, B, kind):
+    """The sliced projection against extended precision: tiles of 16 members and
+    128 coefficients and eighths of the pixels with remainders, more pixels than
+    one conversion of the integer sums; constant rows (all digits alike, the
+    largest integer sums) and rows that span 40 powers of ten."""
+    from my_swampe_gb300.emission import _project
+
+    rng = np.random.default_rng(npix + ncoef)
+    P = rng.standard_normal((ncoef, npix))
+    r = rng.standard_normal((B, npix)) + 1.0
+    if kind == "constant":
+        P[:], r[:] = -(1.0 - 2.0**-53) / 3.0, 0.1
+    if kind == "range":
+        P *= 10.0 ** rng.uniform(-40, 0, P.shape)
+        r *= 10.0 ** rng.uniform(0, 5, r.shape)
+    P[0] = np.abs(P[0]) + 1e-3
+    r = np.abs(r)
+    ok = torch.ones(B, dtype=torch.int32, device="cuda")
+    y = _project(torch.tensor(r, device="cuda").reshape(B, 1, npix), ok, torch.tensor(P, device="cuda")).cpu().numpy()
+    want = (r.astype(np.longdouble) @ P.T.astype(np.longdouble))
+    # each operand is truncated to 2^-53 of its row's maximum, a product's dropped
+    # digits are below 2^-59, the eight partial sums and y0's quotient round once each
+    unit = 2.0**-51 * npix * np.max(np.abs(r), axis=1, keepdims=True) * np.max(np.abs(P), axis=1)
+    err = unit + 9 * EPS * np.abs(r) @ np.abs(P).T
+    bound = (err + np.abs(want / want[:, :1]) * err[:, :1]) / np.abs(want[:, :1]) + 2 * EPS * np.abs(want / want[:, :1])
+    assert np.all(np.abs(y - want / want[:, :1]) <= bound)
+
+
+def test_projection_of_non_finite_members(cuda):
+    """An infinity or a NaN anywhere in a member gives NaN for it and leaves the others of its tile alone."""
+    from my_swampe_gb300.emission import _project
+
+    rng = np.random.default_rng(5)
+    P, r = np.abs(rng.standard_normal((20, 300))), np.abs(rng.standard_normal((5, 300)))
+    ok = torch.ones(5, dtype=torch.int32, device="cuda")
+    clean = _project(torch.tensor(r, device="cuda").reshape(5, 1, 300), ok, torch.tensor(P, device="cuda"))
+    r[1, 7], r[3, 299] = np.inf, np.nan
+    y = _project(torch.tensor(r, device="cuda").reshape(5, 1, 300), ok, torch.tensor(P, device="cuda"))
+    assert torch.isnan(y[[1, 3]]).all() and torch.equal(y[[0, 2, 4]], clean[[0, 2, 4]])
