@@ -33,6 +33,9 @@ struct swp_plan {
   bool tc[MAXG] = {};
   float* tcbasis[MAXG] = {};
   float* tcbasis_adj[MAXG] = {};
+  // FP64 Legendre kernels on integer slices (spectral_f64.cu): packed basis of
+  // the step and of its transpose
+  SliceBasis slices = {}, slices_adj = {};
   void* coefmem[MAXG] = {};              // per-call coefficient tables (CoefTables) of each group
   int* d_err = nullptr;                  // device error word set by bounded waits that ran out
   SchedCounter* d_sched = nullptr;       // persistent-launch counters: one per group chain, one for joint launches
@@ -268,8 +271,10 @@ SpecLaunch<T> simt_only(const swp_plan* p, const SpecLaunch<T>& LS, bool adjoint
   return L;
 }
 
-// The Legendre kernel of a modified-Euler step: tcgen05 (3xTF32) on the FP32
-// path when the plan packed the tensor-core basis, the SIMT kernel otherwise.
+// The Legendre kernel of a step: on the FP32 path tcgen05 (3xTF32) for the
+// modified-Euler scheme when the plan packed the tensor-core basis, the SIMT
+// kernel otherwise; in FP64 the sliced kernel.  The primal step of a tangent run
+// with filter-weight tangents is the SIMT kernel's.
 template <typename T>
 cudaError_t launch_step_spec(const swp_plan* p, const SpecLaunch<T>& LS, int nbs, cudaStream_t s) {
   if constexpr (std::is_same<T, float>::value) {
@@ -283,12 +288,13 @@ cudaError_t launch_step_spec(const swp_plan* p, const SpecLaunch<T>& LS, int nbs
       if (e == cudaSuccess && nb > 0) e = launch_spec<T>(LR, nb, p->spec_smem, s);
       return e;
     }
+  } else if (LS.mode == 0 && !LS.cfg.tl_filter) {
+    return launch_spec_f64(LS, p->slices, false, s);
   }
   return launch_spec<T>(LS, nbs, p->spec_smem, s);
 }
 
-// The Legendre adjoint of a modified-Euler step: tcgen05 on the FP32 path when
-// the plan packed the tensor-core basis, the SIMT kernel otherwise.
+// The Legendre adjoint of a step: as launch_step_spec.
 template <typename T>
 cudaError_t launch_step_spec_adj(const swp_plan* p, const SpecLaunch<T>& LS, int nbs, cudaStream_t s) {
   if constexpr (std::is_same<T, float>::value) {
@@ -302,8 +308,10 @@ cudaError_t launch_step_spec_adj(const swp_plan* p, const SpecLaunch<T>& LS, int
       if (e == cudaSuccess && nb > 0) e = launch_spec_adj<T>(LR, nb, p->spec_adj_smem, s);
       return e;
     }
+    return launch_spec_adj<T>(LS, nbs, p->spec_adj_smem, s);
+  } else {
+    return launch_spec_f64(LS, p->slices_adj, true, s);
   }
-  return launch_spec_adj<T>(LS, nbs, p->spec_adj_smem, s);
 }
 
 // Launch nsteps steps.  In place on st[g].fourier, or -- when `slots` is given --
@@ -981,6 +989,10 @@ int autotune_impl(swp_plan* p, const swp_group_state* st, const swp_group_adjoin
       cudaError_t e = cudaSuccess;
       for (int r = 0; r < nrep + 1 && e == cudaSuccess; ++r) {  // the first repetition warms up
         if (r == 1) cudaEventRecord(e0, s);
+        if (f64) {  // the tile is that of the SIMT kernel (tangent steps, winds)
+          e = launch_spec<T>(LS, nbs, p->spec_smem, s);
+          continue;
+        }
         e = launch_step_spec<T>(p, LS, nbs, s);
         if (e == cudaSuccess) e = launch_step_spec_adj<T>(p, LA, nbs, s);
       }
@@ -1088,6 +1100,7 @@ int swp_plan_create(int ngroups, const int* M, const int* B, int precision, swp_
   const char* ng_env = getenv("SWP_NO_GRAPH");
   p->graphs_enabled = !(ng_env && ng_env[0] == '1');
   spec_set_attributes();
+  spec_f64_set_attributes();
   grid_set_attributes();
   spec_tc_set_attributes();
   cudaStream_t s = 0;
@@ -1161,6 +1174,23 @@ int swp_plan_create(int ngroups, const int* M, const int* B, int precision, swp_
     }
     p->use_tc = true;
   }
+  if (precision == SWP_FP64) {
+    for (int g = 0; g < ngroups; ++g) {
+      void *fwd = nullptr, *adj = nullptr;
+      cudaError_t e = cudaMalloc(&fwd, spec_f64_basis_bytes(M[g]));
+      p->slices.p[g] = fwd;
+      if (e == cudaSuccess) e = cudaMalloc(&adj, spec_f64_basis_bytes(M[g]));
+      p->slices_adj.p[g] = adj;
+      if (e == cudaSuccess) e = pack_spec_f64(p->geom[g], false, fwd, s);
+      if (e == cudaSuccess) e = pack_spec_f64(p->geom[g], true, adj, s);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+      if (e != cudaSuccess) {
+        p->err = std::string("sliced basis packing: ") + cudaGetErrorString(e);
+        *out = p;
+        return SWP_ERR_CUDA;
+      }
+    }
+  }
   *out = p;
   return SWP_OK;
 }
@@ -1180,6 +1210,8 @@ int swp_plan_destroy(swp_plan* p) {
     if (p->geom[g].mem) cudaFree(p->geom[g].mem);
     if (p->tcbasis[g]) cudaFree(p->tcbasis[g]);
     if (p->tcbasis_adj[g]) cudaFree(p->tcbasis_adj[g]);
+    if (p->slices.p[g]) cudaFree(const_cast<void*>(p->slices.p[g]));
+    if (p->slices_adj.p[g]) cudaFree(const_cast<void*>(p->slices_adj.p[g]));
     if (p->coefmem[g]) cudaFree(p->coefmem[g]);
   }
   if (p->d_err) cudaFree(p->d_err);

@@ -366,11 +366,13 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS, 2)
           a[4][q] = digit_pair<4>(u, v);
           a[5][q] = digit_pair<5>(u, v);
           a[6][q] = digit_pair<6>(u, v);
+          a[7][q] = digit_pair<7>(u, v);
         }
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
           if (n >= nn) break;
-          load_b(bf, &S.dig[0][8 * n + g][16 * half + 8 * ks + t], PR_MEMB * PR_ROW);
+          const uint32_t* bp = &S.dig[0][8 * n + g][16 * half + 8 * ks + t];
+          load_b(bf, bp, bp + 4, PR_MEMB * PR_ROW);
           tile[n].step(a, bf);
         }
       }

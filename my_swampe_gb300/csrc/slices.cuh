@@ -7,13 +7,14 @@
 // Oishi, Rump, Numer. Algorithms 59, 2012):
 //
 //   * A row of an operand (its elements along the contraction) is put on one
-//     fixed-point scale: x = q 2^(er - 1076), er the largest exponent field of
-//     the row, |q| < 2^54, truncated: at most 2^-53 of the row's maximum off, 2^-54
-//     on average.  Basis matrices are put on it once, when the plan is made.
-//   * q is written in 7 balanced base-256 digits, each in [-128, 127] (the top
+//     fixed-point scale: x = q 2^(er - 1084), er the largest exponent field of
+//     the row, |q| <= 2^62: at most 2^-62 of the row's maximum off, so elements
+//     down to 2^-9 of it keep all their bits.  Basis matrices are put on it once,
+//     when the plan is made.
+//   * q is written in 8 balanced base-256 digits, each in [-128, 127] (the top
 //     one in [-65, 65]), which FP16 holds exactly.
 //   * Products of digits u and v (0 = top) go to level u + v.  Levels 0..7 are
-//     kept (34 digit products); what is dropped is below 2^-60 of the rows'
+//     kept (36 digit products); what is dropped is about 2^-60 of the rows'
 //     maxima.  A level's sum over K = 32 stays below 2^22 and is therefore exact
 //     in the FP32 accumulator, which starts at 1.5 * 2^23, so that its bit
 //     pattern is the integer.
@@ -22,7 +23,9 @@
 //     output, whatever K.
 //
 // The result's error is that of the inputs on the row's scale and one final
-// rounding; a chain of FP64 FMAs rounds K times.  A row that holds an infinity or
+// rounding; a chain of FP64 FMAs rounds K times.  (With 7 digits, 2^-54 of the
+// maximum, rows that fall by orders of magnitude lost bits: meridional winds were
+// up to 9 times further off the oracle than with FMAs.)  A row that holds an infinity or
 // a NaN gives NaN.
 #pragma once
 #include <cuda_fp16.h>
@@ -31,9 +34,9 @@
 namespace swp {
 namespace slices {
 
-constexpr int ND = 7;                       // digits
+constexpr int ND = 8;                       // digits
 constexpr int NL = 8;                       // levels kept
-constexpr uint64_t BIAS = 0x0080808080808080ull;  // 128 in each digit
+constexpr uint64_t BIAS = 0x8080808080808080ull;  // 128 in each digit
 constexpr float ACC0 = 12582912.0f;         // 1.5 * 2^23
 constexpr int ACC0_BITS = 0x4B400000;
 constexpr int ER_BAD = 4000;                // row exponent of a row with an infinity or a NaN
@@ -42,24 +45,24 @@ constexpr int KFLUSH = 2;                   // mma k-steps (of 16) per flush of 
 
 __device__ __forceinline__ int expo(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
 // A row's exponent from the maximum of expo over it; a row below 2^-959 counts as zero.
-__device__ __forceinline__ int row_exponent(int emax) { return emax == 0x7ff ? ER_BAD : emax < 64 ? ER_ZERO : emax; }
+__device__ __forceinline__ int row_exponent(int emax) { return emax >= 0x7ff ? ER_BAD : emax < 64 ? ER_ZERO : emax; }
 
-// Biased fixed point of x on its row's scale, truncated: byte 6 - u is digit u
-// plus 128.  Elements below the scale's unit, and all of a zero or bad row, give 0.
+// Biased fixed point of x on its row's scale, rounded: byte 7 - u is digit u plus
+// 128.  Elements below half the scale's unit, and all of a zero or bad row, give 0.
 __device__ __forceinline__ uint64_t fixed(double x, int er) {
   const uint32_t h = (uint32_t)__double2hiint(x), l = (uint32_t)__double2loint(x);
   const uint32_t sh = min((uint32_t)(er - (int)((h >> 20) & 0x7ff)), 63u);
-  const uint32_t m1 = __funnelshift_l(l, (h & 0xfffffu) | 0x100000u, 1), m0 = l << 1;  // significand, 54 bits
+  const uint32_t m1 = __funnelshift_l(l, (h & 0xfffffu) | 0x100000u, 10), m0 = l << 10;  // significand, one bit too many
   const uint32_t a1 = __funnelshift_rc(m1, 0u, sh), a0 = __funnelshift_rc(m0, m1, sh);
   const uint32_t b0 = __funnelshift_rc(m1, 0u, sh - 32u);
-  const uint64_t q = sh < 32u ? ((uint64_t)a1 << 32) | a0 : (uint64_t)b0;
+  const uint64_t q = ((sh < 32u ? ((uint64_t)a1 << 32) | a0 : (uint64_t)b0) + 1) >> 1;
   return (h >> 31) ? BIAS - q : BIAS + q;
 }
 
 // Digit u of two elements as an FP16 pair.
 template <int U>
 __device__ __forceinline__ uint32_t digit_pair(uint64_t a, uint64_t b) {
-  constexpr int i = 6 - U;
+  constexpr int i = 7 - U;
   const uint32_t wa = i < 4 ? (uint32_t)a : (uint32_t)(a >> 32), wb = i < 4 ? (uint32_t)b : (uint32_t)(b >> 32);
   // bytes (a, any, b, any), then the upper byte of each half set to 0x64: 1024 + byte, exact in FP16
   const uint32_t p = __byte_perm(wa, wb, (uint32_t)((i & 3) | ((4 + (i & 3)) << 8)));
@@ -67,7 +70,7 @@ __device__ __forceinline__ uint32_t digit_pair(uint64_t a, uint64_t b) {
   const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&h), __floats2half2_rn(1152.0f, 1152.0f));
   return *reinterpret_cast<const uint32_t*>(&v);
 }
-// Digits of two elements adjacent along K: out[u * stride], u = 0..6.
+// Digits of two elements adjacent along K: out[u * stride], u = 0..7.
 __device__ __forceinline__ void store_digits(uint32_t* out, int stride, uint64_t a, uint64_t b) {
   out[0] = digit_pair<0>(a, b);
   out[stride] = digit_pair<1>(a, b);
@@ -76,6 +79,7 @@ __device__ __forceinline__ void store_digits(uint32_t* out, int stride, uint64_t
   out[4 * stride] = digit_pair<4>(a, b);
   out[5 * stride] = digit_pair<5>(a, b);
   out[6 * stride] = digit_pair<6>(a, b);
+  out[7 * stride] = digit_pair<7>(a, b);
 }
 
 __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
@@ -140,13 +144,14 @@ __device__ __forceinline__ double value(long long hi, long long lo, int era, int
   return h + l;
 }
 
-// The B fragment of one k-step from digit planes in shared memory: `p` points
-// at (row of this lane's column, k) of digit 0, words of two elements.
-__device__ __forceinline__ void load_b(uint32_t (&b)[ND][2], const uint32_t* p, int plane) {
+// The B fragment of one k-step from digit planes in shared memory (words of two
+// elements): p0 and p1 point at this lane's words of digit 0, k = 2 t and 2 t + 8
+// of its column's row.
+__device__ __forceinline__ void load_b(uint32_t (&b)[ND][2], const uint32_t* p0, const uint32_t* p1, int plane) {
 #pragma unroll
   for (int v = 0; v < ND; ++v) {
-    b[v][0] = p[v * plane];
-    b[v][1] = p[v * plane + 4];
+    b[v][0] = p0[v * plane];
+    b[v][1] = p1[v * plane];
   }
 }
 // The A fragment of one k-step from a packed static operand (pack_a):

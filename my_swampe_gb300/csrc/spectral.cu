@@ -894,7 +894,6 @@ cudaError_t launch_spec_adj(const SpecLaunch<T>& L, int nblocks, size_t smem, cu
   cudaError_t e = launch_pdl(k_spectral_adj<T>, grid, 256, smem, s, std::is_same<T, float>::value, L);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
-template cudaError_t launch_spec_adj<double>(const SpecLaunch<double>&, int, size_t, cudaStream_t);
 template cudaError_t launch_spec_adj<float>(const SpecLaunch<float>&, int, size_t, cudaStream_t);
 
 // Programmatic dependent launch of the FP32 step kernels, unless SWP_PDL=0.
@@ -909,7 +908,6 @@ bool pdl_enabled() {
 void spec_set_attributes() {
   cudaFuncSetAttribute(k_spectral<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEC_DYN_SMEM_MAX);
   cudaFuncSetAttribute(k_spectral<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEC_DYN_SMEM_MAX);
-  cudaFuncSetAttribute(k_spectral_adj<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEC_DYN_SMEM_MAX);
   cudaFuncSetAttribute(k_spectral_adj<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEC_DYN_SMEM_MAX);
 }
 
