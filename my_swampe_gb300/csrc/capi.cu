@@ -33,9 +33,9 @@ struct swp_plan {
   bool tc[MAXG] = {};
   float* tcbasis[MAXG] = {};
   float* tcbasis_adj[MAXG] = {};
-  // FP64 Legendre kernels on integer slices (spectral_f64.cu): packed basis of
-  // the step and of its transpose
-  SliceBasis slices = {}, slices_adj = {};
+  // FP64 step kernels on integer slices: packed Legendre basis of the step and of
+  // its transpose (spectral_f64.cu), longitude transforms (grid_f64.cu)
+  SliceBasis slices = {}, slices_adj = {}, slices_grid = {};
   void* coefmem[MAXG] = {};              // per-call coefficient tables (CoefTables) of each group
   int* d_err = nullptr;                  // device error word set by bounded waits that ran out
   SchedCounter* d_sched = nullptr;       // persistent-launch counters: one per group chain, one for joint launches
@@ -314,6 +314,22 @@ cudaError_t launch_step_spec_adj(const swp_plan* p, const SpecLaunch<T>& LS, int
   }
 }
 
+// A grid launch (LG.mode): FFTs in FP32; in FP64 the sliced transforms for the
+// step, its adjoint and the output, the FFTs for the other modes.  The residual
+// of initial fields is formed with the transform that the outputs use.
+template <typename T>
+cudaError_t launch_any_grid(const swp_plan* p, const GridLaunch<T>& LG, int nbg, cudaStream_t s) {
+  if constexpr (std::is_same<T, double>::value) {
+    if (LG.mode == GM_STEP || LG.mode == GM_ADJ_STEP || LG.mode == GM_OUTPUT)
+      return launch_grid_f64(LG, p->slices_grid, s);
+    cudaError_t e = launch_grid<T>(LG, nbg, p->grid_smem[LG.mode], s);
+    if (e == cudaSuccess && (LG.mode == GM_INIT || LG.mode == GM_TL_INIT)) e = launch_grid_f64(LG, p->slices_grid, s);
+    return e;
+  } else {
+    return launch_grid<T>(LG, nbg, p->grid_smem[LG.mode], s);
+  }
+}
+
 // Launch nsteps steps.  In place on st[g].fourier, or -- when `slots` is given --
 // out of place: step k reads slot k and writes slot k+1 (slot stride `sstride`
 // complex elements), which keeps every intermediate state of a window.
@@ -353,7 +369,7 @@ int forward_steps(swp_plan* p, const swp_group_state* st, const swp_flags* f, in
     }
     cudaError_t e = launch_step_spec<T>(p, LS, nbs, s);
     if (e != cudaSuccess) return cuda_check(p, e, "spectral kernel launch");
-    e = launch_grid<T>(LG, nbg, p->grid_smem[GM_STEP], s);
+    e = launch_any_grid<T>(p, LG, nbg, s);
     if (e != cudaSuccess) return cuda_check(p, e, "grid kernel launch");
   }
   return SWP_OK;
@@ -502,7 +518,7 @@ int tangent_init_impl(swp_plan* p, const swp_group_state* st, const swp_group_ta
     LG.grp[g].phys_p = (const T*)phys[g];
     LG.grp[g].dpar = tan[g].dparams;
   }
-  return cuda_check(p, launch_grid<T>(LG, nbg, p->grid_smem[GM_TL_INIT], s), "tangent init launch");
+  return cuda_check(p, launch_any_grid<T>(p, LG, nbg, s), "tangent init launch");
 }
 
 // One window of primal + tangent steps.  Per step: the tangent Legendre step
@@ -562,7 +578,7 @@ int tangent_steps(swp_plan* p, const swp_group_state* st, const swp_group_tangen
     if (e != cudaSuccess) return cuda_check(p, e, "tangent spectral kernel launch");
     e = launch_step_spec<T>(p, LS, nbs, s);
     if (e != cudaSuccess) return cuda_check(p, e, "spectral kernel launch");
-    e = launch_grid<T>(LG, nbg, p->grid_smem[GM_STEP], s);
+    e = launch_any_grid<T>(p, LG, nbg, s);
     if (e != cudaSuccess) return cuda_check(p, e, "grid kernel launch");
     e = launch_grid<T>(LGT, nbg, p->grid_smem[GM_TL_STEP], s);
     if (e != cudaSuccess) return cuda_check(p, e, "tangent grid kernel launch");
@@ -594,7 +610,7 @@ int init_impl(swp_plan* p, const swp_group_state* st, void* const* phys, const s
   LG.mode = GM_INIT;
   LG.cfg = make_cfg(f);
   for (int g = 0; g < p->ng; ++g) LG.grp[g].phys_in = (const T*)phys[g];
-  return cuda_check(p, launch_grid<T>(LG, nbg, p->grid_smem[GM_INIT], s), "init kernel launch");
+  return cuda_check(p, launch_any_grid<T>(p, LG, nbg, s), "init kernel launch");
 }
 
 template <typename T>
@@ -613,7 +629,7 @@ int output_impl(swp_plan* p, const swp_group_state* st, void* const* out, const 
       LG.grp[g].dw = tan[g].dweights;
     }
   }
-  return cuda_check(p, launch_grid<T>(LG, nbg, p->grid_smem[GM_OUTPUT], s), "output kernel launch");
+  return cuda_check(p, launch_any_grid<T>(p, LG, nbg, s), "output kernel launch");
 }
 
 template <typename T>
@@ -664,7 +680,7 @@ int adjoint_step_impl(swp_plan* p, const swp_group_state* st_in, const swp_group
     LG.grp[g].grad = adj[g].grad;
     LG.grp[g].member = nullptr;
   }
-  cudaError_t e = launch_grid<T>(LG, nbg, p->grid_smem[GM_ADJ_STEP], s);
+  cudaError_t e = launch_any_grid<T>(p, LG, nbg, s);
   if (e != cudaSuccess) return cuda_check(p, e, "grid adjoint launch");
   SpecLaunch<T> LS = make_spec<T>(p, st_in, nbs);
   LS.mode = 0;
@@ -801,10 +817,10 @@ int time_kernels_impl(swp_plan* p, const swp_group_state* st, const swp_group_ad
     cudaEventRecord(ev[0], s);
     le[0] = launch_step_spec<T>(p, LS, nbs, s);
     cudaEventRecord(ev[1], s);
-    le[1] = launch_grid<T>(LG, nbg, p->grid_smem[GM_STEP], s);
+    le[1] = launch_any_grid<T>(p, LG, nbg, s);
     cudaEventRecord(ev[2], s);
     if (adj) {
-      le[2] = launch_grid<T>(LGa, nbg, p->grid_smem[GM_ADJ_STEP], s);
+      le[2] = launch_any_grid<T>(p, LGa, nbg, s);
       cudaEventRecord(ev[3], s);
       le[3] = launch_step_spec_adj<T>(p, LSa, nbs, s);
       cudaEventRecord(ev[4], s);
@@ -1101,6 +1117,7 @@ int swp_plan_create(int ngroups, const int* M, const int* B, int precision, swp_
   p->graphs_enabled = !(ng_env && ng_env[0] == '1');
   spec_set_attributes();
   spec_f64_set_attributes();
+  grid_f64_set_attributes();
   grid_set_attributes();
   spec_tc_set_attributes();
   cudaStream_t s = 0;
@@ -1176,11 +1193,14 @@ int swp_plan_create(int ngroups, const int* M, const int* B, int precision, swp_
   }
   if (precision == SWP_FP64) {
     for (int g = 0; g < ngroups; ++g) {
-      void *fwd = nullptr, *adj = nullptr;
+      void *fwd = nullptr, *adj = nullptr, *grid = nullptr;
       cudaError_t e = cudaMalloc(&fwd, spec_f64_basis_bytes(M[g]));
       p->slices.p[g] = fwd;
       if (e == cudaSuccess) e = cudaMalloc(&adj, spec_f64_basis_bytes(M[g]));
       p->slices_adj.p[g] = adj;
+      if (e == cudaSuccess) e = cudaMalloc(&grid, grid_f64_basis_bytes(M[g]));
+      p->slices_grid.p[g] = grid;
+      if (e == cudaSuccess) e = pack_grid_f64(M[g], grid, s);
       if (e == cudaSuccess) e = pack_spec_f64(p->geom[g], false, fwd, s);
       if (e == cudaSuccess) e = pack_spec_f64(p->geom[g], true, adj, s);
       if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -1212,6 +1232,7 @@ int swp_plan_destroy(swp_plan* p) {
     if (p->tcbasis_adj[g]) cudaFree(p->tcbasis_adj[g]);
     if (p->slices.p[g]) cudaFree(const_cast<void*>(p->slices.p[g]));
     if (p->slices_adj.p[g]) cudaFree(const_cast<void*>(p->slices_adj.p[g]));
+    if (p->slices_grid.p[g]) cudaFree(const_cast<void*>(p->slices_grid.p[g]));
     if (p->coefmem[g]) cudaFree(p->coefmem[g]);
   }
   if (p->d_err) cudaFree(p->d_err);

@@ -610,17 +610,20 @@ __device__ __forceinline__ void grid_body(const GridLaunch<T>& Lc, const GridGro
       other[(f * JB + r) * n1 + k] = v;  // staged layout of build_c2r
     }
     __syncthreads();
-    // band-limited reconstruction -> residual = x - C2R(trunc FFT(x))
-    T2* zr = c2r_transform<T>(c, other, nf, res);
-    for (int t = threadIdx.x; t < nf * JB * L; t += blockDim.x) {
-      int n = t % L, fr = t / L, r = fr % JB, f = fr / JB;
-      size_t po = f * PS + ((size_t)b * J + j0 + r) * I + 2 * n;
-      const T* x = G.phys_in + po;
-      T2 z = zr[(size_t)fr * LS + n];
-      G.resid[po] = x[0] - z.x;
-      G.resid[po + 1] = x[1] - z.y;
+    // band-limited reconstruction -> residual = x - C2R(trunc FFT(x)); in FP64
+    // grid_f64.cu forms it, with the transform of its outputs
+    if constexpr (sizeof(T) == 4) {
+      T2* zr = c2r_transform<T>(c, other, nf, res);
+      for (int t = threadIdx.x; t < nf * JB * L; t += blockDim.x) {
+        int n = t % L, fr = t / L, r = fr % JB, f = fr / JB;
+        size_t po = f * PS + ((size_t)b * J + j0 + r) * I + 2 * n;
+        const T* x = G.phys_in + po;
+        T2 z = zr[(size_t)fr * LS + n];
+        G.resid[po] = x[0] - z.x;
+        G.resid[po + 1] = x[1] - z.y;
+      }
+      __syncthreads();
     }
-    __syncthreads();
     // batch 2: nonlinear terms and forcing from the raw initial grids (model.py:723-732)
     double lrms = 0.0, lspin = 1e300;
     const int nout = ph.forced ? 8 : 5;
@@ -886,11 +889,11 @@ static void set_attr_one() {
 }
 
 void grid_set_attributes() {
-  set_attr_one<double, GM_STEP>(); set_attr_one<float, GM_STEP>();
+  set_attr_one<float, GM_STEP>();
   set_attr_one<double, GM_INIT>(); set_attr_one<float, GM_INIT>();
-  set_attr_one<double, GM_OUTPUT>(); set_attr_one<float, GM_OUTPUT>();
+  set_attr_one<float, GM_OUTPUT>();
   set_attr_one<double, GM_WINDS>(); set_attr_one<float, GM_WINDS>();
-  set_attr_one<double, GM_ADJ_STEP>(); set_attr_one<float, GM_ADJ_STEP>();
+  set_attr_one<float, GM_ADJ_STEP>();
   set_attr_one<double, GM_ADJ_INIT>(); set_attr_one<float, GM_ADJ_INIT>();
   set_attr_one<double, GM_ADJ_OUTPUT>(); set_attr_one<float, GM_ADJ_OUTPUT>();
   set_attr_one<double, GM_FWD2>(); set_attr_one<float, GM_FWD2>();
@@ -914,12 +917,15 @@ cudaError_t launch_grid(const GridLaunch<T>& L0, int nblocks0, size_t smem, cuda
   L.prefix[L.ng] = nblocks;
   cudaError_t e = cudaSuccess;
   constexpr bool f32 = std::is_same<T, float>::value;
+  if constexpr (f32) {  // in FP64 these modes are grid_f64.cu's
+    if (L.mode == GM_OUTPUT) e = launch_pdl(k_grid<T, GM_OUTPUT>, nblocks, 256, smem, s, true, L);
+    if (L.mode == GM_STEP) e = launch_pdl(k_grid<T, GM_STEP>, nblocks, 256, smem, s, true, L);
+    if (L.mode == GM_ADJ_STEP) e = launch_pdl(k_grid<T, GM_ADJ_STEP>, nblocks, 256, smem, s, true, L);
+    if (L.mode == GM_STEP || L.mode == GM_ADJ_STEP || L.mode == GM_OUTPUT) return e != cudaSuccess ? e : cudaGetLastError();
+  }
   switch (L.mode) {
-    case GM_STEP: e = launch_pdl(k_grid<T, GM_STEP>, nblocks, 256, smem, s, f32, L); break;
     case GM_INIT: e = launch_pdl(k_grid<T, GM_INIT>, nblocks, 256, smem, s, f32, L); break;
-    case GM_OUTPUT: e = launch_pdl(k_grid<T, GM_OUTPUT>, nblocks, 256, smem, s, f32, L); break;
     case GM_WINDS: e = launch_pdl(k_grid<T, GM_WINDS>, nblocks, 256, smem, s, f32, L); break;
-    case GM_ADJ_STEP: e = launch_pdl(k_grid<T, GM_ADJ_STEP>, nblocks, 256, smem, s, f32, L); break;
     case GM_ADJ_INIT: e = launch_pdl(k_grid<T, GM_ADJ_INIT>, nblocks, 256, smem, s, f32, L); break;
     case GM_ADJ_OUTPUT: e = launch_pdl(k_grid<T, GM_ADJ_OUTPUT>, nblocks, 256, smem, s, f32, L); break;
     case GM_FWD2: e = launch_pdl(k_grid<T, GM_FWD2>, nblocks, 256, smem, s, f32, L); break;

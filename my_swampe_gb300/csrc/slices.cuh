@@ -82,6 +82,17 @@ __device__ __forceinline__ void store_digits(uint32_t* out, int stride, uint64_t
   out[7 * stride] = digit_pair<7>(a, b);
 }
 
+// Exchange between the lanes of a pair (l, l ^ 1): each lane holds elements of
+// two rows at its own position; the even lane leaves with row a's pair, the odd
+// lane with row b's.
+__device__ __forceinline__ void pair_exchange(uint64_t& a, uint64_t& b) {
+  const bool odd = threadIdx.x & 1;
+  const uint64_t mine = odd ? b : a, give = odd ? a : b;
+  const uint64_t got = __shfl_xor_sync(0xffffffffu, give, 1);
+  a = odd ? got : mine;  // element at the even position
+  b = odd ? mine : got;
+}
+
 __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"

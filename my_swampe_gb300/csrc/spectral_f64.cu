@@ -166,17 +166,6 @@ struct Mem {
   static constexpr size_t total = A + B + E;
 };
 
-// Exchange between the lanes of a pair (l, l ^ 1): each lane holds elements of
-// two rows at its own position; the even lane leaves with row a's pair, the odd
-// lane with row b's.
-__device__ __forceinline__ void pair_exchange(uint64_t& a, uint64_t& b) {
-  const bool odd = threadIdx.x & 1;
-  const uint64_t mine = odd ? b : a, give = odd ? a : b;
-  const uint64_t got = __shfl_xor_sync(0xffffffffu, give, 1);
-  a = odd ? got : mine;  // element at the even position
-  b = odd ? mine : got;
-}
-
 // Symmetric (s = 0) and antisymmetric (s = 1) parts of the raw rows over the
 // southern latitudes j' (plus / minus their mirror), times 2^ep[j'], sliced on
 // their own scales.
@@ -698,7 +687,7 @@ cudaError_t launch_one(SpecLaunch<double> L, const SliceBasis& basis, cudaStream
   L.prefix[L.ng] = acc;
   if (acc == 0) return cudaSuccess;
   typedef Sh<M_> S;
-  if (ADJ) {
+  if constexpr (ADJ) {
     constexpr size_t smem = Mem<S, MT, 5, 7, 5, 9>::total;
     k_spectral_adj_f64<M_, MT><<<acc, 256, smem, s>>>(L, basis);
   } else {

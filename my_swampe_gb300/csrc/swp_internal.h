@@ -268,13 +268,18 @@ constexpr int SPEC_DYN_SMEM_MAX = 227 * 1024 - 128;
 void grid_set_attributes();
 int grid_rows_per_cta(int M, bool fp64, int mode);  // JB the grid kernel is compiled for
 
-// FP64 Legendre kernels on integer slices (spectral_f64.cu): packed basis of each group
+// FP64 step kernels on integer slices (spectral_f64.cu, grid_f64.cu): packed
+// static matrices of each group
 struct SliceBasis {
   const void* p[MAXG];
 };
 size_t spec_f64_basis_bytes(int M);
 cudaError_t pack_spec_f64(const GroupGeom& gg, bool adjoint, void* out, cudaStream_t s);
 void spec_f64_set_attributes();
+size_t grid_f64_basis_bytes(int M);
+cudaError_t pack_grid_f64(int M, void* out, cudaStream_t s);
+void grid_f64_set_attributes();
+cudaError_t launch_grid_f64(const GridLaunch<double>& L, const SliceBasis& basis, cudaStream_t s);
 cudaError_t launch_spec_f64(const SpecLaunch<double>& L, const SliceBasis& basis, bool adjoint, cudaStream_t s);
 
 // tensor-core Legendre kernels of the FP32 modified-Euler step and its adjoint
