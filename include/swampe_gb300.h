@@ -127,6 +127,15 @@ int swp_plan_destroy(swp_plan* plan);
 int swp_plan_dims(const swp_plan* plan, int g, int* M, int* J, int* I, int* B);
 /* Message of the last failure on this plan (empty string if none). */
 const char* swp_last_error(const swp_plan* plan);
+/* Tables of the reference's Static that depend on the parameters
+ * (model.py:457-557) of a group's truncation, for n members, in one launch.
+ * params: device double [10][n], rows dt, a, omega, g, Phibar, taurad, taudrag,
+ * DPhieq, K6, K6Phi.
+ * out: device double, consecutively a / (n(n+1)) [n][N+1]; sigma, sigmaPhi and
+ * their exponential forms, each [n][N+1]; tstepcoeff [n][J]; 2 dt / a^2 [n];
+ * the planetary vorticity [n][M+1][N+1]; Phieq [n][J][I] (zero unless forced). */
+int swp_static_tables(swp_plan* plan, int group, const double* params, int n, int forced, double* out, void* stream);
+
 /* FP64 copies of mus, w (J each) and dense Pmn, Hmn (J, M+1, M+1) for group g
  * (spectral_transform.py:80-114, 219-287).  Any pointer may be NULL. */
 int swp_geometry(const swp_plan* plan, int g, double* mus, double* w, double* Pmn, double* Hmn, void* stream);

@@ -113,7 +113,7 @@ EXPORTS = (
     "swp_adjoint_stored", "swp_plan_autotune", "swp_plan_tiles", "swp_plan_set_tile",
     "swp_tangent_init", "swp_tangent_forward", "swp_tangent_output", "swp_plan_set_concurrency",
     "swp_plan_set_wait_limit", "swp_emission_map", "swp_emission_project", "swp_phase_curve_linear",
-    "swp_phase_curve_simple",
+    "swp_phase_curve_simple", "swp_static_tables",
 )
 
 _lib = None
@@ -172,6 +172,7 @@ def load(path: os.PathLike | str | None = None) -> ctypes.CDLL:
         "swp_emission_project": (i, [vp, vp, i, i, vp, i, vp, vp]),
         "swp_phase_curve_linear": (i, [vp, vp, vp, i, i, i, vp, vp]),
         "swp_phase_curve_simple": (i, [vp, i, i, i, vp, vp, i, vp, vp]),
+        "swp_static_tables": (i, [vp, i, vp, i, i, vp, vp]),
     }
     for name, (res, args) in sig.items():
         fn = getattr(lib, name)

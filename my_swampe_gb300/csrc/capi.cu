@@ -1271,6 +1271,12 @@ int swp_plan_dims(const swp_plan* p, int g, int* M, int* J, int* I, int* B) {
 
 const char* swp_last_error(const swp_plan* p) { return p ? p->err.c_str() : "null plan"; }
 
+int swp_static_tables(swp_plan* p, int g, const double* params, int n, int forced, double* out, void* stream) {
+  if (!p || g < 0 || g >= p->ng || !params || !out || n < 1) return SWP_ERR_ARG;
+  return cuda_check(p, launch_static_tables(p->geom[g], params, n, forced, out, (cudaStream_t)stream),
+                    "static tables launch");
+}
+
 int swp_geometry(const swp_plan* p, int g, double* mus, double* w, double* Pmn, double* Hmn, void* stream) {
   if (!p || g < 0 || g >= p->ng) return SWP_ERR_ARG;
   swp_plan* q = const_cast<swp_plan*>(p);

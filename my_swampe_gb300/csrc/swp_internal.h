@@ -70,6 +70,8 @@ template <> inline Geom<float> GroupGeom::view<float>() const {
 }
 
 int geometry_build(GroupGeom& gg, int M, cudaStream_t stream, std::string& err);
+cudaError_t launch_static_tables(const GroupGeom& gg, const double* params, int n, int forced, double* out,
+                                 cudaStream_t s);
 int geometry_dense(const GroupGeom& gg, double* Pd, double* Hd, cudaStream_t stream);
 
 constexpr int MAXG = 4;

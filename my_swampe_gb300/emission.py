@@ -107,6 +107,8 @@ def _ensemble(x, name: str) -> Tuple[torch.Tensor, bool]:
 
 
 def _per_member(x, B: int, dev) -> torch.Tensor:
+    if isinstance(x, (int, float)):  # a fill, not a copy from the host, which would wait for the stream
+        return torch.full((B,), float(x), dtype=torch.float64, device=dev)
     return torch.as_tensor(x, dtype=torch.float64, device=dev).reshape(-1).expand(B).contiguous()
 
 

@@ -17,6 +17,7 @@ the model runs in the library's CUDA kernels.
 from __future__ import annotations
 
 import ctypes
+import math
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -53,6 +54,19 @@ class RunFlagsC:
             0 if self.test is None else int(self.test), int(bool(self.diagnostics)), float(self.blowup_rms),
             int(self.t_start), int(bool(self.raw_filter)),
         )
+
+
+def stack_values(vals: Sequence, device) -> torch.Tensor:
+    """Values (floats, 0-d or length-n tensors or sequences) as one float64
+    (len(vals), n) tensor, n = 1 if all are scalars; detached.  The floats cross
+    to the device in one copy."""
+    is_float = [isinstance(v, (int, float)) for v in vals]
+    floats = iter(torch.tensor([float(v) for v, f in zip(vals, is_float) if f], dtype=torch.float64,
+                               device=device).unbind(0)) if any(is_float) else iter(())
+    ts = [next(floats) if f else torch.as_tensor(v, dtype=torch.float64, device=device).detach()
+          for v, f in zip(vals, is_float)]
+    n = max([t.numel() for t in ts if t.dim()], default=1)
+    return torch.stack([t.expand(n) if t.dim() == 0 else t.reshape(n) for t in ts])
 
 
 def _require_cuda(device) -> torch.device:
@@ -209,17 +223,38 @@ class Engine:
         P = torch.empty((J, M + 1, M + 1), dtype=torch.float64, device=self.device)
         H = torch.empty_like(P)
         self._check(self.lib.swp_geometry(self._plan, g, mus.data_ptr(), w.data_ptr(), P.data_ptr(), H.data_ptr(), self.stream), "geometry")
-        out = dict(mus=mus, w=w, Pmn=P, Hmn=H)
+        n = torch.arange(M + 1, dtype=torch.float64, device=self.device)
+        # constants of the grid that Static carries (model.build_static)
+        out = dict(mus=mus, w=w, Pmn=P, Hmn=H, Pmnw=w[:, None, None] * P, Hmnw=w[:, None, None] * H,
+                   lambdas=torch.linspace(-math.pi, math.pi, gd["I"] + 1, dtype=torch.float64, device=self.device)[:-1],
+                   m=n, nn1=n * (n + 1))
         self._geo_cache[g] = out
         return out
+
+    def static_tables(self, g: int, vals: torch.Tensor, forced: bool) -> Dict[str, torch.Tensor]:
+        """Tables of model.Static that depend on the parameters, in one launch.
+        vals: float64 (10, n) rows dt, a, omega, g, Phibar, taurad, taudrag, DPhieq,
+        K6, K6Phi.  Views of one buffer, member axis first."""
+        gd = self.groups[g]
+        N1, J, I, n = gd["M"] + 1, gd["J"], gd["I"], vals.shape[1]
+        shapes = dict(tc=(N1,), sigma=(N1,), sigmaPhi=(N1,), sigma_exp=(N1,), sigmaPhi_exp=(N1,), tsc=(J,), tsc2=(1,),
+                      fmn=(N1, N1), Phieq=(J, I))
+        sizes = [n * math.prod(s) for s in shapes.values()]
+        buf = torch.empty(sum(sizes), dtype=torch.float64, device=self.device)
+        self._check(self.lib.swp_static_tables(self._plan, g, vals.contiguous().data_ptr(), n, int(forced),
+                                               buf.data_ptr(), self.stream), "static_tables")
+        return {k: x.view(n, *s) for (k, s), x in zip(shapes.items(), buf.split(sizes))}
 
     # ------------------------------------------------------------ parameters
     def set_params(self, g: int, **kw) -> None:
         """Set per-member scalars (float or length-B tensor) of group g."""
         gd = self.groups[g]
+        # values only: a parameter's gradient or tangent flows through adjoint.integrate
+        if len(kw) == len(PARAM_NAMES):  # all of them: one launch instead of one per parameter
+            gd["params"].copy_(stack_values([kw[k] for k in PARAM_NAMES], self.device).expand(-1, gd["B"]))
+            return
         for name, v in kw.items():
             row = PARAM_NAMES.index(name)
-            # values only: a parameter's gradient or tangent flows through adjoint.integrate
             t = torch.as_tensor(v, dtype=torch.float64, device=self.device).detach()
             gd["params"][row].copy_(t.expand(gd["B"]) if t.dim() == 0 else t.reshape(gd["B"]))
 
@@ -246,9 +281,8 @@ class Engine:
             keep.append(x)
             ptrs.append(x.data_ptr())
             gd["fourier"].zero_()
-            gd["member"].zero_()
-            gd["member"][_lib.MS_WCURR] = 1.0
-            gd["member"][_lib.MS_WMID] = 1.0
+            gd["member"][:2].fill_(1.0)  # MS_WCURR, MS_WMID
+            gd["member"][2:].zero_()
         self._check(self.lib.swp_init_state(self._plan, self._states(diag=diag), _lib.ptr_array(ptrs), ctypes.byref(flags.c()), self.stream), "init_state")
         self._ic_keep = keep
 

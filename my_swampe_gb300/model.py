@@ -25,7 +25,7 @@ import torch
 import torch.autograd.forward_ad as fwAD
 
 from . import _lib, continuation
-from .engine import Engine, RunFlagsC
+from .engine import PARAM_NAMES, Engine, RunFlagsC, stack_values
 
 _SUPPORTED_M = {42: (64, 128, 1200), 63: (96, 192, 900), 106: (160, 320, 600)}
 
@@ -213,18 +213,33 @@ def build_static(*, M, dt, a, omega, g, Phibar, taurad, taudrag, DPhieq, K6, K6P
     M = int(M)
     N = M
     J, I, _ = _SUPPORTED_M[M]
-    mus, w, Pmn, Hmn = geo["mus"], geo["w"], geo["Pmn"], geo["Hmn"]
-    lambdas = torch.linspace(-math.pi, math.pi, I + 1, dtype=torch.float64, device=dev)[:-1]
-    vals = [_scalar_tensor(v, dev) for v in (dt, a, omega, g, Phibar, taurad, taudrag, DPhieq, K6,
-                                             K6 if K6Phi is None else K6Phi)]
+    mus, Pmn, Hmn, lambdas = geo["mus"], geo["Pmn"], geo["Hmn"], geo["lambdas"]
+    const = dict(M=M, N=N, I=I, J=J, lambdas=lambdas, mus=mus, w=geo["w"], Pmn=Pmn, Hmn=Hmn, Pmnw=geo["Pmnw"],
+                 Hmnw=geo["Hmnw"], marray=geo["m"][:, None].expand(M + 1, N + 1),
+                 mJarray=geo["m"][None, :].expand(J, M + 1), narray=geo["nn1"][None, :].expand(M + 1, N + 1), test=test)
+    given = dict(dt=dt, a=a, omega=omega, g=g, Phibar=Phibar, taurad=taurad, taudrag=taudrag, DPhieq=DPhieq, K6=K6,
+                 K6Phi=K6 if K6Phi is None else K6Phi)
+    if not any(_tracked(v) for v in given.values()):
+        v = stack_values(list(given.values()), dev)
+        t = eng.static_tables(0, v, test is None)
+        one = not any(torch.is_tensor(x) and x.dim() or np.ndim(x) for x in given.values())
+        if one:  # scalars: no member axis
+            t = {k: x[0] for k, x in t.items()}
+        row = lambda x: x[..., None, :].expand(*x.shape[:-1], M + 1, N + 1)  # noqa: E731
+        return Static(**const, **{k: x[0] if one else x for k, x in zip(given, v)}, fmn=t["fmn"],
+                      tstepcoeff=t["tsc"][..., None].expand(*t["tsc"].shape, M + 1),
+                      tstepcoeff2=t["tsc2"][..., None].expand(*t["tsc2"].shape[:-1], J, M + 1),
+                      tstepcoeffmn=row(t["tc"]), sigma=row(t["sigma"]), sigmaPhi=row(t["sigmaPhi"]),
+                      sigma_exp=row(t["sigma_exp"]), sigmaPhi_exp=row(t["sigmaPhi_exp"]),
+                      # unforced: zero, without a member axis
+                      Phieq=t["Phieq"] if one or test is None else t["Phieq"][0])
+    # tracked parameters: tensor expressions, which carry their derivatives
+    vals = [_scalar_tensor(v, dev) for v in given.values()]
     if any(v.dim() for v in vals):  # ensemble: broadcast every scalar to the member axis
         Bn = max(v.shape[0] for v in vals if v.dim())
         vals = [v.expand(Bn) if v.dim() == 0 else v for v in vals]
     dt_, a_, om_, g_, Pb_, tr_, td_, DP, K6_, K6P = vals
-    n = torch.arange(N + 1, dtype=torch.float64, device=dev)
-    mm = torch.arange(M + 1, dtype=torch.float64, device=dev)
-    nn1 = n * (n + 1)
-    den = nn1.clone()
+    n, den = geo["m"], geo["nn1"].clone()
     den[0] = 1.0
     tcmn = a_[..., None, None] / den if a_.dim() else a_ / den
     tcmn = tcmn * (n > 0)
@@ -262,14 +277,10 @@ def build_static(*, M, dt, a, omega, g, Phibar, taurad, taudrag, DPhieq, K6, K6P
             Phieq = Pb_ + torch.where(day, DP * term_shape, 0.0)
     else:
         Phieq = torch.zeros((J, I), dtype=torch.float64, device=dev)
-    return Static(
-        M=M, N=N, I=I, J=J, dt=dt_, a=a_, omega=om_, g=g_, Phibar=Pb_, taurad=tr_, taudrag=td_,
-        lambdas=lambdas, mus=mus, w=w, Pmn=Pmn, Hmn=Hmn, Pmnw=w[:, None, None] * Pmn, Hmnw=w[:, None, None] * Hmn,
-        fmn=fmn, tstepcoeff=tsc, tstepcoeff2=tsc2, tstepcoeffmn=tcmn,
-        marray=mm[:, None].expand(M + 1, N + 1), mJarray=mm[None, :].expand(J, M + 1), narray=nn1[None, :].expand(M + 1, N + 1),
-        sigma=_sig(K6_, True, False), sigmaPhi=_sig(K6P, False, False), sigma_exp=_sig(K6_, True, True),
-        sigmaPhi_exp=_sig(K6P, False, True), Phieq=Phieq, DPhieq=DP, K6=K6_, K6Phi=K6P, test=test,
-    )
+    return Static(**const, dt=dt_, a=a_, omega=om_, g=g_, Phibar=Pb_, taurad=tr_, taudrag=td_, DPhieq=DP, K6=K6_,
+                  K6Phi=K6P, fmn=fmn, tstepcoeff=tsc, tstepcoeff2=tsc2, tstepcoeffmn=tcmn,
+                  sigma=_sig(K6_, True, False), sigmaPhi=_sig(K6P, False, False), sigma_exp=_sig(K6_, True, True),
+                  sigmaPhi_exp=_sig(K6P, False, True), Phieq=Phieq)
 
 
 def _analytic_ic(M, a, omega, Phibar, test, a1, dev):
@@ -566,7 +577,8 @@ def run_model_scan(
         phys, dcurr, last = _run_split(
             M, B, precision, device, flags, starttime_eff, T, ics=torch.stack((eta0, delta0, Phi0, U0, V0), 0),
             pvals=dict(dt=dt, a=a, omega=omega, Phibar=Phibar, taurad=taurad, taudrag=taudrag,
-                       DPhieq=DPhieq if test is None else 0.0, K6=K6, K6Phi=K6Phi_eff, alpha=alpha),
+                       DPhieq=DPhieq if test is None else 0.0, K6=K6, K6Phi=K6Phi_eff, alpha=alpha, si_alpha=si_alpha,
+                       williams_alpha=williams_alpha),
             needs_grad=needs_grad, coef_inputs=coef_inputs, zero_deriv=tuple(zero_deriv), batched=batched)
         return dict(static=static, t_seq=torch.arange(starttime_eff, tmax, dtype=torch.int32, device=dev),
                     last_state=last, starttime=starttime_eff)
@@ -652,15 +664,9 @@ def _run_split(M, B, precision, device, flags: RunFlagsC, t0: int, T: int, ics: 
     dev = eng.device
     sls = (slice(0, sizes[0]), slice(sizes[0], B))
 
-    def part(x, sl):
-        if torch.is_tensor(x) and x.dim() == 1:
-            return x[sl]
-        if not torch.is_tensor(x) and not _is_python_scalar(x) and np.ndim(x) == 1:
-            return torch.as_tensor(x, dtype=torch.float64)[sl]
-        return x
-
-    for g, sl in enumerate(sls):
-        eng.set_params(g, **{k: part(v, sl) for k, v in pvals.items()})
+    rows = stack_values([pvals[k] for k in PARAM_NAMES], dev)
+    for gd, sl in zip(eng.groups, sls):
+        gd["params"].copy_(rows[:, sl] if rows.shape[1] > 1 else rows.expand(-1, gd["B"]))
     ics_g = [ics[:, sl] for sl in sls]
     eng.init_state([x.detach() for x in ics_g], flags)
     # pass-through carries of the semi-implicit scheme's State fields: F + U / taudrag of the initial state
@@ -703,10 +709,12 @@ def _assemble_state(eng: Engine, phys: torch.Tensor, Rum, Rvm, batched: bool, fi
     """The State of the engine's groups, joined along the member axis in group
     order (one group, or the two halves of a split ensemble)."""
 
-    def fo(k):  # (M+1, B, J) -> (B, J, M+1), a copy (the engine's buffers are reused)
-        f = torch.cat([gd["fourier"][k] for gd in eng.groups], dim=1)
-        v = f.permute(1, 2, 0).clone(memory_format=torch.contiguous_format)
-        return v if batched else v[0]
+    # all Fourier fields (NFOURIER, M+1, B, J) -> (NFOURIER, B, J, M+1) in one copy (the engine's buffers are reused)
+    fs = [gd["fourier"].permute(0, 2, 3, 1) for gd in eng.groups]
+    four = fs[0].clone(memory_format=torch.contiguous_format) if len(fs) == 1 else torch.cat(fs, dim=1)
+
+    def fo(k):
+        return four[k] if batched else four[k, 0]
 
     def fr(t):
         v = t.permute(1, 2, 0).clone(memory_format=torch.contiguous_format)
@@ -850,18 +858,17 @@ def _load_state(eng: Engine, flags: "RunFlags", state0: State, test, t0: int, di
         mid = four[[_lib.F_ETA, _lib.F_DELTA, _lib.F_PHI]].clone()
         r_p = resid[:3].clone()
     eng.init_state([pc], _flags_c(flags, test, t0), diag=diag)
-    for name, slot in _STATE_SLOTS:
-        four[slot].copy_(fo(getattr(state0, name)))
     filtered = bool(flags.semi_implicit or flags.raw_filter)
-    for name, ps, ms in zip(_PREV_NAMES, _PREV_SLOTS, _MID_SLOTS):
-        v = fo(getattr(state0, name))
-        if filtered:
-            four[ms].copy_(v)   # the Fourier prev carry is the filtered lineage
-            four[ps].copy_(v)
-        else:
-            four[ps].copy_(v)
-            if mid is not None:
-                four[ms].copy_(mid[_MID_SLOTS.index(ms)])
+    # the 16 given fields in slot order, in one copy
+    by_slot = dict([(slot, name) for name, slot in _STATE_SLOTS] + list(zip(_PREV_SLOTS, _PREV_NAMES)))
+    x = [torch.as_tensor(getattr(state0, by_slot[k]), device=dev).detach().to(cdt) for k in range(len(by_slot))]
+    x = torch.stack(x if batched else [v[None] for v in x])  # (16, B, J, M+1)
+    four[:len(by_slot)].copy_(x.permute(0, 3, 1, 2))
+    for ps, ms in zip(_PREV_SLOTS, _MID_SLOTS):
+        if filtered:  # the Fourier prev carry is the filtered lineage
+            four[ms].copy_(four[ps])
+        elif mid is not None:
+            four[ms].copy_(mid[_MID_SLOTS.index(ms)])
     if flags.semi_implicit:  # the lagged remainders live in the unfiltered prev slots
         four[_lib.F_RU_LAG].copy_(fo(state0.Rum_lag))
         four[_lib.F_RV_LAG].copy_(fo(state0.Rvm_lag))
