@@ -850,30 +850,33 @@ __device__ __forceinline__ void grid_body(const GridLaunch<T>& Lc, const GridGro
 }
 
 // JB (latitude rows per CTA) of a truncation and mode: 8 where the mode's two
-// transform buffers stay within 72 KB (three or more CTAs per SM), else 4, or
-// 2 where even 4 rows would exceed 200 KB (the FP64 adjoint at M=106).
+// transform buffers stay within 72 KB (three or more CTAs per SM), else 4, or 2
+// where even 4 rows would exceed 200 KB, in FP32 100 KB (the adjoint at M = 106:
+// 2 rows leave three CTAs per SM instead of one; 21 members 72 -> 59 us).
 template <typename T>
 __host__ __device__ constexpr size_t grid_buf_bytes(int M, int mode, int jb) {
   return (size_t)2 * grid_ntr(mode) * jb * (trunc_I(M) / 2 + 1) * 2 * sizeof(T);
 }
 template <typename T>
 __host__ __device__ constexpr int grid_jb(int M, int mode) {
-  return grid_buf_bytes<T>(M, mode, 8) <= 72 * 1024 ? 8 : grid_buf_bytes<T>(M, mode, 4) <= 200 * 1024 ? 4 : 2;
+  return grid_buf_bytes<T>(M, mode, 8) <= 72 * 1024 ? 8 : grid_buf_bytes<T>(M, mode, 4) <= (sizeof(T) == 4 ? 100 : 200) * 1024 ? 4 : 2;
 }
+
+__host__ __device__ constexpr int cap_jb(int jb, int cap) { return jb < cap ? jb : cap; }
 
 // Resident CTAs per SM the register budget is sized for: FP32 adjoint 4 (its
 // 52 KB of shared memory allow 4), FP32 forward modes 3 (8 rows per CTA at
 // M=42 take 68 KB), FP64 2.
-template <typename T, int MODE>
+template <typename T, int MODE, int CAP = 8>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (MODE == GM_ADJ_STEP ? 4 : 3) : 2)
     k_grid(const __grid_constant__ GridLaunch<T> Lc) {
   pdl_enter();
   int idx;
   const GridGroup<T>& G = pick_ggroup(Lc, idx);
   switch (G.g.M) {  // groups of different truncations share one launch
-    case 42: grid_body<T, MODE, 42, grid_jb<T>(42, MODE)>(Lc, G, idx); break;
-    case 63: grid_body<T, MODE, 63, grid_jb<T>(63, MODE)>(Lc, G, idx); break;
-    default: grid_body<T, MODE, 106, grid_jb<T>(106, MODE)>(Lc, G, idx); break;
+    case 42: grid_body<T, MODE, 42, cap_jb(grid_jb<T>(42, MODE), CAP)>(Lc, G, idx); break;
+    case 63: grid_body<T, MODE, 63, cap_jb(grid_jb<T>(63, MODE), CAP)>(Lc, G, idx); break;
+    default: grid_body<T, MODE, 106, cap_jb(grid_jb<T>(106, MODE), CAP)>(Lc, G, idx); break;
   }
 }
 
@@ -881,15 +884,16 @@ int grid_rows_per_cta(int M, bool fp64, int mode) { return fp64 ? grid_jb<double
 
 // Largest dynamic shared memory the kernel may request: 227 KB per block minus
 // the kernel's static shared memory (the pointer tables of stage_rows / write_r2c).
-template <typename T, int MODE>
+template <typename T, int MODE, int CAP = 8>
 static void set_attr_one() {
   cudaFuncAttributes fa;
-  size_t stat = cudaFuncGetAttributes(&fa, k_grid<T, MODE>) == cudaSuccess ? fa.sharedSizeBytes : 1024;
-  cudaFuncSetAttribute(k_grid<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - stat));
+  size_t stat = cudaFuncGetAttributes(&fa, k_grid<T, MODE, CAP>) == cudaSuccess ? fa.sharedSizeBytes : 1024;
+  cudaFuncSetAttribute(k_grid<T, MODE, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - stat));
 }
 
 void grid_set_attributes() {
-  set_attr_one<float, GM_STEP>();
+  set_attr_one<float, GM_STEP>(); set_attr_one<float, GM_STEP, 4>(); set_attr_one<float, GM_STEP, 2>();
+  set_attr_one<float, GM_ADJ_STEP, 2>();
   set_attr_one<double, GM_INIT>(); set_attr_one<float, GM_INIT>();
   set_attr_one<float, GM_OUTPUT>();
   set_attr_one<double, GM_WINDS>(); set_attr_one<float, GM_WINDS>();
@@ -907,9 +911,25 @@ cudaError_t launch_grid(const GridLaunch<T>& L0, int nblocks0, size_t smem, cuda
   (void)nblocks0;
   GridLaunch<T> L = L0;
   int nblocks = 0;
+  // Few members: fewer rows per CTA while the launch would leave SMs idle (the
+  // CTAs then run one latency chain each).  M = 42, one member, step / adjoint:
+  // 12.5 / 11.3 us with 8 / 4 rows, 10.4 / 10.2 us with 2; 16 members 12.6 / 12.3
+  // us, with 2 rows 16.4 / 12.3 us.  Rows are independent: the bits stay.
+  int cap = 8;
+  if (std::is_same<T, float>::value && (L.mode == GM_STEP || L.mode == GM_ADJ_STEP)) {
+    int rows = 0;
+    for (int g = 0; g < L.ng; ++g) rows += L.grp[g].B * L.grp[g].g.J;
+    cap = rows <= (L.mode == GM_STEP ? 2 : 4) * 152 ? 2 : rows <= 4 * 152 ? 4 : 8;
+    smem = 0;
+    for (int g = 0; g < L.ng; ++g) {
+      const Geom<T>& q = L.grp[g].g;
+      const size_t need = grid_smem_bytes<T>(q.M, q.J, q.I, cap_jb(grid_jb<T>(q.M, L.mode), cap), L.mode);
+      if (L.grp[g].B > 0 && need > smem) smem = need;
+    }
+  }
   for (int g = 0; g < L.ng; ++g) {
     GridGroup<T>& G = L.grp[g];
-    G.JB = grid_jb<T>(G.g.M, L.mode);
+    G.JB = cap_jb(grid_jb<T>(G.g.M, L.mode), cap);
     G.njb = G.g.J / G.JB;
     L.prefix[g] = nblocks;
     nblocks += G.B * G.njb;
@@ -919,8 +939,11 @@ cudaError_t launch_grid(const GridLaunch<T>& L0, int nblocks0, size_t smem, cuda
   constexpr bool f32 = std::is_same<T, float>::value;
   if constexpr (f32) {  // in FP64 these modes are grid_f64.cu's
     if (L.mode == GM_OUTPUT) e = launch_pdl(k_grid<T, GM_OUTPUT>, nblocks, 256, smem, s, true, L);
-    if (L.mode == GM_STEP) e = launch_pdl(k_grid<T, GM_STEP>, nblocks, 256, smem, s, true, L);
-    if (L.mode == GM_ADJ_STEP) e = launch_pdl(k_grid<T, GM_ADJ_STEP>, nblocks, 256, smem, s, true, L);
+    auto capped = [&](auto k8, auto k4, auto k2) {
+      e = launch_pdl(cap == 8 ? k8 : cap == 4 ? k4 : k2, nblocks, 256, smem, s, true, L);
+    };
+    if (L.mode == GM_STEP) capped(k_grid<T, GM_STEP>, k_grid<T, GM_STEP, 4>, k_grid<T, GM_STEP, 2>);
+    if (L.mode == GM_ADJ_STEP) capped(k_grid<T, GM_ADJ_STEP>, k_grid<T, GM_ADJ_STEP>, k_grid<T, GM_ADJ_STEP, 2>);
     if (L.mode == GM_STEP || L.mode == GM_ADJ_STEP || L.mode == GM_OUTPUT) return e != cudaSuccess ? e : cudaGetLastError();
   }
   switch (L.mode) {
