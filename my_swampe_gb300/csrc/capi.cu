@@ -1147,8 +1147,12 @@ int swp_plan_create(int ngroups, const int* M, const int* B, int precision, swp_
       *out = p;
       return SWP_ERR_CUDA;
     }
+    // member tile of the SIMT Legendre kernels until the autotuner sets it: as large
+    // as leaves a unit for every SM (M = 42, FP32 step: 8 members 18 us with tiles of
+    // 2, 20 with 4, 25 with 8; 16 members 27 with 2, 21 with 4, 24 with 8)
     size_t cap = f64 ? 150 * 1024 : 110 * 1024;
     int mt = 8;
+    while (mt > 1 && (M[g] + 1) * ((B[g] + mt - 1) / mt) < 160) mt /= 2;
     while (mt > 1 && (f64 ? spec_smem_bytes<double>(M[g], J, mt) : spec_smem_bytes<float>(M[g], J, mt)) > cap) mt /= 2;
     p->MT[g] = std::min(mt, B[g]);
     // rows per grid CTA: fixed per truncation and mode at compile time (grid.cu grid_jb)

@@ -23,8 +23,8 @@
 // reference's lax.cond guards do.
 #include <cmath>
 #include <cooperative_groups.h>
-#include "grid_common.cuh"
 #include "slices.cuh"
+#include "swp_internal.h"
 
 namespace swp {
 namespace {

@@ -28,8 +28,14 @@ namespace swp {
 constexpr int NKIN_P = 5;  // inverse inputs on P: eta, delta, Phi, Uprep, Vprep
 constexpr int NKIN_H = 2;  // inverse inputs on H: eta_s (U), -delta_s (V)
 constexpr int NKIN = NKIN_P + NKIN_H;
-constexpr int FWD_TC = 4;  // n-columns per thread in the forward contraction
-constexpr int INV_TJ = 2;  // latitudes per thread in the inverse contraction
+// Register tiles of the contractions: n-columns per thread in the forward one,
+// latitudes in the inverse one.  The small tiles are for units of one or two
+// members, whose few rows would leave most of a CTA's threads without work (FP32,
+// M = 42, 8 members: 25 us with units of 8 members and the large tiles, 18 us with
+// units of 2 and the small ones).  A result is one thread's sum over the latitudes
+// (degrees) in order, whatever the tile.
+template <bool SMALL> struct Reg { static constexpr int FWD_TC = SMALL ? 1 : 4, INV_TJ = SMALL ? 1 : 2; };
+constexpr int SMALL_MT = 2;
 
 template <typename T>
 size_t spec_smem_bytes(int M, int J, int MT) {
@@ -42,6 +48,23 @@ size_t spec_smem_bytes(int M, int J, int MT) {
 }
 template size_t spec_smem_bytes<double>(int, int, int);
 template size_t spec_smem_bytes<float>(int, int, int);
+
+// The two basis matrices of one m (nb elements each, a multiple of 16 bytes) to
+// shared memory; completed by cp_async_wait_all and a block barrier.  Issued at
+// the start of a unit -- both blocks where L.early_inv has room for the second
+// one -- so that their latency runs beside the combined inputs and not, as loads
+// and stores of each thread, between the phases (FP32, one member, M = 106: 36 ->
+// 28 us a step).
+template <typename T>
+__device__ __forceinline__ void copy_basis(T* dst, int ld, const T* srcP, const T* srcH, int nb) {
+  constexpr int E = 16 / (int)sizeof(T);
+  for (int t = threadIdx.x * E; t < nb; t += blockDim.x * E) {
+    cp_async<16>(dst + t, srcP + t);
+    cp_async<16>(dst + ld + t, srcH + t);
+  }
+}
+template <typename T>
+__host__ __device__ __forceinline__ size_t basis_bytes(int M, int J) { return (size_t)2 * (M + 1) * (J / 2) * sizeof(T); }
 
 // Run body(group, unit index) for every unit of the launch: one unit per CTA,
 // or -- persistent launches (L.sched set) -- units taken in turn from the
@@ -79,11 +102,12 @@ __device__ __forceinline__ void for_each_unit(const SpecLaunch<T>& L, F body) {
   }
 }
 
-template <typename T>
+template <typename T, bool SMALL>
 __device__ __forceinline__ void spectral_unit(const SpecLaunch<T>& L, const SpecGroup<T>& G, const int idx) {
   typedef typename cplx<T>::type T2;
   constexpr int NSPX = SlotCount<T>::NP;
   constexpr int NSLOT = NSPX + NSH;
+  constexpr int FWD_TC = Reg<SMALL>::FWD_TC, INV_TJ = Reg<SMALL>::INV_TJ;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const StepCfg& cfg = L.cfg;
   const int mode = L.mode;
@@ -107,6 +131,9 @@ __device__ __forceinline__ void spectral_unit(const SpecLaunch<T>& L, const Spec
   T* sigPm1 = sigm1 + MT * cntmax;
   T* tcmn = sigPm1 + MT * cntmax;
   int* sdead = (int*)(((uintptr_t)(tcmn + MT * cntmax) + 15) & ~(uintptr_t)15);  // [MT]
+  T* Bi = L.early_inv ? (T*)(((uintptr_t)(sdead + 64) + 15) & ~(uintptr_t)15) : Bf;
+  copy_basis<T>(Bf, cntmax * Jh, g.Pw_f + g.boff[m], g.Hw_f + g.boff[m], cnt * Jh);
+  if (L.early_inv) copy_basis<T>(Bi, cntmax * Jh, g.P_i + g.boff[m], g.H_i + g.boff[m], cnt * Jh);
   const bool step_mode = mode == 0 || mode == 3;  // 3: tangent-linear step on the tangent state
   const bool incr = SlotCount<T>::INCR && cfg.incremental && step_mode && cfg.scheme == 0;
 
@@ -175,13 +202,8 @@ __device__ __forceinline__ void spectral_unit(const SpecLaunch<T>& L, const Spec
       base[(1 * Jh + jp) * R + 2 * bt + 1] = xa[q].y;
     }
   }
-  // ---- phase 2: forward basis block for m
-  {
-    const T* srcP = g.Pw_f + g.boff[m];
-    const T* srcH = g.Hw_f + g.boff[m];
-    int nb = cnt * Jh;
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) { Bf[t] = srcP[t]; Bf[cntmax * Jh + t] = srcH[t]; }
-  }
+  // ---- phase 2: the basis blocks have arrived
+  cp_async_wait_all();
   __syncthreads();
 
   // ---- phase 3: forward contraction over J/2 latitudes + spectral epilogue
@@ -413,21 +435,19 @@ __device__ __forceinline__ void spectral_unit(const SpecLaunch<T>& L, const Spec
   __syncthreads();
   }  // pass
   // ---- phase 4: inverse basis block for m
-  {
-    const T* srcP = g.P_i + g.boff[m];
-    const T* srcH = g.H_i + g.boff[m];
-    int nb = cnt * Jh;
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) { Bf[t] = srcP[t]; Bf[cntmax * Jh + t] = srcH[t]; }
+  if (!L.early_inv) {
+    copy_basis<T>(Bi, cntmax * Jh, g.P_i + g.boff[m], g.H_i + g.boff[m], cnt * Jh);
+    cp_async_wait_all();
+    __syncthreads();
   }
-  __syncthreads();
 
   // ---- phase 5: inverse contraction (even/odd n-m) -> Fourier outputs in smem
   T* Out = X;  // [5][MT][J][2]
   {
     const int njt = (Jh + INV_TJ - 1) / INV_TJ;
     const int tasks = R * njt;
-    const T* BP = Bf;
-    const T* BH = Bf + cntmax * Jh;
+    const T* BP = Bi;
+    const T* BH = Bi + cntmax * Jh;
     for (int task = threadIdx.x; task < tasks; task += blockDim.x) {
       int r = task % R;
       int j0 = (task / R) * INV_TJ;
@@ -521,10 +541,12 @@ __device__ __forceinline__ void spectral_unit(const SpecLaunch<T>& L, const Spec
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_spectral(const __grid_constant__ SpecLaunch<T> L) {
+// FP32: 128 registers with a few spills, for a second CTA per SM (M = 42, 32
+// members: 36 -> 29 us)
+template <typename T, bool SMALL>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_spectral(const __grid_constant__ SpecLaunch<T> L) {
   pdl_enter();
-  for_each_unit(L, [&](const SpecGroup<T>& G, int idx) { spectral_unit<T>(L, G, idx); });
+  for_each_unit(L, [&](const SpecGroup<T>& G, int idx) { spectral_unit<T, SMALL>(L, G, idx); });
 }
 
 // ---------------------------------------------------------------------------
@@ -559,11 +581,12 @@ size_t spec_adj_smem_bytes(int M, int J, int MT) {
 template size_t spec_adj_smem_bytes<double>(int, int, int);
 template size_t spec_adj_smem_bytes<float>(int, int, int);
 
-template <typename T>
+template <typename T, bool SMALL>
 __device__ __forceinline__ void spectral_adj_unit(const SpecLaunch<T>& L, const SpecGroup<T>& G, const int idx) {
   typedef typename cplx<T>::type T2;
   constexpr int NKADJ = AdjCount<T>::NK;
   constexpr int NCAD = NKADJ + 4;
+  constexpr int FWD_TC = Reg<SMALL>::FWD_TC, INV_TJ = Reg<SMALL>::INV_TJ;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const StepCfg& cfg = L.cfg;
   const bool incr = SlotCount<T>::INCR && cfg.incremental;
@@ -593,6 +616,9 @@ __device__ __forceinline__ void spectral_adj_unit(const SpecLaunch<T>& L, const 
   // of latitudes (doubles: round the address up to 16 bytes)
   double* sgrad = (double*)(((uintptr_t)(tcmn + MT * cntmax) + 15) & ~(uintptr_t)15);
   const int nws = J / 32;
+  T* Bi = L.early_inv ? (T*)(((uintptr_t)(sgrad + 2 * MT * nws) + 15) & ~(uintptr_t)15) : Bf;
+  copy_basis<T>(Bf, cntmax * Jh, g.P_f + g.boff[m], g.H_f + g.boff[m], cnt * Jh);
+  if (L.early_inv) copy_basis<T>(Bi, cntmax * Jh, g.Pw_i + g.boff[m], g.Hw_i + g.boff[m], cnt * Jh);
 
   load_spec_coefs<T>(G, cfg.diffflag != 0, m, b0, mt, MT, cnt, cntmax, sig, sigP, sigm1, sigPm1, tcmn,
                      cfg.scheme == 2);
@@ -635,12 +661,7 @@ __device__ __forceinline__ void spectral_adj_unit(const SpecLaunch<T>& L, const 
     put(5, 0, ys[3]); put(5, 1, ya[3]);
     put(6, 0, ys[4]); put(6, 1, ya[4]);
   }
-  {
-    const T* srcP = g.P_f + g.boff[m];
-    const T* srcH = g.H_f + g.boff[m];
-    int nb = cnt * Jh;
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) { Bf[t] = srcP[t]; Bf[cntmax * Jh + t] = srcH[t]; }
-  }
+  cp_async_wait_all();
   __syncthreads();
 
   // ---- phase 2: transposed inverse Legendre (contract over J/2 latitudes)
@@ -761,20 +782,18 @@ __device__ __forceinline__ void spectral_adj_unit(const SpecLaunch<T>& L, const 
     }
   }
   __syncthreads();
-  {
-    const T* srcP = g.Pw_i + g.boff[m];
-    const T* srcH = g.Hw_i + g.boff[m];
-    int nb = cnt * Jh;
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) { Bf[t] = srcP[t]; Bf[cntmax * Jh + t] = srcH[t]; }
+  if (!L.early_inv) {
+    copy_basis<T>(Bi, cntmax * Jh, g.Pw_i + g.boff[m], g.Hw_i + g.boff[m], cnt * Jh);
+    cp_async_wait_all();
+    __syncthreads();
   }
-  __syncthreads();
   // ---- phase 4: transposed forward Legendre -> adjoints of the 9 combined inputs
   T* Cad = X;  // [NCAD][MT][J][2]
   {
     const int njt = (Jh + INV_TJ - 1) / INV_TJ;
     const int tasks = R * njt;
-    const T* BP = Bf;
-    const T* BH = Bf + cntmax * Jh;
+    const T* BP = Bi;
+    const T* BH = Bi + cntmax * Jh;
     // P results: K0..K4 on Pw -> PhiP1, PhiP2, dP1, dP2, eP1 ; H results: K0, K2, K3, K4 on Hw -> PhiH1, dH1, dH2, eH1
     for (int task = threadIdx.x; task < tasks; task += blockDim.x) {
       int r = task % R;
@@ -862,10 +881,10 @@ __device__ __forceinline__ void spectral_adj_unit(const SpecLaunch<T>& L, const 
   }
 }
 
-template <typename T>
+template <typename T, bool SMALL>
 __global__ void __launch_bounds__(256) k_spectral_adj(const __grid_constant__ SpecLaunch<T> L) {
   pdl_enter();
-  for_each_unit(L, [&](const SpecGroup<T>& G, int idx) { spectral_adj_unit<T>(L, G, idx); });
+  for_each_unit(L, [&](const SpecGroup<T>& G, int idx) { spectral_adj_unit<T, SMALL>(L, G, idx); });
 }
 
 namespace {
@@ -885,13 +904,45 @@ int persistent_blocks(K kernel, int nunits, size_t smem) {
     per_sm = 1;
   return std::max(1, std::min(nunits, per_sm * nsm));
 }
+
+// Give the second basis block its own buffer where that costs no CTA per SM.
+template <typename T>
+SpecLaunch<T> with_early_inv(const SpecLaunch<T>& L0, size_t& smem) {
+  SpecLaunch<T> L = L0;
+  size_t extra = 0;
+  for (int g = 0; g < L.ng; ++g)
+    if (L.grp[g].B > 0) extra = std::max(extra, basis_bytes<T>(L.grp[g].g.M, L.grp[g].g.J) + 16);
+  auto ctas = [](size_t n) { return (size_t)228 * 1024 / (n + 1024 + 128); };
+  if (smem + extra <= (size_t)SPEC_DYN_SMEM_MAX && ctas(smem + extra) >= std::min<size_t>(ctas(smem), 2)) {
+    smem += extra;
+    L.early_inv = 1;
+  }
+  return L;
+}
+// CTAs of a launch: one per unit where all are resident at once (the unit counter
+// would only add its round trips to L2, 4 us a launch), else persistent.
+template <typename T, typename K>
+int unit_blocks(SpecLaunch<T>& L, K kernel, int nunits, size_t smem) {
+  if (!L.sched) return nunits;
+  const int n = persistent_blocks(kernel, nunits, smem);
+  if (n >= nunits) L.sched = nullptr;
+  return n;
+}
+template <typename T>
+bool small_units(const SpecLaunch<T>& L) {
+  for (int g = 0; g < L.ng; ++g)
+    if (L.grp[g].B > 0 && L.grp[g].MT > SMALL_MT) return false;
+  return true;
+}
 }  // namespace
 
 template <typename T>
-cudaError_t launch_spec_adj(const SpecLaunch<T>& L, int nblocks, size_t smem, cudaStream_t s) {
+cudaError_t launch_spec_adj(const SpecLaunch<T>& L0, int nblocks, size_t smem, cudaStream_t s) {
   if (nblocks <= 0) return cudaSuccess;
-  const int grid = L.sched ? persistent_blocks(k_spectral_adj<T>, nblocks, smem) : nblocks;
-  cudaError_t e = launch_pdl(k_spectral_adj<T>, grid, 256, smem, s, std::is_same<T, float>::value, L);
+  SpecLaunch<T> L = with_early_inv(L0, smem);
+  auto kernel = small_units(L) ? k_spectral_adj<T, true> : k_spectral_adj<T, false>;
+  const int grid = unit_blocks(L, kernel, nblocks, smem);
+  cudaError_t e = launch_pdl(kernel, grid, 256, smem, s, std::is_same<T, float>::value, L);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 template cudaError_t launch_spec_adj<float>(const SpecLaunch<float>&, int, size_t, cudaStream_t);
@@ -906,16 +957,20 @@ bool pdl_enabled() {
 }
 
 void spec_set_attributes() {
-  cudaFuncSetAttribute(k_spectral<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEC_DYN_SMEM_MAX);
-  cudaFuncSetAttribute(k_spectral<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEC_DYN_SMEM_MAX);
-  cudaFuncSetAttribute(k_spectral_adj<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEC_DYN_SMEM_MAX);
+  for (auto k : {k_spectral<double, false>, k_spectral<double, true>})
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEC_DYN_SMEM_MAX);
+  for (auto k : {k_spectral<float, false>, k_spectral<float, true>, k_spectral_adj<float, false>,
+                 k_spectral_adj<float, true>})
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEC_DYN_SMEM_MAX);
 }
 
 template <typename T>
-cudaError_t launch_spec(const SpecLaunch<T>& L, int nblocks, size_t smem, cudaStream_t s) {
+cudaError_t launch_spec(const SpecLaunch<T>& L0, int nblocks, size_t smem, cudaStream_t s) {
   if (nblocks <= 0) return cudaSuccess;
-  const int grid = L.sched ? persistent_blocks(k_spectral<T>, nblocks, smem) : nblocks;
-  cudaError_t e = launch_pdl(k_spectral<T>, grid, 256, smem, s, std::is_same<T, float>::value, L);
+  SpecLaunch<T> L = with_early_inv(L0, smem);
+  auto kernel = small_units(L) ? k_spectral<T, true> : k_spectral<T, false>;
+  const int grid = unit_blocks(L, kernel, nblocks, smem);
+  cudaError_t e = launch_pdl(kernel, grid, 256, smem, s, std::is_same<T, float>::value, L);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 template cudaError_t launch_spec<double>(const SpecLaunch<double>&, int, size_t, cudaStream_t);

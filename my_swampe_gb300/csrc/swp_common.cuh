@@ -347,4 +347,17 @@ __device__ __forceinline__ void pdl_enter() {
   pdl_wait();
 }
 
+// Asynchronous global -> shared copy of one element (8 or 16 bytes, aligned to
+// its size); the issuing thread completes its copies with cp_async_wait_all.
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
+  static_assert(BYTES == 8 || BYTES == 16, "cp.async copies 8 or 16 bytes here");
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  if (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 }  // namespace swp

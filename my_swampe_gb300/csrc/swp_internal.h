@@ -184,6 +184,7 @@ struct SpecLaunch {
   // CTA per resident slot, which take units in order of decreasing truncation
   // (sorder: groups by decreasing M; sprefix: unit offsets in that order)
   SchedCounter* sched;
+  int early_inv;                        // SIMT kernels: the second basis block has a buffer of its own
   int sorder[MAXG];
   int sprefix[MAXG + 1];
 };
