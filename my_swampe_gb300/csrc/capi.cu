@@ -578,10 +578,13 @@ int tangent_steps(swp_plan* p, const swp_group_state* st, const swp_group_tangen
     if (e != cudaSuccess) return cuda_check(p, e, "tangent spectral kernel launch");
     e = launch_step_spec<T>(p, LS, nbs, s);
     if (e != cudaSuccess) return cuda_check(p, e, "spectral kernel launch");
-    e = launch_any_grid<T>(p, LG, nbg, s);
-    if (e != cudaSuccess) return cuda_check(p, e, "grid kernel launch");
-    e = launch_grid<T>(LGT, nbg, p->grid_smem[GM_TL_STEP], s);
-    if (e != cudaSuccess) return cuda_check(p, e, "tangent grid kernel launch");
+    if constexpr (std::is_same<T, float>::value) {
+      e = launch_grid_step_tl(LG, LGT, s);
+    } else {
+      e = launch_any_grid<T>(p, LG, nbg, s);
+      if (e == cudaSuccess) e = launch_grid<T>(LGT, nbg, p->grid_smem[GM_TL_STEP], s);
+    }
+    if (e != cudaSuccess) return cuda_check(p, e, "grid kernels launch");
   }
   return SWP_OK;
 }

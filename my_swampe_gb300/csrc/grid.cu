@@ -18,6 +18,7 @@
 // with 16-byte cp.async issued at the start of the CTA; the kernels are bound
 // by memory instructions in flight per SM rather than by bytes.
 // The kernel is specialised per mode at compile time.
+#include <algorithm>
 #include "grid_common.cuh"
 
 namespace swp {
@@ -880,6 +881,29 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (MODE == GM_ADJ_STEP ? 4
   }
 }
 
+// The primal and the tangent grid step in one launch: both follow the primal
+// Legendre step and neither reads what the other writes, so for few members one
+// launch's latency covers both (the tangent's CTAs come second).
+template <int CAP>
+__global__ void __launch_bounds__(256, 3)
+    k_grid_step_tl(const __grid_constant__ GridLaunch<float> Lp, const __grid_constant__ GridLaunch<float> Lt) {
+  pdl_enter();
+  const int n = Lp.prefix[Lp.ng];
+  const bool tl = (int)blockIdx.x >= n;
+  int idx;
+  const GridGroup<float>& G = tl ? pick_ggroup(Lt, idx, (int)blockIdx.x - n) : pick_ggroup(Lp, idx, (int)blockIdx.x);
+  auto body = [&](auto m) {
+    constexpr int M = decltype(m)::value;
+    if (tl) grid_body<float, GM_TL_STEP, M, cap_jb(grid_jb<float>(M, GM_TL_STEP), CAP)>(Lt, G, idx);
+    else grid_body<float, GM_STEP, M, cap_jb(grid_jb<float>(M, GM_STEP), CAP)>(Lp, G, idx);
+  };
+  switch (G.g.M) {
+    case 42: body(std::integral_constant<int, 42>()); break;
+    case 63: body(std::integral_constant<int, 63>()); break;
+    default: body(std::integral_constant<int, 106>()); break;
+  }
+}
+
 int grid_rows_per_cta(int M, bool fp64, int mode) { return fp64 ? grid_jb<double>(M, mode) : grid_jb<float>(M, mode); }
 
 // Largest dynamic shared memory the kernel may request: 227 KB per block minus
@@ -894,6 +918,11 @@ static void set_attr_one() {
 void grid_set_attributes() {
   set_attr_one<float, GM_STEP>(); set_attr_one<float, GM_STEP, 4>(); set_attr_one<float, GM_STEP, 2>();
   set_attr_one<float, GM_ADJ_STEP, 2>();
+  for (auto k : {k_grid_step_tl<8>, k_grid_step_tl<4>, k_grid_step_tl<2>}) {
+    cudaFuncAttributes fa;
+    const size_t stat = cudaFuncGetAttributes(&fa, k) == cudaSuccess ? fa.sharedSizeBytes : 2048;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - stat));
+  }
   set_attr_one<double, GM_INIT>(); set_attr_one<float, GM_INIT>();
   set_attr_one<float, GM_OUTPUT>();
   set_attr_one<double, GM_WINDS>(); set_attr_one<float, GM_WINDS>();
@@ -901,8 +930,37 @@ void grid_set_attributes() {
   set_attr_one<double, GM_ADJ_INIT>(); set_attr_one<float, GM_ADJ_INIT>();
   set_attr_one<double, GM_ADJ_OUTPUT>(); set_attr_one<float, GM_ADJ_OUTPUT>();
   set_attr_one<double, GM_FWD2>(); set_attr_one<float, GM_FWD2>();
-  set_attr_one<double, GM_TL_STEP>(); set_attr_one<float, GM_TL_STEP>();
+  set_attr_one<double, GM_TL_STEP>();
   set_attr_one<double, GM_TL_INIT>(); set_attr_one<float, GM_TL_INIT>();
+}
+
+// Few members: fewer rows per CTA while the launch would leave SMs idle (the
+// CTAs then run one latency chain each).  M = 42, one member, step / adjoint:
+// 12.5 / 11.3 us with 8 / 4 rows, 10.4 / 10.2 us with 2; 16 members 12.6 / 12.3
+// us, with 2 rows 16.4 / 12.3 us.  Rows are independent: the bits stay.
+template <typename T>
+int row_cap(const GridLaunch<T>& L) {
+  if (!std::is_same<T, float>::value || (L.mode != GM_STEP && L.mode != GM_ADJ_STEP && L.mode != GM_TL_STEP)) return 8;
+  int rows = 0;
+  for (int g = 0; g < L.ng; ++g) rows += L.grp[g].B * L.grp[g].g.J;
+  return rows <= (L.mode == GM_ADJ_STEP ? 4 : 2) * 152 ? 2 : rows <= 4 * 152 ? 4 : 8;
+}
+// Rows per CTA, block prefixes and the block count of a launch; smem is raised to
+// what its CTAs need.
+template <typename T>
+int decompose(GridLaunch<T>& L, int cap, size_t& smem) {
+  int nblocks = 0;
+  smem = 0;
+  for (int g = 0; g < L.ng; ++g) {
+    GridGroup<T>& G = L.grp[g];
+    G.JB = cap_jb(grid_jb<T>(G.g.M, L.mode), cap);
+    G.njb = G.g.J / G.JB;
+    L.prefix[g] = nblocks;
+    nblocks += G.B * G.njb;
+    if (G.B > 0) smem = std::max(smem, grid_smem_bytes<T>(G.g.M, G.g.J, G.g.I, G.JB, L.mode));
+  }
+  L.prefix[L.ng] = nblocks;
+  return nblocks;
 }
 
 template <typename T>
@@ -910,33 +968,16 @@ cudaError_t launch_grid(const GridLaunch<T>& L0, int nblocks0, size_t smem, cuda
   // rows per CTA and the block decomposition follow the mode (grid_jb)
   (void)nblocks0;
   GridLaunch<T> L = L0;
-  int nblocks = 0;
-  // Few members: fewer rows per CTA while the launch would leave SMs idle (the
-  // CTAs then run one latency chain each).  M = 42, one member, step / adjoint:
-  // 12.5 / 11.3 us with 8 / 4 rows, 10.4 / 10.2 us with 2; 16 members 12.6 / 12.3
-  // us, with 2 rows 16.4 / 12.3 us.  Rows are independent: the bits stay.
-  int cap = 8;
-  if (std::is_same<T, float>::value && (L.mode == GM_STEP || L.mode == GM_ADJ_STEP)) {
-    int rows = 0;
-    for (int g = 0; g < L.ng; ++g) rows += L.grp[g].B * L.grp[g].g.J;
-    cap = rows <= (L.mode == GM_STEP ? 2 : 4) * 152 ? 2 : rows <= 4 * 152 ? 4 : 8;
-    smem = 0;
-    for (int g = 0; g < L.ng; ++g) {
-      const Geom<T>& q = L.grp[g].g;
-      const size_t need = grid_smem_bytes<T>(q.M, q.J, q.I, cap_jb(grid_jb<T>(q.M, L.mode), cap), L.mode);
-      if (L.grp[g].B > 0 && need > smem) smem = need;
-    }
-  }
-  for (int g = 0; g < L.ng; ++g) {
-    GridGroup<T>& G = L.grp[g];
-    G.JB = cap_jb(grid_jb<T>(G.g.M, L.mode), cap);
-    G.njb = G.g.J / G.JB;
-    L.prefix[g] = nblocks;
-    nblocks += G.B * G.njb;
-  }
-  L.prefix[L.ng] = nblocks;
+  const int cap = row_cap(L);
+  const int nblocks = decompose(L, cap, smem);
   cudaError_t e = cudaSuccess;
   constexpr bool f32 = std::is_same<T, float>::value;
+  if constexpr (!f32) {  // FP32: k_grid_step_tl
+    if (L.mode == GM_TL_STEP) {
+      e = launch_pdl(k_grid<T, GM_TL_STEP>, nblocks, 256, smem, s, false, L);
+      return e != cudaSuccess ? e : cudaGetLastError();
+    }
+  }
   if constexpr (f32) {  // in FP64 these modes are grid_f64.cu's
     if (L.mode == GM_OUTPUT) e = launch_pdl(k_grid<T, GM_OUTPUT>, nblocks, 256, smem, s, true, L);
     auto capped = [&](auto k8, auto k4, auto k2) {
@@ -952,7 +993,6 @@ cudaError_t launch_grid(const GridLaunch<T>& L0, int nblocks0, size_t smem, cuda
     case GM_ADJ_INIT: e = launch_pdl(k_grid<T, GM_ADJ_INIT>, nblocks, 256, smem, s, f32, L); break;
     case GM_ADJ_OUTPUT: e = launch_pdl(k_grid<T, GM_ADJ_OUTPUT>, nblocks, 256, smem, s, f32, L); break;
     case GM_FWD2: e = launch_pdl(k_grid<T, GM_FWD2>, nblocks, 256, smem, s, f32, L); break;
-    case GM_TL_STEP: e = launch_pdl(k_grid<T, GM_TL_STEP>, nblocks, 256, smem, s, f32, L); break;
     case GM_TL_INIT: e = launch_pdl(k_grid<T, GM_TL_INIT>, nblocks, 256, smem, s, f32, L); break;
     default: return cudaErrorInvalidValue;
   }
@@ -960,5 +1000,16 @@ cudaError_t launch_grid(const GridLaunch<T>& L0, int nblocks0, size_t smem, cuda
 }
 template cudaError_t launch_grid<double>(const GridLaunch<double>&, int, size_t, cudaStream_t);
 template cudaError_t launch_grid<float>(const GridLaunch<float>&, int, size_t, cudaStream_t);
+
+// Primal step and tangent step (FP32); modes GM_STEP and GM_TL_STEP.
+cudaError_t launch_grid_step_tl(const GridLaunch<float>& P0, const GridLaunch<float>& T0, cudaStream_t s) {
+  GridLaunch<float> P = P0, Tl = T0;
+  size_t sp = 0, st = 0;
+  const int cap = row_cap(P), n = decompose(P, cap, sp) + decompose(Tl, cap, st);
+  if (n <= 0) return cudaSuccess;
+  auto kernel = cap == 8 ? k_grid_step_tl<8> : cap == 4 ? k_grid_step_tl<4> : k_grid_step_tl<2>;
+  cudaError_t e = launch_pdl(kernel, n, 256, std::max(sp, st), s, true, P, Tl);
+  return e != cudaSuccess ? e : cudaGetLastError();
+}
 
 }  // namespace swp

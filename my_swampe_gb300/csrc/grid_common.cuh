@@ -27,11 +27,15 @@ template <> __device__ __forceinline__ double tiny_val<double>() { return DBL_MI
 template <> __device__ __forceinline__ float tiny_val<float>() { return FLT_MIN; }
 
 template <typename T>
-__device__ __forceinline__ const GridGroup<T>& pick_ggroup(const GridLaunch<T>& L, int& idx) {
+__device__ __forceinline__ const GridGroup<T>& pick_ggroup(const GridLaunch<T>& L, int& idx, int block) {
   int gi = 0;
-  while (gi + 1 < L.ng && (int)blockIdx.x >= L.prefix[gi + 1]) ++gi;
-  idx = blockIdx.x - L.prefix[gi];
+  while (gi + 1 < L.ng && block >= L.prefix[gi + 1]) ++gi;
+  idx = block - L.prefix[gi];
   return L.grp[gi];
+}
+template <typename T>
+__device__ __forceinline__ const GridGroup<T>& pick_ggroup(const GridLaunch<T>& L, int& idx) {
+  return pick_ggroup(L, idx, (int)blockIdx.x);
 }
 
 // Half-length spectrum Z_k (k < L) of the C2R transform

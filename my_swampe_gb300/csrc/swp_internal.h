@@ -264,6 +264,7 @@ template <typename T> size_t grid_smem_bytes(int M, int J, int I, int JB, int mo
 template <typename T> cudaError_t launch_spec(const SpecLaunch<T>& L, int nblocks, size_t smem, cudaStream_t s);
 template <typename T> cudaError_t launch_spec_adj(const SpecLaunch<T>& L, int nblocks, size_t smem, cudaStream_t s);
 template <typename T> cudaError_t launch_grid(const GridLaunch<T>& L, int nblocks, size_t smem, cudaStream_t s);
+cudaError_t launch_grid_step_tl(const GridLaunch<float>& P, const GridLaunch<float>& T, cudaStream_t s);
 void spec_set_attributes();
 // dynamic shared memory a SIMT Legendre kernel may use (the rest of the 227 KB
 // is kept for its static shared memory)
