@@ -825,9 +825,9 @@ def _init_state_from_fields(*, static: Static, flags: "RunFlags", test: Optional
                        dead=torch.zeros(st.dead.shape, dtype=torch.bool, device=dev))
 
 
-def _load_state(eng: Engine, flags: "RunFlags", state0: State, test, t0: int, diag=None) -> int:
-    """Put a reference-layout State into the engine; returns the t_start the
-    steps must use.
+def _load_state(eng: Engine, flags: "RunFlags", state0: State, test, t0: int, diag=None, copies: int = 1) -> int:
+    """Put a reference-layout State into the engine (`copies` times along the
+    member axis); returns the t_start the steps must use.
 
     The Fourier carries are taken as given.  The physical fields enter as the
     synthesis of their truncated Fourier coefficients plus their part beyond
@@ -847,10 +847,13 @@ def _load_state(eng: Engine, flags: "RunFlags", state0: State, test, t0: int, di
 
     def fo(x):  # (B, J, M+1) -> (M+1, B, J)
         t = torch.as_tensor(x, device=dev).detach().to(cdt)
-        return (t if batched else t[None]).permute(2, 0, 1)
+        return rep((t if batched else t[None]).permute(2, 0, 1))
 
-    pc = torch.stack([ph(getattr(state0, n)) for n in ("eta_curr", "delta_curr", "Phi_curr", "U_curr", "V_curr")])
-    pp = torch.stack([ph(getattr(state0, n)) for n in ("eta_prev", "delta_prev", "Phi_prev")])
+    def rep(x):  # members: axis 1
+        return x if copies == 1 else x.repeat(1, copies, *[1] * (x.dim() - 2))
+
+    pc = rep(torch.stack([ph(getattr(state0, n)) for n in ("eta_curr", "delta_curr", "Phi_curr", "U_curr", "V_curr")]))
+    pp = rep(torch.stack([ph(getattr(state0, n)) for n in ("eta_prev", "delta_prev", "Phi_prev")]))
     fresh = (pp == pc[:3]).flatten(2).all(dim=2).all(dim=0)  # (B,): prev == curr
     mid = r_p = None
     if not bool(fresh.all()):
@@ -862,7 +865,7 @@ def _load_state(eng: Engine, flags: "RunFlags", state0: State, test, t0: int, di
     # the 16 given fields in slot order, in one copy
     by_slot = dict([(slot, name) for name, slot in _STATE_SLOTS] + list(zip(_PREV_SLOTS, _PREV_NAMES)))
     x = [torch.as_tensor(getattr(state0, by_slot[k]), device=dev).detach().to(cdt) for k in range(len(by_slot))]
-    x = torch.stack(x if batched else [v[None] for v in x])  # (16, B, J, M+1)
+    x = rep(torch.stack(x if batched else [v[None] for v in x]))  # (16, B, J, M+1)
     four[:len(by_slot)].copy_(x.permute(0, 3, 1, 2))
     for ps, ms in zip(_PREV_SLOTS, _MID_SLOTS):
         if filtered:  # the Fourier prev carry is the filtered lineage
@@ -892,8 +895,8 @@ def _load_state(eng: Engine, flags: "RunFlags", state0: State, test, t0: int, di
         member[_lib.MS_WCURR].copy_(torch.where(stepped, torch.zeros_like(w1), w1))
         member[_lib.MS_WMID].copy_(w1)
         member[_lib.MS_UPDATED].copy_(stepped.to(member.dtype))
-    dead = torch.as_tensor(state0.dead, device=dev).reshape(-1).to(member.dtype)
-    member[_lib.MS_DEAD].copy_(dead.expand(member.shape[1]))
+    dead = torch.as_tensor(state0.dead, device=dev).reshape(1, -1).to(member.dtype)
+    member[_lib.MS_DEAD].copy_(rep(dead)[0].expand(member.shape[1]))
     # stepped members advance by increments from the first step (fast precision);
     # the semi-implicit scheme takes its lagged remainders from the state
     return t0 - 1 if (flags.semi_implicit or bool(stepped.all())) else t0
@@ -957,12 +960,16 @@ def _state_after(eng: Engine, flags: "RunFlags", phys, batched: bool, state0: St
     return st
 
 
+# copies of a small ensemble that share a tangent run: up to this many members
+_TANGENT_MEMBERS = 24
+
+
 class _ScanLastFn(torch.autograd.Function):
     """Derivatives of simulate_scan_last's curr fields (eta, delta, Phi, U, V)
     in the Static's scalar parameters, with state0 held fixed (as the
     retrieval's fast path does: its state0 is built once from the base
     parameters).  Forward mode: the tangent-linear model from a zero initial
-    tangent.  Reverse mode: one tangent run per parameter that needs a
+    tangent.  Reverse mode: a tangent run along each parameter that needs a
     gradient (members are independent: one run serves every member)."""
 
     @staticmethod
@@ -973,11 +980,19 @@ class _ScanLastFn(torch.autograd.Function):
         return ctl["out"]
 
     @staticmethod
-    def _tangent(ctx, dpar_rows):
+    def _tangent(ctx, dpar_rows, copies: int = 1):
+        """Tangent run along dpar_rows (NTANGENT, copies B): `copies` copies of the
+        members, each with tangents of its own, as one ensemble."""
         ctl = ctx.ctl
         eng, flags, state0, test, t0, n = ctl["eng"], ctl["flags"], ctl["state0"], ctl["test"], ctl["t0"], ctl["n"]
-        _set_static_params(eng, ctl["vals"])
-        t_start = _load_state(eng, flags, state0, test, t0)
+        if copies == 1:
+            _set_static_params(eng, ctl["vals"])
+        else:
+            B = ctl["B"]
+            eng = _engine_for(eng.groups[0]["M"], copies * B, eng.precision, eng.device, steps=False)
+            vals = stack_values([ctl["vals"][k] for k in PARAM_NAMES], eng.device)
+            eng.groups[0]["params"].copy_(vals.expand(-1, B).repeat(1, copies))
+        t_start = _load_state(eng, flags, state0, test, t0, copies=copies)
         fc = _flags_c(flags, test, t_start, diagnostics=False)
         tfour, tresid, _ = eng.new_tangent_buffers()
         eng.tangent_forward(fc, t0, n, tfour, tresid, [dpar_rows])
@@ -1003,15 +1018,19 @@ class _ScanLastFn(torch.autograd.Function):
         params = ctx.saved_tensors
         res = [None] * (1 + len(params))
         w = gout.to(torch.float64)
-        for k in range(len(params)):
-            if not ctx.needs_input_grad[1 + k]:
-                continue
-            rows = torch.zeros((_lib.NTANGENT, B), dtype=torch.float64, device=dev)
-            rows[k] = 1.0
-            jk = _ScanLastFn._tangent(ctx, rows).to(torch.float64)
-            g = (w * jk).sum(dim=(0, 2, 3))
-            res[1 + k] = g.sum().reshape(params[k].shape).to(params[k].dtype) if params[k].dim() == 0 else \
-                g.reshape(params[k].shape).to(params[k].dtype)
+        want = [k for k in range(len(params)) if ctx.needs_input_grad[1 + k]]
+        # for few members the parameters' tangent runs go as copies of the members in
+        # one ensemble (8 members, 2 parameters: 38 us a step each, 47 us together)
+        per = max(1, _TANGENT_MEMBERS // B)
+        for i in range(0, len(want), per):
+            ks = want[i:i + per]
+            rows = torch.zeros((_lib.NTANGENT, len(ks) * B), dtype=torch.float64, device=dev)
+            for c, k in enumerate(ks):
+                rows[k, c * B:(c + 1) * B] = 1.0
+            js = _ScanLastFn._tangent(ctx, rows, len(ks)).to(torch.float64)
+            for c, k in enumerate(ks):
+                g = (w * js[:, c * B:(c + 1) * B]).sum(dim=(0, 2, 3))
+                res[1 + k] = (g.sum() if params[k].dim() == 0 else g).reshape(params[k].shape).to(params[k].dtype)
         return tuple(res)
 
 
