@@ -87,8 +87,14 @@ def _engine_for(M: int, B: int, precision: str, device=None, steps: bool = True)
 # kernels of one half fill the SMs the other half's leave idle.  Members are
 # independent: each half's results are those of the same members run alone.
 # (Forward only, M = 42, fast, 7,199 steps: 1.70M -> 2.09M member-steps/s at
-# B = 64, 2.16M -> 2.47M at B = 128.)
+# B = 64, 2.16M -> 2.47M at B = 128.)  The count is that of M = 42 in the fast
+# precision, whose Legendre kernel passes one wave of CTAs there (two per SM); a
+# member weighs more where that comes earlier: one CTA per SM on the finer grids,
+# and the FP64 kernels' smaller tiles.  Microseconds per step, one chain and two:
+# fast M = 63, 16 members 34 / 33 (adjoint 39 / 35), 37 members 67 / 58; M = 106,
+# 21 members 118 / 97; FP64 M = 42, 16 members 77 / 78, 32 members 126 / 108.
 _SPLIT_MIN_B = 64
+_SPLIT_WEIGHT = {"fast": {42: 1, 63: 4, 106: 7}, "fp64": {42: 2, 63: 4, 106: 8}}
 
 
 def _split_engine_for(M: int, sizes: Tuple[int, int], precision: str, device=None) -> Engine:
@@ -97,7 +103,9 @@ def _split_engine_for(M: int, sizes: Tuple[int, int], precision: str, device=Non
     key = (int(M), tuple(int(b) for b in sizes), precision, "split", dev.type, dev.index)
     eng = _ENGINE_CACHE.pop(key, None)
     if eng is None:
-        eng = Engine([(int(M), int(b)) for b in sizes], precision, device, concurrent=True, autotune=True)
+        # as _engine_for: the autotuner for ensembles of 32 members or more
+        eng = Engine([(int(M), int(b)) for b in sizes], precision, device, concurrent=True,
+                     autotune=sum(sizes) >= 32)
     _ENGINE_CACHE[key] = eng
     while len(_ENGINE_CACHE) > _ENGINE_CACHE_SIZE:
         _ENGINE_CACHE.popitem(last=False)
@@ -507,7 +515,8 @@ def run_model_scan(
             raise NotImplementedError("reverse-mode initial-field gradients through the RAW filter are not "
                                       "implemented (forward mode and parameter gradients are)")
 
-    split = (batched and B >= _SPLIT_MIN_B and tmax > starttime_eff and test != 1
+    split = (batched and B * _SPLIT_WEIGHT.get(precision, {}).get(M, 0) >= _SPLIT_MIN_B
+             and tmax > starttime_eff and test != 1
              and not (return_history or diagnostics or semi_implicit or raw_filter))
     eng = _engine_for(M, B, precision, device, steps=not split)
     dev = eng.device
@@ -659,7 +668,8 @@ def _run_split(M, B, precision, device, flags: RunFlagsC, t0: int, T: int, ics: 
     parameters are scalars or per-member tensors, sliced per half.  Returns the
     physical final fields (5, B, J, I), the differentiable final curr fields
     (or None) and the final State, all joined along the member axis."""
-    sizes = (B // 2, B - B // 2)
+    half = 8 * ((B + 7) // 8 // 2) or B // 2  # whole tiles of 8 members in the first half
+    sizes = (half, B - half)
     eng = _split_engine_for(M, sizes, precision, device)
     dev = eng.device
     sls = (slice(0, sizes[0]), slice(sizes[0], B))
