@@ -6,10 +6,10 @@
 // SM): of about 32,000 FP64 instructions per latitude row of a step at M = 42,
 // 24,000 were the 12 transforms.  A transform of truncated Fourier rows is a
 // product with a static cosine and sine matrix of M + 1 by I / 2; on slices it
-// costs three FP64 additions per output and none per input, 3,600 a row.  The
-// remaining 4,000 are the physics.  M = 42, step / adjoint: 256 members 806 / 1174
-// -> 426 / 770 us, one member 39 / 55 -> 16 / 20 us.  The FP64 pipe is busy half of
-// the time; the rest is the phases' latency at two CTAs per SM (128 registers).
+// costs no FP64 instruction, and the physics' 4,000 remain.  M = 42, step / adjoint:
+// 256 members 806 / 1174 -> 394 / 638 us, one member 39 / 55 -> 14 / 18 us.  FP64
+// pipe, tensor cores and integer issue each account for about a third of that; the
+// phases between barriers overlap only across the two CTAs of an SM (128 registers).
 //
 // One CTA: one member, JB latitude rows.
 //   1. cp.async of the rows' truncated Fourier coefficients;
@@ -584,8 +584,12 @@ __global__ void __launch_bounds__(256, 2) k_grid_out_f64(const __grid_constant__
   }
 }
 
-// Rows per CTA: as many as leave two CTAs per SM their shared memory, fewer
-// while the launch would not give every SM its two.
+// Rows per CTA: at most as many as leave two CTAs per SM their shared memory.  Few
+// rows for few members: two from 1.5 CTAs of one row per SM on (the two then share
+// the SM's FP64 pipe), four from 1.5 rounds of two.  Step, M = 42, us with 1 / 2 /
+// 4 rows (before the conversions moved to integers): 2 members 17 / 19 / 29, 4
+// members 21 / 19 / 29, 8 members 33 / 27 / 29, 12 members 45 / 39 / 41, 16 members
+// 55 / 45 / 41.
 enum Kind { STEP, ADJ, OUT };
 template <int M_, Kind K>
 constexpr int max_rows() { return K == OUT ? 1 : K == ADJ ? (M_ == 106 ? 1 : 2) : M_ == 42 ? 4 : M_ == 63 ? 2 : 1; }
@@ -617,9 +621,9 @@ cudaError_t launch_trunc(const GridLaunch<double>& L, const SliceBasis& basis, c
   constexpr int most = max_rows<M_, K>();
   const int rows = members * trunc_J(M_);
   if constexpr (most >= 4)
-    if (rows >= 4 * 2 * 152) return launch_one<M_, 4, K>(L, basis, s);
+    if (rows >= 6 * 152) return launch_one<M_, 4, K>(L, basis, s);
   if constexpr (most >= 2)
-    if (rows >= 2 * 2 * 152) return launch_one<M_, 2, K>(L, basis, s);
+    if (2 * rows >= 3 * 152) return launch_one<M_, 2, K>(L, basis, s);
   return launch_one<M_, 1, K>(L, basis, s);
 }
 

@@ -19,8 +19,8 @@
 //     in the FP32 accumulator, which starts at 1.5 * 2^23, so that its bit
 //     pattern is the integer.
 //   * The levels are added up in 64-bit integers (hi: levels 0..3, lo: 4..7),
-//     over any number of K = 32 blocks, and converted once: 3 FP64 additions an
-//     output, whatever K.
+//     over any number of K = 32 blocks, and converted once, also in integers: no
+//     FP64 instruction is left of a contraction.
 //
 // The result's error is that of the inputs on the row's scale and one final
 // rounding; a chain of FP64 FMAs rounds K times.  (With 7 digits, 2^-54 of the
@@ -140,19 +140,42 @@ struct Tile {
 };
 
 // The FP64 value of integer sums over at most 2^14 elements on the scales of an
-// A row and a B row.
+// A row and a B row: (hi 2^32 + lo) 2^(era + erb - 2112), rounded to nearest.  In
+// integers: about 35 instructions, where the three FP64 additions of two
+// magic-number conversions would cost the SM 57 cycles a warp against 9.
 __device__ __forceinline__ double value(long long hi, long long lo, int era, int erb) {
   const int s = era + erb;
   hi += lo >> 32;  // a unit of hi is 2^32 units of lo
-  lo &= 0xffffffffll;
-  // 1.5 * 2^(52 + k) with unit 2^k: adding the integer to its bits adds integer * 2^k
-  const long long mh = ((long long)(s - 1005) << 52) | 0x8000000000000ll;
-  const long long ml = ((long long)(s - 1037) << 52) | 0x8000000000000ll;
-  const double h = __longlong_as_double(mh + hi) - __longlong_as_double(mh);
-  const double l = __longlong_as_double(ml + lo) - __longlong_as_double(ml);
-  if (s < 1038) return 0.0;                                       // a zero row, or below 2^-1000
-  if (s > 3051) return __longlong_as_double(0x7ff8000000000000ll);  // a bad row
-  return h + l;
+  // magnitude as three words, most significant first
+  const uint32_t neg = (uint32_t)(hi >> 63);
+  uint32_t w0 = (uint32_t)lo ^ neg;
+  uint64_t h = (uint64_t)hi ^ (((uint64_t)neg << 32) | neg);
+  w0 += neg & 1u;
+  h += (neg && w0 == 0) ? 1u : 0u;
+  uint32_t w2 = (uint32_t)(h >> 32), w1 = (uint32_t)h;
+  // normalise: leading one to bit 31 of w2
+  int p = s - 1089 + 95;
+  if (w2 == 0) {
+    w2 = w1;
+    w1 = w0;
+    w0 = 0;
+    p -= 32;
+  }
+  if (w2 == 0) {
+    w2 = w1;
+    w1 = 0;
+    p -= 32;
+  }
+  const int z = __clz(w2);
+  const uint32_t a2 = __funnelshift_lc(w1, w2, z), a1 = __funnelshift_lc(w0, w1, z);
+  p -= z;
+  // 53 significant bits, rounded; the leading one adds 1 to the exponent field
+  uint64_t m = (((uint64_t)a2 << 32) | a1) >> 11;
+  m += (a1 >> 10) & 1u;
+  const uint64_t bits = ((uint64_t)(uint32_t)(p - 1) << 52) + m;
+  const bool zero = p < 1 || w2 == 0 || s < 1038;  // zero sum or row, or below 2^-1000
+  const uint64_t r = s > 3051 ? 0x7ff8000000000000ull : zero ? 0ull : bits | ((uint64_t)neg << 63);
+  return __longlong_as_double((long long)r);
 }
 
 // The B fragment of one k-step from digit planes in shared memory (words of two
@@ -164,6 +187,12 @@ __device__ __forceinline__ void load_b(uint32_t (&b)[ND][2], const uint32_t* p0,
     b[v][0] = p0[v * plane];
     b[v][1] = p1[v * plane];
   }
+}
+// Bring a packed static operand (bytes, 128-byte lines) towards the SM while the
+// data that it multiplies are still being formed.
+__device__ __forceinline__ void prefetch_lines(const void* p, int bytes) {
+  for (int o = threadIdx.x * 128; o < bytes; o += blockDim.x * 128)
+    asm volatile("prefetch.global.L1 [%0];" ::"l"((const char*)p + o));
 }
 // The A fragment of one k-step from a packed static operand (pack_a):
 // [k-step][digit][lane] of 16 bytes.

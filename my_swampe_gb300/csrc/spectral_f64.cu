@@ -6,13 +6,12 @@
 // What bounds it: on the FMA kernel the contractions were two thirds of the FP64
 // instructions and ran at the FP64 pipe's rate (0.88 ms a step at M = 42, B = 256;
 // 98 us for one member, whose contraction filled one warp of one sub-partition).
-// Left on the FP64 pipe now are the pointwise parts and three additions per
-// contraction output.  One unit is one m and MT members; 8 warps:
+// Left on the FP64 pipe now are the pointwise parts.  One unit is one m and MT members; 8 warps:
 //
 //   1. a thread per (member, latitude) forms the combined inputs (FP64) into
 //      shared memory, rows (slot, member component) x J latitudes;
-//   2. a warp per row forms its equatorially symmetric and antisymmetric parts,
-//      finds their exponents and slices them (lanes over latitudes);
+//   2. a warp per row finds its scale and slices its equatorially symmetric and
+//      antisymmetric parts (lanes over latitudes);
 //   3. warps take 16 x 8 output tiles (degrees x rows) over J/2 latitudes, the
 //      basis slices coming from global memory in fragment order (packed once
 //      per plan, L2 resident), and convert them to FP64;
@@ -162,13 +161,14 @@ struct Mem {
   static constexpr size_t cmax(size_t a, size_t b) { return a > b ? a : b; }
   static constexpr size_t A = cmax(cmax(raw, spec), cmax(kin, out)) * 8;
   static constexpr size_t B = cmax((size_t)ND * NIN * R * 2 * S::XW, (size_t)ND * NK * R * S::KW) * 4;
-  static constexpr size_t E = (size_t)(2 * NIN * R + NK * R) * 4;
+  static constexpr size_t E = (size_t)(NIN * R + NK * R) * 4;
   static constexpr size_t total = A + B + E;
 };
 
 // Symmetric (s = 0) and antisymmetric (s = 1) parts of the raw rows over the
-// southern latitudes j' (plus / minus their mirror), times 2^ep[j'], sliced on
-// their own scales.
+// southern latitudes j' (plus / minus their mirror), times 2^ep[j'], sliced.  Both
+// are formed in integers, on the scale of the row's largest element with one bit of
+// headroom.
 __device__ __forceinline__ int expo_scaled(double x, int ep) {
   const int e = expo(x);
   return e == 0x7ff ? ER_BAD : max(e + ep, 0);
@@ -183,27 +183,23 @@ __device__ __forceinline__ void slice_latitudes(const double* raw, int rows, con
   for (int i = 0; i < KI; ++i) p[i] = S::Jh % 32 == 0 || lane + 32 * i < S::Jh ? __ldg(ep + lane + 32 * i) : 0;
   for (int r = warp; r < rows; r += 8) {
     const double* x = raw + (size_t)r * S::J;
-    double xs[KI], xa[KI];
-    int es = 0, ea = 0;
+    double xn[KI], xs[KI];
+    int e = 0;
 #pragma unroll
     for (int i = 0; i < KI; ++i) {
       const int k = lane + 32 * i;
       const bool on = S::Jh % 32 == 0 || k < S::Jh;
-      const double a = on ? x[k] : 0.0, b = on ? x[S::J - 1 - k] : 0.0;
-      xs[i] = a + b;
-      xa[i] = a - b;
-      es = max(es, expo_scaled(xs[i], p[i]));
-      ea = max(ea, expo_scaled(xa[i], p[i]));
+      xn[i] = on ? x[k] : 0.0;
+      xs[i] = on ? x[S::J - 1 - k] : 0.0;
+      e = max(e, max(expo_scaled(xn[i], p[i]), expo_scaled(xs[i], p[i])));
     }
-    es = row_exponent((int)__reduce_max_sync(0xffffffffu, (unsigned)es));
-    ea = row_exponent((int)__reduce_max_sync(0xffffffffu, (unsigned)ea));
-    if (lane == 0) {
-      er[2 * r] = es;
-      er[2 * r + 1] = ea;
-    }
+    e = (int)__reduce_max_sync(0xffffffffu, (unsigned)e);
+    e = row_exponent(e >= 0x7ff ? e : e + 1);
+    if (lane == 0) er[r] = e;
 #pragma unroll
     for (int i = 0; i < KI; ++i) {
-      uint64_t a = fixed(xs[i], es - p[i]), b = fixed(xa[i], ea - p[i]);
+      const uint64_t fn = fixed(xn[i], e - p[i]), fs = fixed(xs[i], e - p[i]);
+      uint64_t a = fn + fs - BIAS, b = fn - fs + BIAS;
       pair_exchange(a, b);
       if (S::Jh % 32 == 0 || lane + 32 * i < S::Jh)
         store_digits(dig + S::xrow(r, lane & 1) + S::xword(r, (lane >> 1) + 16 * i), plane, a, b);
@@ -245,7 +241,7 @@ __device__ __forceinline__ void contract_latitudes(const PackView<S>& pk, int C0
       const int c = 16 * mt + g + 8 * (e >> 1), n = n0 + 2 * t + (e & 1);
       if (c < Cp && n < nrow)
         out[(size_t)((mat ? nP : 0) + n) * S::CNT + (par ? C0 + c : c)] =
-            value(tile.hi[e], tile.lo[e], ef[g + 8 * (e >> 1)], er[2 * (rbase + n) + sym]);
+            value(tile.hi[e], tile.lo[e], ef[g + 8 * (e >> 1)], er[rbase + n]);
     }
   }
 }
@@ -343,8 +339,8 @@ __global__ void __launch_bounds__(256, 2) k_spectral_f64(const __grid_constant__
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* A = (double*)smem_raw;
   uint32_t* D = (uint32_t*)(smem_raw + Mm::A);
-  int* erx = (int*)(smem_raw + Mm::A + Mm::B);  // [NIN R][2]
-  int* erk = erx + 2 * NIN * R;                 // [7 R]
+  int* erx = (int*)(smem_raw + Mm::A + Mm::B);  // [NIN R]
+  int* erk = erx + NIN * R;                     // [7 R]
   __shared__ int sdead[MT];
   int idx;
   const SpecGroup<double>& G = pick_group(L, idx);
@@ -353,6 +349,10 @@ __global__ void __launch_bounds__(256, 2) k_spectral_f64(const __grid_constant__
   const int cnt = S::CNT - m, C0 = (cnt + 1) / 2, C1 = cnt / 2;
   const size_t FS = (size_t)S::CNT * G.B * J;
   const PackView<S> pk(basis.p[&G - L.grp], m);
+  if (MT == 1) {  // few units: their basis is not in L1 yet
+    prefetch_lines(pk.f, (int)(Pack<S>::F * 16));
+    prefetch_lines(pk.i, (int)(Pack<S>::I * 16));
+  }
 
   // blow-up gate (model.py:838-864)
   if (threadIdx.x < MT) {
@@ -369,20 +369,35 @@ __global__ void __launch_bounds__(256, 2) k_spectral_f64(const __grid_constant__
     }
     sdead[bt] = dead;
   }
-  // 1. combined inputs
-  for (int t = threadIdx.x; t < MT * J; t += 256) {
-    const int bt = t / J, j = t % J;
+  // 1. combined inputs.  One member: two threads per latitude, real and imaginary
+  // parts (each form drops the other's arithmetic), since two warps alone would use
+  // half of the SM's FP64 sub-partitions
+  for (int t = threadIdx.x; t < (MT == 1 ? 2 : MT) * J; t += 256) {
+    const int bt = MT == 1 ? 0 : t / J, j = t % J;
+    auto combos = [&](double2* c) {
+      if (bt < mt) {
+        step_combos<double>(G, cfg, 0, false, m, b0 + bt, j, FS, c);
+      } else {
+#pragma unroll
+        for (int q = 0; q < NIN; ++q) c[q] = make_double2(0.0, 0.0);
+      }
+    };
     double2 c[NIN];
-    if (bt < mt) {
-      step_combos<double>(G, cfg, 0, false, m, b0 + bt, j, FS, c);
+    if (MT == 1 && t >= J) {
+      combos(c);
+#pragma unroll
+      for (int q = 0; q < NIN; ++q) A[(size_t)(q * R + 1) * J + j] = c[q].y;
+    } else if (MT == 1) {
+      combos(c);
+#pragma unroll
+      for (int q = 0; q < NIN; ++q) A[(size_t)(q * R) * J + j] = c[q].x;
     } else {
+      combos(c);
 #pragma unroll
-      for (int q = 0; q < NIN; ++q) c[q] = make_double2(0.0, 0.0);
-    }
-#pragma unroll
-    for (int q = 0; q < NIN; ++q) {
-      A[(size_t)(q * R + 2 * bt) * J + j] = c[q].x;
-      A[(size_t)(q * R + 2 * bt + 1) * J + j] = c[q].y;
+      for (int q = 0; q < NIN; ++q) {
+        A[(size_t)(q * R + 2 * bt) * J + j] = c[q].x;
+        A[(size_t)(q * R + 2 * bt + 1) * J + j] = c[q].y;
+      }
     }
   }
   __syncthreads();
@@ -392,14 +407,17 @@ __global__ void __launch_bounds__(256, 2) k_spectral_f64(const __grid_constant__
   __syncthreads();
   contract_latitudes<S>(pk, C0, C1, D, planeX, erx, NSP * R, NSP * R, NSH * R, A);
   __syncthreads();
-  // 4. spectral epilogue: a thread per (member, degree), both components
+  // 4. spectral epilogue: a thread per (member, degree) and, where the CTA has the
+  // threads, component
+  constexpr int NC = 2 * MT * S::CNT <= 256 ? 1 : 2;  // components per thread
   static_assert(MT * S::CNT <= 256, "one spectral point per thread");
   {
-    const int t = threadIdx.x, bt = t / cnt, kk = t % cnt;
-    const bool on = bt < mt;
+    const int comp0 = NC == 1 ? (int)threadIdx.x / (MT * cnt) : 0, t = (int)threadIdx.x - comp0 * MT * cnt;
+    const int bt = t / cnt, kk = t % cnt;
+    const bool on = comp0 < 2 && bt < mt;
     const int par = kk & 1, c = kk >> 1, pc = par ? C0 + c : c, n = m + kk, b = b0 + bt;
-    double e[2], d[2], p[2];  // new spectral eta, delta, Phi
-    double tc = 0.0;
+    double e[NC], d[NC], p[NC];  // new spectral eta, delta, Phi
+    double tc = 0.0, om = 0.0;
     if (on) {
       const size_t qs = (size_t)G.B * S::CNT, qo = (size_t)b * S::CNT + n;
       const bool expo_sig = cfg.scheme == 2;
@@ -408,7 +426,7 @@ __global__ void __launch_bounds__(256, 2) k_spectral_f64(const __grid_constant__
       tc = G.nco[NC_TC * qs + qo];
       const double nn1 = (double)(n * (n + 1));
       const double* mc = G.mco;
-      const double om = (m == 0 && n == 1) ? mc[MC_OM * G.B + b] : 0.0;
+      om = (m == 0 && n == 1) ? mc[MC_OM * G.B + b] : 0.0;
       // semi-implicit solve (semi_implicit_tdiff.py): shares and rates as in k_spectral
       double xi = 0.0, kd = 0.0, kr = 0.0, gd = 0.0, bq = 0.0, cq = 0.0, ikr = 1.0, ed = 1.0, Dn = 1.0;
       if (cfg.scheme == 2) {
@@ -426,40 +444,47 @@ __global__ void __launch_bounds__(256, 2) k_spectral_f64(const __grid_constant__
         Dn = (1.0 + kd) + bq * cq * ikr;
       }
 #pragma unroll
-      for (int comp = 0; comp < 2; ++comp) {
+      for (int k = 0; k < NC; ++k) {
+        const int comp = comp0 + k;
         auto a = [&](int q) { return A[(size_t)(q * R + 2 * bt + comp) * S::CNT + pc]; };
         const double sphi = a(SP_PHI1) + a(NSP + SH_PHI1), seta = a(SP_E1) + a(NSP + SH_E1);
         if (cfg.scheme == 2) {
           const double sdel = a(SP_D1) + a(NSP + SH_D1) + nn1 * a(SP_D2);
           const double se = comp == 0 ? seta + (gd * om + kd * om) : seta;
           const double dn = (sdel + bq * sphi * ikr) / Dn;
-          p[comp] = sp * ((sphi - cq * dn) * ikr);
-          d[comp] = s * dn;
-          e[comp] = s * (se / ed);
+          p[k] = sp * ((sphi - cq * dn) * ikr);
+          d[k] = s * dn;
+          e[k] = s * (se / ed);
         } else {
-          p[comp] = sp * (sphi + nn1 * a(SP_PHI2));
-          d[comp] = s * (a(SP_D1) + a(NSP + SH_D1) + nn1 * (a(SP_D2) + a(NSP + SH_D2)));
-          e[comp] = s * seta;
+          p[k] = sp * (sphi + nn1 * a(SP_PHI2));
+          d[k] = s * (a(SP_D1) + a(NSP + SH_D1) + nn1 * (a(SP_D2) + a(NSP + SH_D2)));
+          e[k] = s * seta;
         }
       }
-      // planetary vorticity: a constant of the wind inversion
       if (n == 0) tc = 0.0;
     }
     __syncthreads();  // the spectra are read: their place takes the inverse inputs
     if (on) {
-      const double om = (m == 0 && n == 1) ? G.mco[MC_OM * G.B + b] : 0.0;
-      double* K = A + (size_t)2 * bt * 2 * S::PC + par * S::PC + c;
       constexpr size_t RS = 2 * S::PC, QS = (size_t)R * 2 * S::PC;
       const double xm = (double)m;
-      const double es0 = (e[0] - om) * tc, es1 = e[1] * tc, ds0 = d[0] * tc, ds1 = d[1] * tc;
-      K[0] = e[0];            K[RS] = e[1];
-      K[QS] = d[0];           K[QS + RS] = d[1];
-      K[2 * QS] = p[0];       K[2 * QS + RS] = p[1];
-      // wind inversion inputs (spectral_transform.py:577-594): on P -i m delta_s, -i m eta_s; on H eta_s, -delta_s
-      K[3 * QS] = xm * ds1;   K[3 * QS + RS] = -xm * ds0;
-      K[4 * QS] = xm * es1;   K[4 * QS + RS] = -xm * es0;
-      K[5 * QS] = es0;        K[5 * QS + RS] = es1;
-      K[6 * QS] = -ds0;       K[6 * QS + RS] = -ds1;
+#pragma unroll
+      for (int k = 0; k < NC; ++k) {
+        const int comp = comp0 + k;
+        double* K = A + (size_t)(2 * bt + comp) * RS + par * S::PC + c;
+        // planetary vorticity: a real constant of the wind inversion
+        const double es = (comp == 0 ? e[k] - om : e[k]) * tc, ds = d[k] * tc;
+        K[0] = e[k];
+        K[QS] = d[k];
+        K[2 * QS] = p[k];
+        // wind inversion inputs (spectral_transform.py:577-594): on P -i m delta_s,
+        // -i m eta_s (into the other component's row); on H eta_s, -delta_s
+        double* Ko = comp == 0 ? K + RS : K - RS;
+        const double xs = comp == 0 ? -xm : xm;
+        Ko[3 * QS] = xs * ds;
+        Ko[4 * QS] = xs * es;
+        K[5 * QS] = es;
+        K[6 * QS] = -ds;
+      }
     }
     // rows of absent members of the last tile
     for (int i = threadIdx.x; i < 7 * (R - 2 * mt) * 2 * S::PC; i += 256) {
@@ -473,18 +498,49 @@ __global__ void __launch_bounds__(256, 2) k_spectral_f64(const __grid_constant__
   __syncthreads();
   contract_degrees<S>(pk, C0, C1, D, planeK, erk, 5 * R, 2 * R, [](int n) { return 5 * R + n; }, A);
   __syncthreads();
-  // 7. write-out and carries (coalesced along j)
-  const bool uv = cfg.test != 1;
-  for (int t = threadIdx.x; t < MT * J; t += 256) {
-    const int bt = t / J, j = t % J;
+  // 7. write-out and carries (coalesced along j): a thread per (field, member,
+  // latitude), the winds and the semi-implicit scheme's lagged remainders fourth.
+  // All loads of a thread precede its stores (input and output may be one buffer),
+  // and no two threads share a field.  Filters as write_step_point.
+  for (int t = threadIdx.x; t < 4 * MT * J; t += 256) {
+    const int j = t % J, bt = (t / J) % MT, q = t / (J * MT);
     if (bt >= mt || sdead[bt]) continue;
     const int b = b0 + bt;
-    auto get = [&](int q) {
-      return make_double2(A[(size_t)(q * R + 2 * bt) * J + j], A[(size_t)(q * R + 2 * bt + 1) * J + j]);
+    const size_t o = ((size_t)m * G.B + b) * J + j;
+    auto get = [&](int f) {
+      return make_double2(A[(size_t)(f * R + 2 * bt) * J + j], A[(size_t)(f * R + 2 * bt + 1) * J + j]);
     };
-    const double2 nw[3] = {get(0), get(1), get(2)};
-    write_step_point<double>(G, cfg, false, FS, ((size_t)m * G.B + b) * J + j, b, nw, uv, cadd(get(3), get(5)),
-                             cadd(get(4), get(6)));
+    const double2* Fi = G.four;
+    double2* Fo = G.four_out;
+    if (q < 3) {
+      const int cf = q == 0 ? F_ETA : q == 1 ? F_DELTA : F_PHI;
+      const int pf = q == 0 ? F_ETA_PREV : q == 1 ? F_DELTA_PREV : F_PHI_PREV;
+      const int rf = q == 0 ? F_ETA_MID : q == 1 ? F_DELTA_MID : F_PHI_MID;
+      double2 nw = get(q), old = make_double2(0.0, 0.0), mid = old;
+      if (cfg.write_prev || cfg.ra_mode) old = Fi[cf * FS + o];
+      if (cfg.ra_mode == 2) mid = Fi[rf * FS + o];
+      if (cfg.write_prev) Fo[pf * FS + o] = old;
+      if (cfg.ra_mode == 1) {
+        Fo[rf * FS + o] = old;
+      } else if (cfg.ra_mode == 2) {
+        const double2 d = cadd(csub(mid, cscale(old, 2.0)), nw);
+        Fo[rf * FS + o] = cadd(old, cscale(d, G.mco[(cfg.raw ? MC_RAWM : MC_ALPHA) * G.B + b]));
+        if (cfg.raw) nw = csub(nw, cscale(d, G.mco[MC_RAWN * G.B + b]));
+      }
+      Fo[cf * FS + o] = nw;
+    } else {
+      if (cfg.scheme == 2) {
+        const double itd = G.mco[MC_SIITD * G.B + b];
+        const double2 l0 = cadd(Fi[F_F * FS + o], cscale(Fi[F_U * FS + o], itd));
+        const double2 l1 = cadd(Fi[F_G * FS + o], cscale(Fi[F_V * FS + o], itd));
+        Fo[F_RU_LAG * FS + o] = l0;
+        Fo[F_RV_LAG * FS + o] = l1;
+      }
+      if (cfg.test != 1) {
+        Fo[F_U * FS + o] = cadd(get(3), get(5));
+        Fo[F_V * FS + o] = cadd(get(4), get(6));
+      }
+    }
   }
   // residual weights of the initial condition in the physical curr / prev fields
   if (m == 0 && threadIdx.x < mt && !sdead[threadIdx.x]) {
@@ -511,7 +567,7 @@ __global__ void __launch_bounds__(256, 2) k_spectral_adj_f64(const __grid_consta
   double* A = (double*)smem_raw;
   uint32_t* D = (uint32_t*)(smem_raw + Mm::A);
   int* erx = (int*)(smem_raw + Mm::A + Mm::B);
-  int* erk = erx + 2 * 5 * R;
+  int* erk = erx + 5 * R;
   __shared__ double sgrad[2][MT][NWS];
   int idx;
   const SpecGroup<double>& G = pick_group(L, idx);
@@ -520,6 +576,10 @@ __global__ void __launch_bounds__(256, 2) k_spectral_adj_f64(const __grid_consta
   const int cnt = S::CNT - m, C0 = (cnt + 1) / 2, C1 = cnt / 2;
   const size_t FS = (size_t)S::CNT * G.B * J;
   const PackView<S> pk(basis.p[&G - L.grp], m);
+  if (MT == 1) {  // few units: their basis is not in L1 yet
+    prefetch_lines(pk.f, (int)(Pack<S>::F * 16));
+    prefetch_lines(pk.i, (int)(Pack<S>::I * 16));
+  }
   for (int t = threadIdx.x; t < 2 * MT * NWS; t += 256) (&sgrad[0][0][0])[t] = 0.0;
 
   // 1. lambda of the outputs; the semi-implicit step's new level also enters its
@@ -549,12 +609,14 @@ __global__ void __launch_bounds__(256, 2) k_spectral_adj_f64(const __grid_consta
   contract_latitudes<S>(pk, C0, C1, D, planeX, erx, 5 * R, 3 * R, 2 * R, A);
   __syncthreads();
   // 4. transposed wind inversion, n(n+1) and hyperdiffusion (solve per degree in scheme 2)
+  constexpr int NC = 2 * MT * S::CNT <= 256 ? 1 : 2;  // components per thread
   static_assert(MT * S::CNT <= 256, "one spectral point per thread");
   {
-    const int t = threadIdx.x, bt = t / cnt, kk = t % cnt;
-    const bool on = bt < mt;
+    const int comp0 = NC == 1 ? (int)threadIdx.x / (MT * cnt) : 0, t = (int)threadIdx.x - comp0 * MT * cnt;
+    const int bt = t / cnt, kk = t % cnt;
+    const bool on = comp0 < 2 && bt < mt;
     const int par = kk & 1, c = kk >> 1, pc = par ? C0 + c : c, n = m + kk, b = b0 + bt;
-    double k[5][2];
+    double k[5][NC];
     if (on) {
       auto S_ = [&](int q, int comp) { return A[(size_t)(q * R + 2 * bt + comp) * S::CNT + pc]; };
       const size_t qs = (size_t)G.B * S::CNT, qo = (size_t)b * S::CNT + n;
@@ -564,8 +626,8 @@ __global__ void __launch_bounds__(256, 2) k_spectral_adj_f64(const __grid_consta
       const double w = n == 0 ? 0.0 : G.nco[NC_TC * qs + qo];
       const double nn1 = (double)(n * (n + 1)), xm = (double)m;
       // lambda delta_s = (i m) lambda Uprep - lambda Hin_V ; lambda eta_s = (i m) lambda Vprep + lambda Hin_U
-      const double lds[2] = {-xm * S_(3, 1) - S_(6, 0), xm * S_(3, 0) - S_(6, 1)};
-      const double les[2] = {-xm * S_(4, 1) + S_(5, 0), xm * S_(4, 0) + S_(5, 1)};
+      auto lds = [&](int comp) { return (comp == 0 ? -xm * S_(3, 1) : xm * S_(3, 0)) - S_(6, comp); };
+      auto les = [&](int comp) { return (comp == 0 ? -xm * S_(4, 1) : xm * S_(4, 0)) + S_(5, comp); };
       double bq = 0.0, cq = 0.0, ikr = 1.0, ikd = 1.0, Dn = 1.0;
       if (cfg.scheme == 2) {
         const double* mc = G.mco;
@@ -582,32 +644,32 @@ __global__ void __launch_bounds__(256, 2) k_spectral_adj_f64(const __grid_consta
         Dn = (1.0 + kd) + bq * cq * ikr;
       }
 #pragma unroll
-      for (int comp = 0; comp < 2; ++comp) {
-        const double lce = S_(0, comp) + w * les[comp], lcd = S_(1, comp) + w * lds[comp], lcp = S_(2, comp);
+      for (int i = 0; i < NC; ++i) {
+        const int comp = comp0 + i;
+        const double lce = S_(0, comp) + w * les(comp), lcd = S_(1, comp) + w * lds(comp), lcp = S_(2, comp);
         if (cfg.scheme == 2) {
           const double lpn = sp * lcp, ldn = s * lcd - cq * ikr * lpn, lsd = ldn / Dn;
-          k[0][comp] = ikr * lpn + bq * ikr * lsd;
-          k[1][comp] = 0.0;
-          k[2][comp] = lsd;
-          k[3][comp] = nn1 * lsd;
-          k[4][comp] = ikd * s * lce;
+          k[0][i] = ikr * lpn + bq * ikr * lsd;
+          k[1][i] = 0.0;
+          k[2][i] = lsd;
+          k[3][i] = nn1 * lsd;
+          k[4][i] = ikd * s * lce;
         } else {
-          k[0][comp] = sp * lcp;
-          k[1][comp] = nn1 * sp * lcp;
-          k[2][comp] = s * lcd;
-          k[3][comp] = nn1 * s * lcd;
-          k[4][comp] = s * lce;
+          k[0][i] = sp * lcp;
+          k[1][i] = nn1 * sp * lcp;
+          k[2][i] = s * lcd;
+          k[3][i] = nn1 * s * lcd;
+          k[4][i] = s * lce;
         }
       }
     }
     __syncthreads();
     if (on) {
-      double* K = A + (size_t)2 * bt * 2 * S::PC + par * S::PC + c;
+      double* K = A + (size_t)(2 * bt + comp0) * 2 * S::PC + par * S::PC + c;
 #pragma unroll
-      for (int q = 0; q < 5; ++q) {
-        K[(size_t)q * R * 2 * S::PC] = k[q][0];
-        K[(size_t)(q * R + 1) * 2 * S::PC] = k[q][1];
-      }
+      for (int q = 0; q < 5; ++q)
+#pragma unroll
+        for (int i = 0; i < NC; ++i) K[(size_t)(q * R + i) * 2 * S::PC] = k[q][i];
     }
     for (int i = threadIdx.x; i < 5 * (R - 2 * mt) * 2 * S::PC; i += 256) {
       const int kx = i % (2 * S::PC), r = 2 * mt + (i / (2 * S::PC)) % (R - 2 * mt), q = i / (2 * S::PC * (R - 2 * mt));
@@ -657,21 +719,23 @@ __global__ void __launch_bounds__(256, 2) k_spectral_adj_f64(const __grid_consta
   }
 }
 
-// Members per unit: the largest tile that still gives every SM its two CTAs
-// (units of low m, the long ones, come first); instantiated where the unit's
-// shared memory fits twice in an SM.  (M = 42, B = 256, step / transpose: 4 members
-// 359 / 347 us, 2 members 399 / 422 us, the FMA kernels 880 / 840 us; one member
-// 21 / 20 us, before 98 / 80 us.)
+// Members per unit.  One round of CTAs (two per SM) at one member each, then two;
+// four (M = 42 only: the unit's shared memory has to fit twice in an SM) once
+// those are most of a round themselves.  Step, M = 42, us with 1 / 2 / 4 members:
+// 6 members 23 / 24 / 36, 8 members 36 / 30 / 37, 16 members 51 / 42 / 46, 24
+// members 67 / 50 / 47 (before the conversion of the sums moved to integers; since
+// then 8 members 25, 16 members 34, 256 members 297, their transpose 294; the FMA
+// kernels 880 / 840 us there and 98 / 80 us for one member, now 17 / 18).
 template <int M_>
 int tile_for(const SpecLaunch<double>& L) {
-  for (int mt : {4, 2}) {
-    if (mt > (M_ == 42 ? 4 : M_ == 63 ? 2 : 1)) continue;
-    int units = 0;
+  auto units = [&](int mt) {
+    int n = 0;
     for (int g = 0; g < L.ng; ++g)
-      if (L.grp[g].g.M == M_) units += (M_ + 1) * ((L.grp[g].B + mt - 1) / mt);
-    if (units >= 2 * 152) return mt;
-  }
-  return 1;
+      if (L.grp[g].g.M == M_) n += (M_ + 1) * ((L.grp[g].B + mt - 1) / mt);
+    return n;
+  };
+  if (M_ == 42 && units(4) >= 256) return 4;
+  return M_ <= 63 && units(1) > 2 * 152 ? 2 : 1;
 }
 
 template <int M_, int MT, bool ADJ>

@@ -41,7 +41,7 @@ def _run(eng, ics, scheme, adjoint):
     return [out, dic[0], grad[0].clone()]
 
 
-@pytest.mark.parametrize("M,B", [(42, 3), (42, 17), (42, 33), (63, 2), (63, 11), (106, 2)])
+@pytest.mark.parametrize("M,B", [(42, 3), (42, 9), (42, 17), (42, 33), (63, 2), (63, 11), (106, 2)])
 @pytest.mark.parametrize("scheme", [0, 1, 2])
 @pytest.mark.parametrize("adjoint", [False, True])
 def test_members_do_not_depend_on_the_tile(cuda, M, B, scheme, adjoint):
