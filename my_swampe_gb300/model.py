@@ -81,20 +81,24 @@ def _engine_for(M: int, B: int, precision: str, device=None, steps: bool = True)
     return eng
 
 
-# Ensembles of this many members or more run, on the plain paths (no history,
-# diagnostics, semi-implicit scheme or RAW filter), as two halves of one
-# concurrent plan: each half's step chain on its own stream, so that the
-# kernels of one half fill the SMs the other half's leave idle.  Members are
-# independent: each half's results are those of the same members run alone.
+# Ensembles of this many members or more run (without history or diagnostics) as
+# two halves of one concurrent plan: each half's step chain on its own stream, so
+# that the kernels of one half fill the SMs the other half's leave idle.  Members
+# are independent: each half's results are those of the same members run alone.
 # (Forward only, M = 42, fast, 7,199 steps: 1.70M -> 2.09M member-steps/s at
-# B = 64, 2.16M -> 2.47M at B = 128.)  The count is that of M = 42 in the fast
-# precision, whose Legendre kernel passes one wave of CTAs there (two per SM); a
-# member weighs more where that comes earlier: one CTA per SM on the finer grids,
-# and the FP64 kernels' smaller tiles.  Microseconds per step, one chain and two:
-# fast M = 63, 16 members 34 / 33 (adjoint 39 / 35), 37 members 67 / 58; M = 106,
-# 21 members 118 / 97; FP64 M = 42, 16 members 77 / 78, 32 members 126 / 108.
+# B = 64, 2.16M -> 2.47M at B = 128.)  The count is that of M = 42, modified Euler,
+# fast, whose Legendre kernel passes one wave of CTAs there (two per SM); a member
+# weighs more where that comes earlier: one CTA per SM on the finer grids, the
+# SIMT kernel of the other schemes, the FP64 kernels' smaller tiles.  Microseconds
+# per step, one chain and two: fast M = 63, 16 members 34 / 33 (adjoint 39 / 35), 37
+# members 67 / 58; M = 106, 21 members 118 / 97; semi-implicit M = 42, 24 members 30 /
+# 31, 28 members 40 / 31, 40 members 40 / 34, M = 63, 16 members 44 / 41, 24 members 63
+# / 46, M = 106, 4 members 49 / 43; FP64 M = 42, 9 members 41 / 40 (adjoint 52 / 53),
+# 10 members 52 / 42 (67 / 56), 16 members 63 / 53 (90 / 68), 32 members 110 / 84; M =
+# 63, 6 members 61 / 65, 7 members 77 / 70; M = 106, 4 members 185 / 154 (237 / 238).
 _SPLIT_MIN_B = 64
-_SPLIT_WEIGHT = {"fast": {42: 1, 63: 4, 106: 7}, "fp64": {42: 2, 63: 4, 106: 8}}
+_SPLIT_WEIGHT = {"fast": {42: 1, 63: 4, 106: 7}, "fp64": {42: 7, 63: 10, 106: 16},
+                 "fast other schemes": {42: 2.3, 63: 4, 106: 16}}
 
 
 def _split_engine_for(M: int, sizes: Tuple[int, int], precision: str, device=None) -> Engine:
@@ -515,9 +519,10 @@ def run_model_scan(
             raise NotImplementedError("reverse-mode initial-field gradients through the RAW filter are not "
                                       "implemented (forward mode and parameter gradients are)")
 
-    split = (batched and B * _SPLIT_WEIGHT.get(precision, {}).get(M, 0) >= _SPLIT_MIN_B
-             and tmax > starttime_eff and test != 1
-             and not (return_history or diagnostics or semi_implicit or raw_filter))
+    other = precision == "fast" and bool(semi_implicit or expflag)
+    weight = _SPLIT_WEIGHT.get("fast other schemes" if other else precision, {}).get(M, 0)
+    split = (batched and B * weight >= _SPLIT_MIN_B and tmax > starttime_eff and test != 1
+             and not (return_history or diagnostics) and not (needs_grad and (semi_implicit or raw_filter)))
     eng = _engine_for(M, B, precision, device, steps=not split)
     dev = eng.device
     K6Phi_eff = K6 if K6Phi is None else K6Phi
@@ -668,7 +673,11 @@ def _run_split(M, B, precision, device, flags: RunFlagsC, t0: int, T: int, ics: 
     parameters are scalars or per-member tensors, sliced per half.  Returns the
     physical final fields (5, B, J, I), the differentiable final curr fields
     (or None) and the final State, all joined along the member axis."""
-    half = 8 * ((B + 7) // 8 // 2) or B // 2  # whole tiles of 8 members in the first half
+    # whole tiles of the kernels' members in the first half (FP64, M = 42, 12 members: 4 + 8
+    # 43 us per step, 6 + 6 47); equal halves on the SIMT kernel, whose tiles follow the
+    # member count (M = 63, 28 members: 8 + 20 63, 14 + 14 54)
+    tile = 4 if precision == "fp64" else 8 if flags.scheme == 0 else 1
+    half = tile * ((B + tile - 1) // tile // 2) or B // 2
     sizes = (half, B - half)
     eng = _split_engine_for(M, sizes, precision, device)
     dev = eng.device
@@ -708,7 +717,9 @@ def _run_split(M, B, precision, device, flags: RunFlagsC, t0: int, T: int, ics: 
         eng.forward(flags, t0=t0, nsteps=T, row0=0, write_prev_last=True)
     phys = torch.cat(eng.output_physical(flags), dim=1)
     eng.check_device_status()
-    last = _assemble_state(eng, phys, Rum, Rvm, batched)
+    if flags.scheme == 2:  # the lagged remainders the steps advanced
+        Rum, Rvm = (torch.cat([gd["fourier"][k] for gd in eng.groups], dim=1) for k in (_lib.F_RU_LAG, _lib.F_RV_LAG))
+    last = _assemble_state(eng, phys, Rum, Rvm, batched, filtered_prev=flags.scheme == 2 or flags.raw_filter)
     if dcurr is not None:
         last = last._replace(eta_curr=dcurr[0], delta_curr=dcurr[1], Phi_curr=dcurr[2], U_curr=dcurr[3],
                              V_curr=dcurr[4])
