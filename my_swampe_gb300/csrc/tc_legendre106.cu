@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(256, 1) k_spectral_tc106(const __grid_constant
     if (threadIdx.x < 32) bl.copy(4, buf[0], mblock + S::B1, B2_BYTES);
     // ---- phase 2: D1 -> staging sRes[g][n-m][member, re/im]; zero the A2 operands
     read_d1(tbase, sRes, 8, C0, C1);
-    for (int i = threadIdx.x; i < 4 * S::A2; i += blockDim.x) sA2[i] = 0.f;
+    for (int i = threadIdx.x; i < S::A2; i += blockDim.x) ((float4*)sA2)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     tc::fence_before_sync();
     __syncthreads();
     // ---- phase 3: spectral epilogue -> A2 operands [par][hi, lo][112 rows][K2]
@@ -771,7 +771,7 @@ __global__ void __launch_bounds__(256, 1) k_spectral_adj_tc106(const __grid_cons
     if (threadIdx.x < 32) bl.copy(4, buf[0], mblock + S::B1, B2_BYTES);
     // ---- phase 2: D1' -> sRes[q][n-m][member, re/im] (7 groups); zero the A2' operands
     read_d1(tbase, sRes, 7, C0, C1);
-    for (int i = threadIdx.x; i < 4 * S::AA2; i += blockDim.x) sA2[i] = 0.f;
+    for (int i = threadIdx.x; i < S::AA2; i += blockDim.x) ((float4*)sA2)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     tc::fence_before_sync();
     __syncthreads();
     // ---- phase 3: transposed wind inversion, n(n+1), hyperdiffusion -> A2' [par][hi, lo][128][K2]
