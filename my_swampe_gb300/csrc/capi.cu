@@ -229,6 +229,9 @@ template <typename Launch>
 cudaError_t launch_tc_per_truncation(const swp_plan* p, const SpecLaunch<float>& LS, float* const* bases,
                                      bool adjoint, Launch launch) {
   const int mt = spec_tc_members_per_cta();
+  int ctas = 0;  // of all the plan's groups: their chains run side by side on a concurrent plan
+  for (int g = 0; g < p->ng; ++g)
+    if (tc_group(p, g, adjoint)) ctas += (p->M[g] + 1) * ((p->B[g] + mt - 1) / mt);
   for (int Mt : {42, 63, 106}) {
     SpecLaunch<float> LT = LS;
     int acc = 0;
@@ -247,7 +250,7 @@ cudaError_t launch_tc_per_truncation(const swp_plan* p, const SpecLaunch<float>&
     }
     LT.prefix[p->ng] = acc;
     if (!any) continue;
-    cudaError_t e = launch(Mt, LT, acc, tb);
+    cudaError_t e = launch(Mt, LT, acc, tb, ctas <= (adjoint ? 152 : 114));  // all, or three quarters, of the SMs
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -280,8 +283,8 @@ cudaError_t launch_step_spec(const swp_plan* p, const SpecLaunch<T>& LS, int nbs
   if constexpr (std::is_same<T, float>::value) {
     if (p->use_tc && LS.mode == 0 && LS.cfg.scheme == 0 && !LS.cfg.tl_filter) {
       cudaError_t e = launch_tc_per_truncation(p, LS, p->tcbasis, false,
-                                               [&](int Mt, const SpecLaunch<float>& LT, int n, const TcBasis& tb) {
-                                                 return launch_spec_tc(Mt, LT, n, tb, p->d_err, s);
+                                               [&](int Mt, const SpecLaunch<float>& LT, int n, const TcBasis& tb, bool lone) {
+                                                 return launch_spec_tc(Mt, LT, n, tb, p->d_err, lone, s);
                                                });
       int nb = 0;
       SpecLaunch<float> LR = simt_only(p, LS, false, nb);
@@ -300,8 +303,8 @@ cudaError_t launch_step_spec_adj(const swp_plan* p, const SpecLaunch<T>& LS, int
   if constexpr (std::is_same<T, float>::value) {
     if (p->use_tc && LS.cfg.scheme == 0) {
       cudaError_t e = launch_tc_per_truncation(p, LS, p->tcbasis_adj, true,
-                                               [&](int Mt, const SpecLaunch<float>& LT, int n, const TcBasis& tb) {
-                                                 return launch_spec_adj_tc(Mt, LT, n, tb, p->d_err, s);
+                                               [&](int Mt, const SpecLaunch<float>& LT, int n, const TcBasis& tb, bool lone) {
+                                                 return launch_spec_adj_tc(Mt, LT, n, tb, p->d_err, lone, s);
                                                });
       int nb = 0;
       SpecLaunch<float> LR = simt_only(p, LS, true, nb);

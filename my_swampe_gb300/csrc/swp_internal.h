@@ -302,12 +302,12 @@ bool spec_tc_adj_supported(int M);  // adjoint kernel
 size_t spec_tc_adj_basis_floats(int M);
 int pack_tc_basis(const GroupGeom& gg, float* out, cudaStream_t s);
 void spec_tc_set_attributes();
-cudaError_t launch_spec_tc(int M, const SpecLaunch<float>& L, int nblocks, const TcBasis& basis, int* err,
+cudaError_t launch_spec_tc(int M, const SpecLaunch<float>& L, int nblocks, const TcBasis& basis, int* err, bool lone,
                            cudaStream_t s);
 int pack_tc_basis_adj(const GroupGeom& gg, float* out, cudaStream_t s);
 size_t spec_tc_adj_smem_bytes(int M);
 cudaError_t launch_spec_adj_tc(int M, const SpecLaunch<float>& L, int nblocks, const TcBasis& basis, int* err,
-                               cudaStream_t s);
+                               bool lone, cudaStream_t s);
 size_t spec_tc106_smem_bytes();
 size_t spec_tc106_adj_smem_bytes();
 size_t spec_tc106_basis_floats();

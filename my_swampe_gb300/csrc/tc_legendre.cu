@@ -116,6 +116,12 @@ auto tc_dispatch(int M, F f) -> decltype(f(Tc42())) {
 }
 }  // namespace
 
+// shared memory of the one-CTA-per-SM forms, forward and adjoint
+template <class S>
+constexpr size_t wide_smem_bytes() {
+  static_assert(2 * S::A >= S::AA, "the adjoint's A region");
+  return (size_t)(2 * S::A + S::BLOCK + S::COEF) * sizeof(float) + 256;
+}
 size_t spec_tc_smem_bytes(int M) {
   if (M == 106) return spec_tc106_smem_bytes();
   return tc_dispatch(M, [](auto S) { return (size_t)(S.A + S.B1 + S.COEF) * sizeof(float) + 256; });
@@ -226,8 +232,18 @@ __device__ __forceinline__ void mma_3xtf32_2(uint32_t d_tmem, uint32_t aH, uint3
 }
 }  // namespace
 
-template <class S>
-__global__ void __launch_bounds__(256, S::MINB) k_spectral_tc(const __grid_constant__ SpecLaunch<float> L,
+// W: the form for launches of no more CTAs than SMs (M = 42), which are one
+// latency chain per CTA.  With the SM to itself a CTA keeps both parities' A1 and
+// both basis blocks in shared memory (196 KB): parity 1 is formed while the MMAs
+// of parity 0 run, one commit and one wait cover both, and the inverse basis
+// comes with the forward one, before the wait for the previous kernel.  The same
+// sums in the same order.  Microseconds per step (Legendre and grid kernel), two
+// CTAs per SM and this form: 1 member 15.4 / 15.2, adjoint 17.5 / 15.1; 8 members
+// 20.7 / 16.9 (21.3 / 19.0); 16 members 22.4 / 21.3 (25.0 / 21.9); 24 members 22.0 /
+// 22.4 (25.5 / 22.0), where the forward launch leaves the next grid kernel's early
+// CTAs too few free SMs: it takes the form up to three quarters of the SMs.
+template <class S, bool W>
+__global__ void __launch_bounds__(256, W ? 1 : S::MINB) k_spectral_tc(const __grid_constant__ SpecLaunch<float> L,
                                                               const __grid_constant__ TcBasis basis, int* err) {
   typedef float T;
   typedef float2 T2;
@@ -254,9 +270,10 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_tc(const __grid_const
   }
 
   float* sA = (float*)smem_raw;            // staged inputs | A1 | A2 + D1 staging | output staging
-  float* sB = sA + S::A;                   // B1, then B2
+  float* sB = sA + (W ? 2 * S::A : S::A);  // B1, then B2 unless that has its own buffer sB2
+  float* sB2 = W ? sB + S::B1 : sB;
   float* sRes = sA + S::RES0;
-  float* sig = sB + S::B1;                 // [MT][CNT] x 5
+  float* sig = W ? sB2 + S::B2 : sB + S::B1;  // [MT][CNT] x 5
   float* sigP = sig + MT * CNT;
   float* sigm1 = sigP + MT * CNT;
   float* sigPm1 = sigm1 + MT * CNT;
@@ -280,8 +297,8 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_tc(const __grid_const
 #pragma unroll
     for (int q = 0; q < 4; ++q) tc::mbar_init(&mbar[q], 1);
     tc::fence_mbar_init();
-    tc::mbar_expect_tx(&mbar[0], (uint32_t)(S::B1 * sizeof(float)));
-    tc::bulk_g2s(sB, gbasis + (size_t)m * S::BLOCK, (uint32_t)(S::B1 * sizeof(float)), &mbar[0]);
+    tc::mbar_expect_tx(&mbar[0], (uint32_t)((W ? S::BLOCK : S::B1) * sizeof(float)));
+    tc::bulk_g2s(sB, gbasis + (size_t)m * S::BLOCK, (uint32_t)((W ? S::BLOCK : S::B1) * sizeof(float)), &mbar[0]);
     n_tma = 1;
   }
   if (warp == 0) {
@@ -392,8 +409,8 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_tc(const __grid_const
   // 16-byte zeroing of A2, two concurrent halves of 128 members, M = 42: 99.6 -> 98.5 us per step,
   // adjoint 123.0 -> 121.0; these stores queue in the shared memory both CTAs of the SM use).
   auto write_A1 = [&](int par) {
-    float* aH = sA;
-    float* aL = sA + S::ROWS * S::K1;
+    float* aH = sA + (W ? par * S::A : 0);
+    float* aL = aH + S::ROWS * S::K1;
 #pragma unroll
     for (int k = 0; k < S::NPAIR; ++k) {
       if (!has[k]) continue;
@@ -410,7 +427,7 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_tc(const __grid_const
           tc::split_tf32(comp ? vp.y : vp.x, hi, lo);
           aH[tc::cm_index(row, jp[k], S::K1)] = hi;
           aL[tc::cm_index(row, jp[k], S::K1)] = lo;
-          if (sh < 0 && par) continue;  // the zeros of parity 0 are still there
+          if (sh < 0 && par && !W) continue;  // the zeros of parity 0 are still there
           tc::split_tf32(comp ? vh.y : vh.x, hi, lo);
           aH[tc::cm_index(row, JH + jp[k], S::K1)] = hi;
           aL[tc::cm_index(row, JH + jp[k], S::K1)] = lo;
@@ -433,8 +450,21 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_tc(const __grid_const
       const bool good = tc::mbar_wait_bounded_warp(&mbar[0], 0, basis.wait_limit);
       if (!good) *sflag = 1;
       if (good) mma_3xtf32_2(tbase, aHs, aLs, bbase, S::N1, S::K1, idesc1w, idesc1);
-      tc::mma_commit_warp(&mbar[1]);
-      n_c1 = 1;
+      if (!W || !good) {
+        tc::mma_commit_warp(&mbar[1]);
+        n_c1 = 1;
+      }
+    }
+    if (W) {  // parity 1 into its own buffer while the MMAs of parity 0 run; one commit for both
+      write_A1(1);
+      tc::fence_proxy_async();
+      __syncthreads();
+      if (warp == 0 && !*sflag) {
+        mma_3xtf32_2(tbase + 2 * S::N1, aHs + (uint32_t)(S::A * 4), aLs + (uint32_t)(S::A * 4),
+                     bbase + 2u * S::N1 * S::K1 * 4u, S::N1, S::K1, idesc1w, idesc1);
+        tc::mma_commit_warp(&mbar[1]);
+        n_c1 = 1;
+      }
     }
     // the epilogue's per-(member, n) coefficients, gathered while the MMAs run
     load_spec_coefs<T>(G, cfg.diffflag != 0, m, b0, mt, MT, cnt, CNT, sig, sigP, sigm1, sigPm1, tcmn);
@@ -443,7 +473,7 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_tc(const __grid_const
     tc::fence_after_sync();
     ok = ok && !*sflag;  // written by thread 0 before the barrier: the same value for every thread
   }
-  if (ok) {
+  if (!W && ok) {
     write_A1(1);
     tc::fence_proxy_async();
     __syncthreads();
@@ -459,7 +489,7 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_tc(const __grid_const
   }
   if (ok) {
     // B1 is no longer read: fetch B2 into the same buffer, overlapped with the epilogue
-    if (threadIdx.x == 0) {
+    if (!W && threadIdx.x == 0) {
       tc::mbar_expect_tx(&mbar[0], (uint32_t)(S::B2 * sizeof(float)));
       tc::bulk_g2s(sB, gbasis + (size_t)m * S::BLOCK + S::B1, (uint32_t)(S::B2 * sizeof(float)), &mbar[0]);
       n_tma = 2;
@@ -554,12 +584,12 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_tc(const __grid_const
     // Warp 0 issues the MMAs first; then every thread issues the global loads
     // of its write-out pairs, whose latency overlaps the GEMM.
     if (warp == 0) {
-      const bool good = tc::mbar_wait_bounded_warp(&mbar[0], 1, basis.wait_limit);
+      const bool good = W || tc::mbar_wait_bounded_warp(&mbar[0], 1, basis.wait_limit);
       if (!good) *sflag = 1;
       if (good) {
         for (int par = 0; par < 2; ++par) {
           const uint32_t a2 = aHs + (uint32_t)(2 * par * S::A2) * 4u;
-          const uint32_t bp = bbase + (uint32_t)(2 * par * S::N2 * S::K2) * 4u;
+          const uint32_t bp = tc::smem_u32(sB2) + (uint32_t)(2 * par * S::N2 * S::K2) * 4u;
           mma_3xtf32(tbase + 2 * S::N1 + par * S::N2, a2, a2 + S::A2 * 4, bp, bp + S::N2 * S::K2 * 4, S::K2,
                      idesc2);
         }
@@ -682,9 +712,9 @@ size_t spec_tc_adj_smem_bytes(int M) {
   return tc_dispatch(M, [](auto S) { return (size_t)(S.AA + S.B1 + S.COEF) * sizeof(float) + 256; });
 }
 
-template <class S>
-__global__ void __launch_bounds__(256, S::MINB) k_spectral_adj_tc(const __grid_constant__ SpecLaunch<float> L,
-                                                                  const __grid_constant__ TcBasis basis, int* err) {
+template <class S, bool W>
+__global__ void __launch_bounds__(256, W ? 1 : S::MINB) k_spectral_adj_tc(const __grid_constant__ SpecLaunch<float> L,
+                                                                          const __grid_constant__ TcBasis basis, int* err) {
   typedef float T;
   typedef float2 T2;
   constexpr int NKADJ = 8;
@@ -709,9 +739,10 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_adj_tc(const __grid_c
   }
 
   float* sA = (float*)smem_raw;            // staged lambda | A1' | A2' + D1' staging | output staging
-  float* sB = sA + S::AA;                  // B1', then B2'; after GEMM2' the per-pair Phibar terms
+  float* sB = sA + (W ? 2 * S::A : S::AA); // B1', then B2' unless in sB2; after GEMM2' the per-pair Phibar terms
+  float* sB2 = W ? sB + S::B1 : sB;
   float* sRes = sA + S::ARES0;
-  float* sig = sB + S::B1;
+  float* sig = W ? sB2 + S::B2 : sB + S::B1;
   float* sigP = sig + MT * CNT;
   float* sigm1 = sigP + MT * CNT;
   float* sigPm1 = sigm1 + MT * CNT;
@@ -730,8 +761,8 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_adj_tc(const __grid_c
 #pragma unroll
     for (int q = 0; q < 4; ++q) tc::mbar_init(&mbar[q], 1);
     tc::fence_mbar_init();
-    tc::mbar_expect_tx(&mbar[0], (uint32_t)(S::B1 * sizeof(float)));
-    tc::bulk_g2s(sB, gbasis + (size_t)m * S::BLOCK, (uint32_t)(S::B1 * sizeof(float)), &mbar[0]);
+    tc::mbar_expect_tx(&mbar[0], (uint32_t)((W ? S::BLOCK : S::B1) * sizeof(float)));
+    tc::bulk_g2s(sB, gbasis + (size_t)m * S::BLOCK, (uint32_t)((W ? S::BLOCK : S::B1) * sizeof(float)), &mbar[0]);
     n_tma = 1;
   }
   if (warp == 0) {
@@ -795,8 +826,8 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_adj_tc(const __grid_c
   // parity 0: the P groups take the symmetric sums, the H groups the antisymmetric ones; the half of
   // the columns a group does not have is zeroed for both parities by the first
   auto write_A1 = [&](int par) {
-    float* aH = sA;
-    float* aL = sA + S::ROWS * S::K1;
+    float* aH = sA + (W ? par * S::A : 0);
+    float* aL = aH + S::ROWS * S::K1;
 #pragma unroll
     for (int k = 0; k < S::NPAIR; ++k) {
       if (!has[k]) continue;
@@ -812,7 +843,7 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_adj_tc(const __grid_c
           tc::split_tf32(comp ? v.y : v.x, hi, lo);
           aH[tc::cm_index(row, hg ? JH + jp[k] : jp[k], S::K1)] = hi;
           aL[tc::cm_index(row, hg ? JH + jp[k] : jp[k], S::K1)] = lo;
-          if (par) continue;  // the zeros of parity 0 are still there
+          if (par && !W) continue;  // the zeros of parity 0 are still there
           aH[tc::cm_index(row, hg ? jp[k] : JH + jp[k], S::K1)] = 0.f;
           aL[tc::cm_index(row, hg ? jp[k] : JH + jp[k], S::K1)] = 0.f;
         }
@@ -834,8 +865,21 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_adj_tc(const __grid_c
       const bool good = tc::mbar_wait_bounded_warp(&mbar[0], 0, basis.wait_limit);
       if (!good) *sflag = 1;
       if (good) mma_3xtf32_2(tbase, aHs, aLs, bbase, S::N1, S::K1, idesc1w, idesc1);
-      tc::mma_commit_warp(&mbar[1]);
-      n_c1 = 1;
+      if (!W || !good) {
+        tc::mma_commit_warp(&mbar[1]);
+        n_c1 = 1;
+      }
+    }
+    if (W) {  // parity 1 into its own buffer while the MMAs of parity 0 run; one commit for both
+      write_A1(1);
+      tc::fence_proxy_async();
+      __syncthreads();
+      if (warp == 0 && !*sflag) {
+        mma_3xtf32_2(tbase + 2 * S::N1, aHs + (uint32_t)(S::A * 4), aLs + (uint32_t)(S::A * 4),
+                     bbase + 2u * S::N1 * S::K1 * 4u, S::N1, S::K1, idesc1w, idesc1);
+        tc::mma_commit_warp(&mbar[1]);
+        n_c1 = 1;
+      }
     }
     // the epilogue's per-(member, n) coefficients, gathered while the MMAs run
     load_spec_coefs<T>(G, cfg.diffflag != 0, m, b0, mt, MT, cnt, CNT, sig, sigP, sigm1, sigPm1, tcmn);
@@ -844,7 +888,7 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_adj_tc(const __grid_c
     tc::fence_after_sync();
     ok = ok && !*sflag;
   }
-  if (ok) {
+  if (!W && ok) {
     write_A1(1);
     tc::fence_proxy_async();
     __syncthreads();
@@ -859,7 +903,7 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_adj_tc(const __grid_c
     tc::fence_after_sync();
   }
   if (ok) {
-    if (threadIdx.x == 0) {
+    if (!W && threadIdx.x == 0) {
       tc::mbar_expect_tx(&mbar[0], (uint32_t)(S::B2 * sizeof(float)));
       tc::bulk_g2s(sB, gbasis + (size_t)m * S::BLOCK + S::B1, (uint32_t)(S::B2 * sizeof(float)), &mbar[0]);
       n_tma = 2;
@@ -934,12 +978,12 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_adj_tc(const __grid_c
     tc::fence_after_sync();
     // ---- phase 5: GEMM2', both parities; write-out inputs loaded meanwhile (after the MMA issue)
     if (warp == 0) {
-      const bool good = tc::mbar_wait_bounded_warp(&mbar[0], 1, basis.wait_limit);
+      const bool good = W || tc::mbar_wait_bounded_warp(&mbar[0], 1, basis.wait_limit);
       if (!good) *sflag = 1;
       if (good) {
         for (int par = 0; par < 2; ++par) {
           const uint32_t a2 = aHs + (uint32_t)(2 * par * S::AA2) * 4u;
-          const uint32_t bp = bbase + (uint32_t)(2 * par * S::N2 * S::K2) * 4u;
+          const uint32_t bp = tc::smem_u32(sB2) + (uint32_t)(2 * par * S::N2 * S::K2) * 4u;
           mma_3xtf32(tbase + 2 * S::N1 + par * S::N2, a2, a2 + S::AA2 * 4, bp, bp + S::N2 * S::K2 * 4, S::K2,
                      idesc2);
         }
@@ -1023,33 +1067,39 @@ __global__ void __launch_bounds__(256, S::MINB) k_spectral_adj_tc(const __grid_c
 }
 
 void spec_tc_set_attributes() {
-  cudaFuncSetAttribute(k_spectral_tc<Tc42>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spec_tc_smem_bytes(42));
-  cudaFuncSetAttribute(k_spectral_adj_tc<Tc42>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)spec_tc_adj_smem_bytes(42));
-  cudaFuncSetAttribute(k_spectral_tc<Tc63>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spec_tc_smem_bytes(63));
-  cudaFuncSetAttribute(k_spectral_adj_tc<Tc63>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)spec_tc_adj_smem_bytes(63));
+  const auto lift = [](auto* kernel, size_t bytes) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  lift(k_spectral_tc<Tc42, false>, spec_tc_smem_bytes(42));
+  lift(k_spectral_tc<Tc42, true>, wide_smem_bytes<Tc42>());
+  lift(k_spectral_tc<Tc63, false>, spec_tc_smem_bytes(63));
+  lift(k_spectral_adj_tc<Tc42, false>, spec_tc_adj_smem_bytes(42));
+  lift(k_spectral_adj_tc<Tc42, true>, wide_smem_bytes<Tc42>());
+  lift(k_spectral_adj_tc<Tc63, false>, spec_tc_adj_smem_bytes(63));
   spec_tc106_set_attributes();
 }
 
 // One launch per truncation: L holds only the groups of truncation M (the
-// others have no members, so no CTAs).
-cudaError_t launch_spec_tc(int M, const SpecLaunch<float>& L, int nblocks, const TcBasis& basis, int* err,
+// others have no members, so no CTAs).  lone: few enough CTAs in the whole plan
+// for the one-CTA-per-SM form (see k_spectral_tc).
+cudaError_t launch_spec_tc(int M, const SpecLaunch<float>& L, int nblocks, const TcBasis& basis, int* err, bool lone,
                            cudaStream_t s) {
   if (nblocks <= 0) return cudaSuccess;
   if (M == 106) return launch_spec_tc106(L, nblocks, basis, err, s);
-  cudaError_t e = M == 63 ? launch_pdl(k_spectral_tc<Tc63>, nblocks, 256, spec_tc_smem_bytes(63), s, true, L, basis, err)
-                          : launch_pdl(k_spectral_tc<Tc42>, nblocks, 256, spec_tc_smem_bytes(42), s, true, L, basis, err);
+  auto* kernel = M == 63 ? k_spectral_tc<Tc63, false> : lone ? k_spectral_tc<Tc42, true> : k_spectral_tc<Tc42, false>;
+  const size_t smem = M == 42 && lone ? wide_smem_bytes<Tc42>() : spec_tc_smem_bytes(M);
+  cudaError_t e = launch_pdl(kernel, nblocks, 256, smem, s, true, L, basis, err);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_spec_adj_tc(int M, const SpecLaunch<float>& L, int nblocks, const TcBasis& basis, int* err,
-                               cudaStream_t s) {
+                               bool lone, cudaStream_t s) {
   if (nblocks <= 0) return cudaSuccess;
   if (M == 106) return launch_spec_adj_tc106(L, nblocks, basis, err, s);
-  cudaError_t e =
-      M == 63 ? launch_pdl(k_spectral_adj_tc<Tc63>, nblocks, 256, spec_tc_adj_smem_bytes(63), s, true, L, basis, err)
-              : launch_pdl(k_spectral_adj_tc<Tc42>, nblocks, 256, spec_tc_adj_smem_bytes(42), s, true, L, basis, err);
+  auto* kernel =
+      M == 63 ? k_spectral_adj_tc<Tc63, false> : lone ? k_spectral_adj_tc<Tc42, true> : k_spectral_adj_tc<Tc42, false>;
+  const size_t smem = M == 42 && lone ? wide_smem_bytes<Tc42>() : spec_tc_adj_smem_bytes(M);
+  cudaError_t e = launch_pdl(kernel, nblocks, 256, smem, s, true, L, basis, err);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
