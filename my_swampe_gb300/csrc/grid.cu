@@ -282,7 +282,11 @@ __device__ __forceinline__ void grid_body(const GridLaunch<T>& Lc, const GridGro
   // step: likewise eta, Phi, U, V (and delta for the history); the diagnostic
   // Phi row, which depends on the member's blow-up flag, follows the set-up
   const int step_nfix = G.hist ? 5 : 4;
-  if (MODE == GM_STEP) step_stage_issue<T>(c, G.four, 0, step_nfix, -1, c.bufB);
+  if (MODE == GM_STEP) {
+    step_stage_issue<T>(c, G.four, 0, step_nfix, -1, c.bufB);
+    // the diagnosed Phi is the filtered level's; a dead member's, the current's, replaces it below
+    if (cfg.diagnostics) step_stage_issue<T>(c, G.four, step_nfix, 1, F_PHI_MID, c.bufB);
+  }
   // tangent step: the primal eta, Phi, U, V, then their tangents
   if (MODE == GM_TL_STEP) {
     step_stage_issue<T>(c, G.primal, 0, 4, -1, c.bufB);
@@ -290,7 +294,6 @@ __device__ __forceinline__ void grid_body(const GridLaunch<T>& Lc, const GridGro
   }
   for (int i = threadIdx.x; i < I; i += blockDim.x) c.sday[i] = G.g.dayc[i];
   for (int i = threadIdx.x; i < 2 * L + 1; i += blockDim.x) stw[i] = i < L ? G.g.twL[i] : G.g.twI[i - L];
-  if (threadIdx.x == 0) { c.sred[0] = 0.0; c.sred[1] = 1e300; c.sred[2] = 1e300; c.sred[3] = -1e300; }
 
   const int B = G.B, b = c.b, j0 = c.j0;
   const size_t FS = c.FS, PS = c.PS;
@@ -302,6 +305,7 @@ __device__ __forceinline__ void grid_body(const GridLaunch<T>& Lc, const GridGro
   __shared__ int s_flag[2];  // no drag (taudrag == -1), member blown up
   __shared__ T s_dpar[NGRAD];  // tangent-linear modes: d(taurad, taudrag, DPhieq, Phibar)
   __shared__ T s_dw[2];        // tangent step and output: tangents of w_curr, w_mid
+  __shared__ typename StepDiag<T>::Block s_diag;
   if (threadIdx.x == 0) {
     if (MODE == GM_TL_STEP || MODE == GM_TL_INIT)
       for (int q = 0; q < NGRAD; ++q) s_dpar[q] = (T)G.dpar[q * B + b];
@@ -371,9 +375,12 @@ __device__ __forceinline__ void grid_body(const GridLaunch<T>& Lc, const GridGro
       }
     }
     if (MODE == GM_STEP) {
-      // the copies issued at the start of the CTA, plus the diagnostic row
-      if (cfg.diagnostics) step_stage_issue<T>(c, G.four, step_nfix, 1, dead ? F_PHI : F_PHI_MID, bufB);
+      // the copies issued at the start of the CTA (each thread overwrites its own)
       cp_async_wait_all();
+      if (dead) {
+        step_stage_issue<T>(c, G.four, step_nfix, 1, F_PHI, bufB);
+        cp_async_wait_all();
+      }
     } else {
       __syncthreads();
       stage_rows<T>(c, src, nf, bufB);
@@ -409,7 +416,7 @@ __device__ __forceinline__ void grid_body(const GridLaunch<T>& Lc, const GridGro
       }
       __syncthreads();
     }
-    double lrms = 0.0, lspin = 1e300, lmin = 1e300, lmax = -1e300;
+    StepDiag<T> dg;
 #pragma unroll 2
     for (int t = threadIdx.x; t < JB * L; t += blockDim.x) {
       int n = t % L, r = t / L, j = j0 + r;
@@ -454,42 +461,22 @@ __device__ __forceinline__ void grid_body(const GridLaunch<T>& Lc, const GridGro
         base[4 * PS] = vals[3][0]; base[4 * PS + 1] = vals[3][1];
       }
       if (cfg.diagnostics) {
-        double aw = g.area[j];
-        int fp = G.hist ? 5 : 4;
+        const double aw = g.area[j];
+        const int fp = G.hist ? 5 : 4;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          double U = vals[2][e], V = vals[3][e];
-          lrms += aw * (U * U + V * V);
-          lspin = fmin(lspin, sqrt(U * U + V * V));
-          double p = fp == 5 ? vals[5][e] : vals[4][e];
-          lmin = fmin(lmin, p);
-          lmax = fmax(lmax, p);
+          const double U = vals[2][e], V = vals[3][e];
+          dg.speed(aw, U * U + V * V);
+          dg.phi(fp == 5 ? vals[5][e] : vals[4][e]);
         }
       }
     }
     if (MODE == GM_OUTPUT || MODE == GM_WINDS) return;
-    if (cfg.diagnostics) {
-      for (int o = 16; o > 0; o >>= 1) {
-        lrms += __shfl_down_sync(0xffffffffu, lrms, o);
-        lspin = fmin(lspin, __shfl_down_sync(0xffffffffu, lspin, o));
-        lmin = fmin(lmin, __shfl_down_sync(0xffffffffu, lmin, o));
-        lmax = fmax(lmax, __shfl_down_sync(0xffffffffu, lmax, o));
-      }
-      if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&c.sred[0], lrms);
-        atomic_min_d(&c.sred[1], lspin);
-        atomic_min_d(&c.sred[2], lmin);
-        atomic_max_d(&c.sred[3], lmax);
-      }
-    }
+    if (cfg.diagnostics) dg.put(s_diag);
     __syncthreads();
-    if (cfg.diagnostics && threadIdx.x == 0) {
-      double* dn = G.diag + (size_t)(cfg.step + 1) * NDIAG * B;
+    if (cfg.diagnostics) {
       double* dc = G.diag + (size_t)cfg.step * NDIAG * B;
-      atomicAdd(&dn[D_RMS2 * B + b], c.sred[0]);
-      atomic_min_d(&dn[D_SPIN * B + b], c.sred[1]);
-      atomic_min_d(&dc[D_PHIMIN * B + b], c.sred[2]);
-      atomic_max_d(&dc[D_PHIMAX * B + b], c.sred[3]);
+      StepDiag<T>::add(s_diag, dc + NDIAG * B, dc, B, b);
     }
     const int nout = ph.forced ? 8 : 5;
     T2* res = cfft_batch_c<-1, L>(zout, zin, nout * JB, c.twL);
@@ -626,7 +613,7 @@ __device__ __forceinline__ void grid_body(const GridLaunch<T>& Lc, const GridGro
       __syncthreads();
     }
     // batch 2: nonlinear terms and forcing from the raw initial grids (model.py:723-732)
-    double lrms = 0.0, lspin = 1e300;
+    StepDiag<T> dg;
     const int nout = ph.forced ? 8 : 5;
     for (int t = threadIdx.x; t < JB * L; t += blockDim.x) {
       int n = t % L, r = t / L, j = j0 + r;
@@ -649,27 +636,17 @@ __device__ __forceinline__ void grid_body(const GridLaunch<T>& Lc, const GridGro
         }
         ph.eval(eta, Phi, U, V, ihalf, c.sday[2 * n + e] * s, outs[e]);
         if (cfg.diagnostics) {
-          double Ud = U, Vd = V;
-          lrms += g.area[j] * (Ud * Ud + Vd * Vd);
-          lspin = fmin(lspin, sqrt(Ud * Ud + Vd * Vd));
+          const double Ud = U, Vd = V;
+          dg.speed(g.area[j], Ud * Ud + Vd * Vd);
         }
       }
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         if (q < nout) bufA[((size_t)q * JB + r) * LS + n] = mk<T2>(outs[0][q], outs[1][q]);
     }
-    if (cfg.diagnostics) {
-      for (int o = 16; o > 0; o >>= 1) {
-        lrms += __shfl_down_sync(0xffffffffu, lrms, o);
-        lspin = fmin(lspin, __shfl_down_sync(0xffffffffu, lspin, o));
-      }
-      if ((threadIdx.x & 31) == 0) { atomicAdd(&c.sred[0], lrms); atomic_min_d(&c.sred[1], lspin); }
-    }
+    if (cfg.diagnostics) dg.put(s_diag);
     __syncthreads();
-    if (cfg.diagnostics && threadIdx.x == 0) {
-      atomicAdd(&G.diag[D_RMS2 * B + b], c.sred[0]);
-      atomic_min_d(&G.diag[D_SPIN * B + b], c.sred[1]);
-    }
+    if (cfg.diagnostics) StepDiag<T>::add(s_diag, G.diag, nullptr, B, b);
     T2* res2 = cfft_batch_c<-1, L>(bufA, bufB, nout * JB, c.twL);
     T2* dst[8];
 #pragma unroll

@@ -65,26 +65,103 @@ __device__ __forceinline__ T2 r2c_post(const T2* Z, int L, int k, const T2* twI,
   return cscale(cadd(e, cmul(o, twI[k])), scale);
 }
 
+// Extremes of doubles by integer atomics, which take one trip and no answer: above
+// zero a double's bits order as its value, below in reverse.  NaN changes nothing.
 __device__ __forceinline__ void atomic_min_d(double* addr, double v) {
-  unsigned long long* a = (unsigned long long*)addr;
-  unsigned long long old = *a, assumed;
-  int guard = 0;
-  while (__longlong_as_double(old) > v && guard++ < 4096) {
-    assumed = old;
-    old = atomicCAS(a, assumed, __double_as_longlong(v));
-    if (old == assumed) break;
-  }
+  if (v != v) return;
+  const long long k = __double_as_longlong(v + 0.0);  // -0 as 0
+  if (k >= 0) atomicMin((long long*)addr, k);
+  else atomicMax((unsigned long long*)addr, (unsigned long long)k);
 }
 __device__ __forceinline__ void atomic_max_d(double* addr, double v) {
-  unsigned long long* a = (unsigned long long*)addr;
-  unsigned long long old = *a, assumed;
-  int guard = 0;
-  while (__longlong_as_double(old) < v && guard++ < 4096) {
-    assumed = old;
-    old = atomicCAS(a, assumed, __double_as_longlong(v));
-    if (old == assumed) break;
-  }
+  if (v != v) return;
+  const long long k = __double_as_longlong(v + 0.0);
+  if (k >= 0) atomicMax((long long*)addr, k);
+  else atomicMin((unsigned long long*)addr, (unsigned long long)k);
 }
+
+// Order-preserving integers of floats and doubles.
+template <typename T> struct Order;
+template <> struct Order<float> {
+  typedef int K;
+  static __device__ __forceinline__ K flip(K b) { return b ^ ((b >> 31) & 0x7fffffff); }
+  static __device__ __forceinline__ K key(float v) { return flip(__float_as_int(v)); }
+  static __device__ __forceinline__ double value(K k) { return (double)__int_as_float(flip(k)); }
+  static constexpr K INF_BITS = 0x7f800000;
+};
+template <> struct Order<double> {
+  typedef long long K;
+  static __device__ __forceinline__ K flip(K b) { return b ^ ((b >> 63) & 0x7fffffffffffffffll); }
+  static __device__ __forceinline__ K key(double v) { return flip(__double_as_longlong(v)); }
+  static __device__ __forceinline__ double value(K k) { return __longlong_as_double(flip(k)); }
+  static constexpr K INF_BITS = 0x7ff0000000000000ll;
+};
+
+// The diagnostics of a step over a CTA's points: the area-weighted sum of squared
+// speed, the least speed, the extremes of Phi (NaN counts for none of the three).
+// All but the sum are compared as integers and the root is taken of the least
+// square: an FP64 comparison is a trip through the slow pipe, and a chain of five
+// shuffles and eight warps of them, retried CAS loops on the member's four words and
+// a root per point made the diagnostics the larger part of a small run's step
+// (M = 42, us per step without and with them: one member FP64 23.1 / 31.3, fast
+// 15.3 / 24.6, 16 members fast 21.2 / 46.3; now 22.8 / 24.1, 15.2 / 18.0, 21.2 / 28.1).
+template <typename T>
+struct StepDiag {
+  typedef typename Order<T>::K K;
+  static constexpr K PINF = Order<T>::INF_BITS, NINF = ~PINF;  // the keys of +inf and -inf; NaN's are outside
+  struct Block { double rms[8]; unsigned long long spin[8]; K lo[8], hi[8]; };
+  double rms = 0.0;
+  unsigned long long spin = 0x7ff0000000000000ull;  // bits of the least square, NaN's are above
+  K lo = PINF, hi = NINF;
+  __device__ __forceinline__ void speed(double aw, double s2) {
+    rms += aw * s2;
+    spin = min(spin, (unsigned long long)__double_as_longlong(s2));
+  }
+  __device__ __forceinline__ void phi(T p) {
+    const K k = Order<T>::key(p);
+    if (k < NINF || k > PINF) return;
+    lo = min(lo, k);
+    hi = max(hi, k);
+  }
+  // a warp's result to the block's slots (followed by a barrier)
+  __device__ __forceinline__ void put(Block& s) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      rms += __shfl_down_sync(0xffffffffu, rms, o);
+      spin = min(spin, __shfl_down_sync(0xffffffffu, spin, o));
+      lo = min(lo, __shfl_down_sync(0xffffffffu, lo, o));
+      hi = max(hi, __shfl_down_sync(0xffffffffu, hi, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+      const int w = threadIdx.x >> 5;
+      s.rms[w] = rms; s.spin[w] = spin; s.lo[w] = lo; s.hi[w] = hi;
+    }
+  }
+  // the block's contribution to a member's row, one quantity per warp
+  // (Phi's extremes only where dc is given)
+  static __device__ __forceinline__ void add(const Block& s, double* dn, double* dc, int B, int b) {
+    if ((threadIdx.x & 31) != 0) return;
+    const int q = 7 - (threadIdx.x >> 5);
+    if (q == 0) {
+      double r = s.rms[0];
+      for (int w = 1; w < 8; ++w) r += s.rms[w];
+      atomicAdd(&dn[D_RMS2 * B + b], r);
+    } else if (q == 1) {
+      unsigned long long m = s.spin[0];
+      for (int w = 1; w < 8; ++w) m = min(m, s.spin[w]);
+      const double v = __longlong_as_double((long long)m);
+      if (v < 1e300) atomic_min_d(&dn[D_SPIN * B + b], sqrt(v));
+    } else if (q == 2 && dc) {
+      K m = s.lo[0];
+      for (int w = 1; w < 8; ++w) m = min(m, s.lo[w]);
+      atomic_min_d(&dc[D_PHIMIN * B + b], Order<T>::value(m));
+    } else if (q == 3 && dc) {
+      K m = s.hi[0];
+      for (int w = 1; w < 8; ++w) m = max(m, s.hi[w]);
+      atomic_max_d(&dc[D_PHIMAX * B + b], Order<T>::value(m));
+    }
+  }
+};
 
 template <typename T>
 struct Physics {

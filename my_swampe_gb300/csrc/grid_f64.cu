@@ -294,7 +294,8 @@ __global__ void __launch_bounds__(256, 2) k_grid_step_f64(const __grid_constant_
   long long* qmid = (long long*)(smem_raw + Mm::A + Mm::B);
   int* ery = (int*)(qmid + STEP_NZ * JB);
   int* erz = ery + STEP_NF * JB;
-  __shared__ double s_mid[STEP_NF * JB], s_par[7], s_red[4][8];
+  __shared__ double s_mid[STEP_NF * JB], s_par[7];
+  __shared__ StepDiag<double>::Block s_diag;
   __shared__ int s_flag[2];
   int idx;
   const GridGroup<double>& G = pick_ggroup(Lc, idx);
@@ -306,6 +307,9 @@ __global__ void __launch_bounds__(256, 2) k_grid_step_f64(const __grid_constant_
   double2* raw = (double2*)A;
   copy_rows([&](int f) { return G.four + (size_t)(f == 0 ? F_ETA : f == 1 ? F_PHI : f == 2 ? F_U : f == 3 ? F_V : F_DELTA) * FS; },
             nfix, S::N1, JB, B, b, S::J, j0, raw);
+  // the diagnosed Phi is the filtered level's; a dead member's, the current's, replaces it below
+  if (cfg.diagnostics)
+    copy_rows([&](int) { return G.four + (size_t)F_PHI_MID * FS; }, 1, S::N1, JB, B, b, S::J, j0, raw, nfix);
   if (threadIdx.x == 0) {
     const double tr = G.par[P_TAURAD * B + b], td = G.par[P_TAUDRAG * B + b];
     const bool stepped = G.member && G.member[MS_UPDATED * B + b] != 0.0;
@@ -323,9 +327,11 @@ __global__ void __launch_bounds__(256, 2) k_grid_step_f64(const __grid_constant_
   }
   __syncthreads();
   const bool dead = s_flag[1] != 0;
-  if (cfg.diagnostics)
-    copy_rows([&](int) { return G.four + (size_t)(dead ? F_PHI : F_PHI_MID) * FS; }, 1, S::N1, JB, B, b, S::J, j0,
-              raw, nfix);
+  if (dead) {
+    cp_async_wait_all();
+    __syncthreads();
+    copy_rows([&](int) { return G.four + (size_t)F_PHI * FS; }, 1, S::N1, JB, B, b, S::J, j0, raw, nfix);
+  }
   Physics<double> ph;
   ph.Pb = s_par[0]; ph.itr = s_par[1]; ph.itd = s_par[2]; ph.DPe = s_par[3];
   ph.nodrag = s_flag[0] != 0; ph.forced = cfg.test == 0;
@@ -337,7 +343,7 @@ __global__ void __launch_bounds__(256, 2) k_grid_step_f64(const __grid_constant_
   c2r_tiles<S, JB>(mats, D, planeY, ery, s_mid, nf * JB, 0, A);
   __syncthreads();
   // physics: a thread per point, outputs in place of the fields
-  double lrms = 0.0, lspin = 1e300, lmin = 1e300, lmax = -1e300;
+  StepDiag<double> dg;
   const int nout = ph.forced ? 8 : 5;
   for (int t = threadIdx.x; t < JB * S::I; t += 256) {
     const int i = t % S::I, r = t / S::I, j = j0 + r;
@@ -368,40 +374,12 @@ __global__ void __launch_bounds__(256, 2) k_grid_step_f64(const __grid_constant_
       h[4 * PS] = v[3];
     }
     if (cfg.diagnostics) {
-      const double s2 = v[2] * v[2] + v[3] * v[3], p = nfix == 5 ? v[5] : v[4];
-      lrms += G.g.area[j] * s2;
-      lspin = fmin(lspin, s2);  // the least speed is the root of the least square
-      lmin = fmin(lmin, p);
-      lmax = fmax(lmax, p);
+      dg.speed(G.g.area[j], v[2] * v[2] + v[3] * v[3]);
+      dg.phi(nfix == 5 ? v[5] : v[4]);
     }
   }
-  if (cfg.diagnostics) {
-    for (int o = 16; o > 0; o >>= 1) {
-      lrms += __shfl_down_sync(0xffffffffu, lrms, o);
-      lspin = fmin(lspin, __shfl_down_sync(0xffffffffu, lspin, o));
-      lmin = fmin(lmin, __shfl_down_sync(0xffffffffu, lmin, o));
-      lmax = fmax(lmax, __shfl_down_sync(0xffffffffu, lmax, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-      const int w = threadIdx.x >> 5;
-      s_red[0][w] = lrms; s_red[1][w] = lspin; s_red[2][w] = lmin; s_red[3][w] = lmax;
-    }
-  }
+  if (cfg.diagnostics) dg.put(s_diag);
   __syncthreads();
-  if (cfg.diagnostics && threadIdx.x == 0) {
-    for (int w = 1; w < 8; ++w) {
-      lrms += s_red[0][w];
-      lspin = fmin(lspin, s_red[1][w]);
-      lmin = fmin(lmin, s_red[2][w]);
-      lmax = fmax(lmax, s_red[3][w]);
-    }
-    double* dn = G.diag + (size_t)(cfg.step + 1) * NDIAG * B;
-    double* dc = G.diag + (size_t)cfg.step * NDIAG * B;
-    atomicAdd(&dn[D_RMS2 * B + b], lrms);
-    atomic_min_d(&dn[D_SPIN * B + b], lspin < 1e300 ? sqrt(lspin) : lspin);
-    atomic_min_d(&dc[D_PHIMIN * B + b], lmin);
-    atomic_max_d(&dc[D_PHIMAX * B + b], lmax);
-  }
   slice_grid<S>(A, nout * JB, D, planeZ, erz, qmid);
   __syncthreads();
   double* four = (double*)(G.four + (size_t)F_A * FS);
@@ -410,6 +388,11 @@ __global__ void __launch_bounds__(256, 2) k_grid_step_f64(const __grid_constant_
                  if (!S::POW2) x *= 1.0 / S::I;
                  four[2 * ((size_t)(n / JB) * FS + ((size_t)m * B + b) * S::J + j0 + n % JB) + comp] = x;
                });
+  // after the products, which leave the last warps without a tile for few rows
+  if (cfg.diagnostics) {
+    double* dc = G.diag + (size_t)cfg.step * NDIAG * B;
+    StepDiag<double>::add(s_diag, dc + NDIAG * B, dc, B, b);
+  }
   // unforced runs: zero forcing terms, written explicitly (model.py:601-603)
   if (!ph.forced)
     for (int t = threadIdx.x; t < 3 * S::N1 * JB; t += 256) {

@@ -5,6 +5,13 @@
 
 namespace swp {
 
+// The blow-up gate (model.py:838-864) of a mean squared speed.  The root, an FP64
+// chain of twenty instructions, is taken only where the square is near the limit.
+__device__ __forceinline__ bool blown_up(const StepCfg& cfg, double ms) {
+  if (cfg.blowup > 0.0 && ms < 0.99 * cfg.blowup * cfg.blowup) return false;
+  return sqrt(ms) > cfg.blowup;
+}
+
 // combined-input slots of the forward contraction.  The FP32 path carries three
 // more P slots (the current eta, delta, Phi on their own) for the incremental
 // form of the step; the FP64 path keeps the reference's projection form.

@@ -144,8 +144,8 @@ __device__ __forceinline__ void spectral_unit(const SpecLaunch<T>& L, const Spec
     int bt = threadIdx.x, dead = 0;
     if (bt < mt && cfg.diagnostics && mode == 0) {
       int b = b0 + bt;
-      double rms = sqrt(G.diag[((size_t)cfg.step * NDIAG + D_RMS2) * G.B + b]);
-      dead = (G.member[MS_DEAD * G.B + b] != 0.0) || (rms > cfg.blowup);
+      const double ms = G.diag[((size_t)cfg.step * NDIAG + D_RMS2) * G.B + b];
+      dead = (G.member[MS_DEAD * G.B + b] != 0.0) || blown_up(cfg, ms);
       if (m == 0) {
         G.member[MS_DEAD * G.B + b] = dead ? 1.0 : 0.0;
         G.diag[((size_t)cfg.step * NDIAG + D_DEAD) * G.B + b] = dead ? 1.0 : 0.0;

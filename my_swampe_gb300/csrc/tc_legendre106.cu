@@ -509,8 +509,8 @@ __global__ void __launch_bounds__(256, 1) k_spectral_tc106(const __grid_constant
     int dead = 0;
     if (bt < mt && cfg.diagnostics) {
       const int b = b0 + bt;
-      const double rms = sqrt(G.diag[((size_t)cfg.step * NDIAG + D_RMS2) * G.B + b]);
-      dead = (G.member[MS_DEAD * G.B + b] != 0.0) || (rms > cfg.blowup);
+      const double ms = G.diag[((size_t)cfg.step * NDIAG + D_RMS2) * G.B + b];
+      dead = (G.member[MS_DEAD * G.B + b] != 0.0) || blown_up(cfg, ms);
       if (m == 0) {
         G.member[MS_DEAD * G.B + b] = dead ? 1.0 : 0.0;
         G.diag[((size_t)cfg.step * NDIAG + D_DEAD) * G.B + b] = dead ? 1.0 : 0.0;
