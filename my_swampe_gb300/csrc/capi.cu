@@ -184,6 +184,7 @@ GridLaunch<T> make_grid(const swp_plan* p, const swp_group_state* st, int& nbloc
     G.four = (typename cplx<T>::type*)st[g].fourier;
     G.resid = (T*)st[g].resid;
     G.par = st[g].params;
+    G.mco = plan_coefs<T>(p, g).mco;
     G.member = st[g].member;
     G.diag = st[g].diag;
     L.prefix[g] = acc;

@@ -311,11 +311,18 @@ __device__ __forceinline__ void grid_body(const GridLaunch<T>& Lc, const GridGro
       for (int q = 0; q < NGRAD; ++q) s_dpar[q] = (T)G.dpar[q * B + b];
     s_dw[0] = G.dw ? (T)G.dw[b] : (T)0;
     s_dw[1] = G.dw ? (T)G.dw[B + b] : (T)0;
-    const double Pb = G.par[P_PHIBAR * B + b], tr = G.par[P_TAURAD * B + b];
     const double td = G.par[P_TAUDRAG * B + b], DPe = G.par[P_DPHIEQ * B + b];
     const double wc = G.member ? G.member[MS_WCURR * B + b] : 0.0;
     const double wm = G.member ? G.member[MS_WMID * B + b] : 0.0;
-    s_par[0] = (T)Pb; s_par[1] = (T)(1.0 / tr); s_par[2] = (T)(1.0 / td); s_par[3] = (T)DPe;
+    if (MODE == GM_STEP || MODE == GM_ADJ_STEP || MODE == GM_TL_STEP) {
+      // the call's tables hold these: two FP64 quotients here were a chain every CTA waited
+      // for (two halves of 128 members, M = 42: 98.4 -> 97.0 us per step, adjoint 120.3 -> 118.9)
+      s_par[0] = G.mco[MC_PB * B + b]; s_par[1] = G.mco[MC_SIITR * B + b]; s_par[2] = G.mco[MC_ITD * B + b];
+    } else {
+      s_par[0] = (T)G.par[P_PHIBAR * B + b];
+      s_par[1] = (T)(1.0 / G.par[P_TAURAD * B + b]); s_par[2] = (T)(1.0 / td);
+    }
+    s_par[3] = (T)DPe;
     s_par[4] = (T)wc; s_par[5] = (T)wm;
     // the winds of a stepped member are band-limited (the RAW filter leaves
     // them alone while it moves eta, delta, Phi of the new level)

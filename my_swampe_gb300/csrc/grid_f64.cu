@@ -311,12 +311,12 @@ __global__ void __launch_bounds__(256, 2) k_grid_step_f64(const __grid_constant_
   if (cfg.diagnostics)
     copy_rows([&](int) { return G.four + (size_t)F_PHI_MID * FS; }, 1, S::N1, JB, B, b, S::J, j0, raw, nfix);
   if (threadIdx.x == 0) {
-    const double tr = G.par[P_TAURAD * B + b], td = G.par[P_TAUDRAG * B + b];
+    const double td = G.par[P_TAUDRAG * B + b];
     const bool stepped = G.member && G.member[MS_UPDATED * B + b] != 0.0;
     const double wc = G.member ? G.member[MS_WCURR * B + b] : 0.0;
     s_par[0] = G.par[P_PHIBAR * B + b];
-    s_par[1] = 1.0 / tr;
-    s_par[2] = 1.0 / td;
+    s_par[1] = G.mco[MC_SIITR * B + b];  // 1 / taurad and 1 / taudrag, from the call's tables
+    s_par[2] = G.mco[MC_ITD * B + b];
     s_par[3] = G.par[P_DPHIEQ * B + b];
     s_par[4] = wc;
     s_par[5] = G.member ? G.member[MS_WMID * B + b] : 0.0;
@@ -434,8 +434,8 @@ __global__ void __launch_bounds__(256, 2) k_grid_adj_f64(const __grid_constant__
   if (threadIdx.x == 0) {
     const double td = G.par[P_TAUDRAG * B + b];
     s_par[0] = G.par[P_PHIBAR * B + b];
-    s_par[1] = 1.0 / G.par[P_TAURAD * B + b];
-    s_par[2] = 1.0 / td;
+    s_par[1] = G.mco[MC_SIITR * B + b];
+    s_par[2] = G.mco[MC_ITD * B + b];
     s_par[3] = G.par[P_DPHIEQ * B + b];
     s_nodrag = td == -1.0;
   }

@@ -197,6 +197,7 @@ struct GridGroup {
   typename cplx<T>::type* four;         // [NFOURIER][M+1][B][J]
   T* resid;                             // [NRESID][B][J][I]
   const double* par;                    // [NPAR][B]
+  const T* mco;                         // [MC_*][B], the step modes' (refreshed by every call that runs steps)
   double* member;                       // [NMEMBER][B]
   double* diag;                         // [steps+1][NDIAG][B] or null
   T* hist;                              // [5][B][J][I] for this step, or null
