@@ -244,6 +244,19 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS)
 // are added in a fixed order, and neither they nor the scales of a member depend
 // on the other members of its tile.
 //
+// The slices' error is a part of the product of the rows' scales, below npix 2^-59
+// of it, and not of what the products add up to: a coefficient whose row is
+// non-zero only where the map is faint (a sector, the night side, a patch) could
+// lose every digit.  So the products of the top digits' magnitudes are summed
+// beside the result (a 37th MMA a step): each is at most four times the product of
+// the elements' magnitudes, and where their sum does not reach PR_GUARD, so that
+// sum |P r| is not shown to reach the product of the scales, the output is taken
+// again with FP64 FMAs (a warp, lanes over pixels), as is any whose scales are near
+// the ends of FP64's range, infinite or NaN.  An output of slices is then within
+// npix 2^-59 sum |P r| and its roundings, one of FMAs within npix / 32 2^-53
+// sum |P r|.  Of the sums over a whole disc, which the guard leaves alone, none
+// comes near it.
+//
 // FP64 FMAs took 475 us for 256 members (M = 42, 121 coefficients), 96% of the
 // FP64 pipe.  64 coefficients a CTA rather than 128: twice the CTAs for small
 // ensembles, two CTAs per SM.
@@ -252,14 +265,21 @@ constexpr int PR_KMAX = 8192;                  // pixels of a CTA per forced con
 constexpr int PR_ROW = PR_KC / 2 + 4;          // words of a sliced member row, padded: conflict-free B fragments
 constexpr int PR_LD = PR_KC + 8;               // doubles of a staged row, padded: conflict-free A fragments
 constexpr int PR_ROWS = PR_COEF + PR_MEMB;     // staged rows of a buffer: coefficients, then members
+constexpr float PR_GUARD = 32768.0f;  // top-digit products: 2^-2 of it in units of 2^112 reaches 2^124, a scale's square
 struct ProjectSmem {
   union {
     double stage[2][PR_ROWS][PR_LD];
-    double part[2][PR_COEF][PR_MEMB + 1];  // the halves' results, once the last chunk is read
+    struct {  // the halves' results, once the last chunk is read
+      double part[2][PR_COEF][PR_MEMB + 1];
+      float mag[2][PR_COEF][PR_MEMB + 1];  // sums of the top digits' magnitudes
+      int ec[2][PR_COEF];                  // coefficient scales
+    };
   };
   uint32_t dig[slices::ND][PR_MEMB][PR_ROW];
   int er[2][PR_MEMB];  // member scales: current, and before this chunk
 };
+// 2^-n, n >= 0; zero beyond FP32's normal range
+__device__ __forceinline__ float pow2_down(int n) { return __int_as_float(max(127 - n, 0) << 23); }
 // VEC: 16-byte copies (every row starts on 16 bytes)
 template <bool VEC>
 __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS, 2)
@@ -301,6 +321,7 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS, 2)
   Tile tile[2];
   tile[0].reset();
   tile[1].reset();
+  float mag[2][4] = {};
   if (threadIdx.x < PR_MEMB) S.er[0][threadIdx.x] = S.er[1][threadIdx.x] = 0;
   stage(0, k0);
   int buf = 0;
@@ -341,9 +362,11 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS, 2)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int c = 8 * n + 2 * t + (e & 1), h = e >> 1;
+          const int rise = en[h] - ea[h] + S.er[0][c] - S.er[1][c];
           if (force || en[h] != ea[h] || S.er[0][c] != S.er[1][c]) {
             res[n][e] += value(tile[n].hi[e], tile[n].lo[e], ea[h], S.er[1][c]);
             tile[n].hi[e] = tile[n].lo[e] = 0;
+            mag[n][e] *= pow2_down(rise);  // to the new scales
           }
         }
     }
@@ -374,6 +397,12 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS, 2)
           const uint32_t* bp = &S.dig[0][8 * n + g][16 * half + 8 * ks + t];
           load_b(bf, bp, bp + 4, PR_MEMB * PR_ROW);
           tile[n].step(a, bf);
+          uint32_t am[4], bm[2];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) am[q] = a[0][q] & 0x7fff7fffu;
+#pragma unroll
+          for (int q = 0; q < 2; ++q) bm[q] = bf[0][q] & 0x7fff7fffu;
+          mma(mag[n], am, bm);
         }
       }
       tile[0].flush();
@@ -389,17 +418,53 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS, 2)
       const int c = 8 * n + 2 * t + (e & 1);
       if (k1 > k0) res[n][e] += value(tile[n].hi[e], tile[n].lo[e], ea[e >> 1], S.er[0][c]);
       S.part[half][mt * 16 + g + 8 * (e >> 1)][c] = res[n][e];
+      S.mag[half][mt * 16 + g + 8 * (e >> 1)][c] = mag[n][e];
     }
+  if (t == 0) {
+    S.ec[half][mt * 16 + g] = ea[0];
+    S.ec[half][mt * 16 + g + 8] = ea[1];
+  }
   cl.sync();
-  // an eighth of the coefficients per rank: the sum over ranks and halves, in order
-  for (int i = threadIdx.x; i < PR_COEF * PR_MEMB / EM_CL; i += EM_THREADS) {
-    const int c = rank * (PR_COEF / EM_CL) + i % (PR_COEF / EM_CL), r = i / (PR_COEF / EM_CL);
+  // every eighth coefficient per rank: the sum over ranks and halves, in order
+  static_assert(PR_COEF * PR_MEMB / EM_CL == EM_THREADS / 2, "an output per thread of four warps");
+  bool again = false;
+  int c = 0, r = 0;
+  if (threadIdx.x < PR_COEF * PR_MEMB / EM_CL) {
+    c = rank + EM_CL * (threadIdx.x % (PR_COEF / EM_CL));
+    r = threadIdx.x / (PR_COEF / EM_CL);
     double s = 0.0;
+    float m = 0.0f, mq[EM_CL];
+    int top = 0, sq[EM_CL];
+#pragma unroll
     for (int q = 0; q < EM_CL; ++q) {
-      const double* p = cl.map_shared_rank(&S.part[0][c][r], q);
-      s += p[0] + p[PR_COEF * (PR_MEMB + 1)];
+      const ProjectSmem* p = cl.map_shared_rank(&S, q);
+      s += p->part[0][c][r] + p->part[1][c][r];
+      const int e0 = p->ec[0][c], e1 = p->ec[1][c], e = max(e0, e1);
+      sq[q] = p->er[0][r] + e;
+      mq[q] = p->mag[0][c][r] * pow2_down(e - e0) + p->mag[1][c][r] * pow2_down(e - e1);
+      top = max(top, sq[q]);
     }
-    if (c0 + c < ncoef && r < nm) yraw[(size_t)(b0 + r) * ncoef + c0 + c] = s;
+#pragma unroll
+    for (int q = 0; q < EM_CL; ++q) m += mq[q] * pow2_down(top - sq[q]);
+    const bool out = c0 + c < ncoef && r < nm;
+    // scales within 2^1200 and 2^3000: no partial sum was cut off at either end (value())
+    again = out && !(m >= PR_GUARD && top >= 1200 && top <= 3000);
+    if (out && !again) yraw[(size_t)(b0 + r) * ncoef + c0 + c] = s;
+  }
+  // the outputs below the guard, spread over the CTA's warps
+  __shared__ int s_again[PR_COEF * PR_MEMB / EM_CL], s_nagain;
+  if (threadIdx.x == 0) s_nagain = 0;
+  __syncthreads();
+  if (again) s_again[atomicAdd(&s_nagain, 1)] = (c0 + c) * PR_MEMB + r;
+  __syncthreads();
+  for (int i = warp; i < s_nagain; i += EM_WARPS) {
+    const int cc = s_again[i] / PR_MEMB, bb = b0 + s_again[i] % PR_MEMB;
+    const double *x = rhs + (size_t)bb * npix, *w = P + (size_t)cc * npix;
+    double s = 0.0;
+#pragma unroll 8
+    for (int p = lane; p < npix; p += 32) s = fma(w[p], x[p], s);
+    s = warp_sum(s);
+    if (lane == 0) yraw[(size_t)bb * ncoef + cc] = s;
   }
   cl.sync();
 }
