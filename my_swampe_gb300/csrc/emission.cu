@@ -22,6 +22,7 @@
 // run to run.  Non-finite inputs give all-NaN outputs per member, as the
 // reference's lax.cond guards do.
 #include <cmath>
+#include <type_traits>
 #include <cooperative_groups.h>
 #include "slices.cuh"
 #include "swp_internal.h"
@@ -234,8 +235,8 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS)
 }
 
 // Y[b][c] = sum_p P[c][p] rhs[b][p] on the FP16 tensor cores (slices.cuh): a
-// cluster of EM_CL CTAs takes 16 members and 64 coefficients, each CTA an eighth
-// of the pixels, 64 at a time (cp.async, double-buffered).  A warp owns 16
+// cluster of EM_CL CTAs takes 16 members and PR_COEF (32 or 64) coefficients, each
+// CTA an eighth of the pixels, 64 at a time (cp.async, double-buffered).  A warp owns 16
 // coefficients and half of a chunk: it slices its projector rows in registers,
 // in the fragment layout; the members' rows are sliced into shared memory by
 // all threads.  A row's scale is the largest exponent it has shown so far: a
@@ -258,17 +259,16 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS)
 // comes near it.
 //
 // FP64 FMAs took 475 us for 256 members (M = 42, 121 coefficients), 96% of the
-// FP64 pipe.  64 coefficients a CTA rather than 128: twice the CTAs for small
-// ensembles, two CTAs per SM.
-constexpr int PR_MEMB = 16, PR_COEF = 64, PR_KC = 64;  // members, coefficients, pixels per chunk
+// FP64 pipe.  At most 64 coefficients a CTA, for two CTAs per SM.
+constexpr int PR_MEMB = 16, PR_KC = 64;        // members, pixels per chunk
 constexpr int PR_KMAX = 8192;                  // pixels of a CTA per forced conversion (integer range of the sums)
 constexpr int PR_ROW = PR_KC / 2 + 4;          // words of a sliced member row, padded: conflict-free B fragments
 constexpr int PR_LD = PR_KC + 8;               // doubles of a staged row, padded: conflict-free A fragments
-constexpr int PR_ROWS = PR_COEF + PR_MEMB;     // staged rows of a buffer: coefficients, then members
 constexpr float PR_GUARD = 32768.0f;  // top-digit products: 2^-2 of it in units of 2^112 reaches 2^124, a scale's square
+template <int PR_COEF>
 struct ProjectSmem {
   union {
-    double stage[2][PR_ROWS][PR_LD];
+    double stage[2][PR_COEF + PR_MEMB][PR_LD];  // coefficients, then members
     struct {  // the halves' results, once the last chunk is read
       double part[2][PR_COEF][PR_MEMB + 1];
       float mag[2][PR_COEF][PR_MEMB + 1];  // sums of the top digits' magnitudes
@@ -281,23 +281,25 @@ struct ProjectSmem {
 // 2^-n, n >= 0; zero beyond FP32's normal range
 __device__ __forceinline__ float pow2_down(int n) { return __int_as_float(max(127 - n, 0) << 23); }
 // VEC: 16-byte copies (every row starts on 16 bytes)
-template <bool VEC>
+template <bool VEC, int PR_COEF>
 __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS, 2)
     k_emission_project(const double* __restrict__ rhs, int B, int npix, const double* __restrict__ P, int ncoef,
                        double* __restrict__ yraw) {
   using namespace slices;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  ProjectSmem& S = *reinterpret_cast<ProjectSmem*>(smem_raw);
+  constexpr int PR_ROWS = PR_COEF + PR_MEMB, NMT = PR_COEF / 16;  // staged rows; coefficient tiles
+  typedef ProjectSmem<PR_COEF> Smem;
+  Smem& S = *reinterpret_cast<Smem*>(smem_raw);
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int mt = warp & 3, half = warp >> 2;
+  const int mt = warp % NMT, half = (warp / NMT) & 1;  // warps from 2 NMT on only stage and slice members
   const int c0 = (blockIdx.x / EM_CL) * PR_COEF, b0 = blockIdx.y * PR_MEMB;
   const int nm = min(PR_MEMB, B - b0), nn = nm > 8 ? 2 : 1;
   // this CTA's pixels: a multiple of the chunk but for the last
   const int per = ((npix + EM_CL * PR_KC - 1) / (EM_CL * PR_KC)) * PR_KC;
   const int k0 = min(rank * per, npix), k1 = min(k0 + per, npix);
-  const bool busy = c0 + mt * 16 < ncoef;
+  const bool busy = warp < 2 * NMT && c0 + mt * 16 < ncoef;
   // rows beyond the last coefficient or member, and pixels beyond the end, are zero
   constexpr int STEP = VEC ? 2 : 1, NS = PR_KC / STEP;  // a thread copies the same pixels of every EM_THREADS / NS rows
   const int sk = (threadIdx.x % NS) * STEP;
@@ -412,7 +414,8 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS, 2)
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll
-  for (int n = 0; n < 2; ++n)
+  for (int n = 0; n < 2; ++n) {
+    if (warp >= 2 * NMT) break;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int c = 8 * n + 2 * t + (e & 1);
@@ -420,13 +423,14 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS, 2)
       S.part[half][mt * 16 + g + 8 * (e >> 1)][c] = res[n][e];
       S.mag[half][mt * 16 + g + 8 * (e >> 1)][c] = mag[n][e];
     }
-  if (t == 0) {
+  }
+  if (t == 0 && warp < 2 * NMT) {
     S.ec[half][mt * 16 + g] = ea[0];
     S.ec[half][mt * 16 + g + 8] = ea[1];
   }
   cl.sync();
   // every eighth coefficient per rank: the sum over ranks and halves, in order
-  static_assert(PR_COEF * PR_MEMB / EM_CL == EM_THREADS / 2, "an output per thread of four warps");
+  static_assert(PR_COEF * PR_MEMB / EM_CL <= EM_THREADS, "an output per thread");
   bool again = false;
   int c = 0, r = 0;
   if (threadIdx.x < PR_COEF * PR_MEMB / EM_CL) {
@@ -437,7 +441,7 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS, 2)
     int top = 0, sq[EM_CL];
 #pragma unroll
     for (int q = 0; q < EM_CL; ++q) {
-      const ProjectSmem* p = cl.map_shared_rank(&S, q);
+      const Smem* p = cl.map_shared_rank(&S, q);
       s += p->part[0][c][r] + p->part[1][c][r];
       const int e0 = p->ec[0][c], e1 = p->ec[1][c], e = max(e0, e1);
       sq[q] = p->er[0][r] + e;
@@ -635,13 +639,26 @@ extern "C" int swp_emission_project(const double* rhs, const int* ok, int B, int
                                     int ncoef, double* y, void* stream) {
   if (!rhs || !projector || !y || B < 1 || npix < 1 || ncoef < 1 || B > 65535) return SWP_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  dim3 grid(EM_CL * ((ncoef + PR_COEF - 1) / PR_COEF), (B + PR_MEMB - 1) / PR_MEMB);
-  auto kernel = npix % 2 == 0 && ((uintptr_t)rhs | (uintptr_t)projector) % 16 == 0 ? k_emission_project<true>
-                                                                                   : k_emission_project<false>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ProjectSmem));
-  if (e != cudaSuccess) return em_check(e);
-  kernel<<<grid, EM_THREADS, sizeof(ProjectSmem), s>>>(rhs, B, npix, projector, ncoef, y);
-  e = cudaGetLastError();
+  const bool vec = npix % 2 == 0 && ((uintptr_t)rhs | (uintptr_t)projector) % 16 == 0;
+  auto run = [&](auto vk, auto ck) {
+    constexpr int COEF = decltype(ck)::value;
+    auto kernel = k_emission_project<decltype(vk)::value, COEF>;
+    const dim3 grid(EM_CL * ((ncoef + COEF - 1) / COEF), (B + PR_MEMB - 1) / PR_MEMB);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ProjectSmem<COEF>));
+    if (e != cudaSuccess) return e;
+    kernel<<<grid, EM_THREADS, sizeof(ProjectSmem<COEF>), s>>>(rhs, B, npix, projector, ncoef, y);
+    return cudaGetLastError();
+  };
+  // 32 coefficients per CTA while those CTAs fit two per SM at once: a small ensemble's
+  // chain per chunk is shorter by half the MMAs and the slicing.  121 coefficients, M = 42,
+  // us with 64 / 32: 1 member 90 / 62, 16 members 105 / 72 (FP64 FMAs 82 and 86), 48
+  // members 105 / 72, 64 members 106 / 99, 128 members 150 / 104, 256 members 155 / 194;
+  // 36 coefficients, 256 members 141 / 98.
+  const long long small = (long long)EM_CL * ((ncoef + 31) / 32) * ((B + PR_MEMB - 1) / PR_MEMB);
+  auto by_coef = [&](auto vk) {
+    return small <= 2 * 152 ? run(vk, std::integral_constant<int, 32>()) : run(vk, std::integral_constant<int, 64>());
+  };
+  const cudaError_t e = vec ? by_coef(std::true_type()) : by_coef(std::false_type());
   if (e != cudaSuccess) return em_check(e);
   k_emission_normalise<<<(B + 7) / 8, 256, 0, s>>>(ok, B, ncoef, y);
   return em_check(cudaGetLastError());

@@ -92,6 +92,18 @@ def test_outputs_do_not_depend_on_the_tile_of_members(cuda):
         assert np.array_equal(_project(r[b:b + 1], P)[0], y[b])
 
 
+@pytest.mark.parametrize("B,ncoef", [(144, 121), (145, 129), (160, 121)])
+def test_outputs_do_not_depend_on_the_tile_of_coefficients(cuda, B, ncoef):
+    """Members of launches on both sides of the rule for coefficients per CTA, alone."""
+    rng = np.random.default_rng(B)
+    r, P = rng.uniform(0.5, 1.0, (B, 700)), rng.standard_normal((ncoef, 700))
+    P[0] = np.abs(P[0])
+    y = _project(r, P)
+    for b in (0, 31, B - 1):
+        assert np.array_equal(_project(r[b:b + 1], P)[0], y[b])
+    assert np.array_equal(_project(r, P[:40]), y[:, :40])
+
+
 @pytest.mark.parametrize("npix", [64, 128, 512])
 def test_every_digit_counts(cuda, npix):
     """Pairs of pixels whose products cancel to 2^-30: the rounding of the result is
