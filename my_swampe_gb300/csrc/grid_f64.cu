@@ -104,7 +104,8 @@ struct Mem {
 
 // Slices of the raw rows [f][m][r] (complex).  Rows of fields f < nhalf have the
 // coefficients of m >= 1 halved (adjoint rows: their weight is 1, the matrix'
-// 2).  mid: the value at longitude I/2, sum_m w_m (-1)^m Re Y_m.
+// 2).  mid: the value at longitude I/2, sum_m w_m (-1)^m Re Y_m, in integers
+// from every digit, as the tiles' sums.
 template <class S, int JB>
 __device__ __forceinline__ void slice_fourier(const double2* raw, int nrow, int nhalf, uint32_t* dig, int plane,
                                               int* er, double* mid) {
@@ -125,24 +126,25 @@ __device__ __forceinline__ void slice_fourier(const double2* raw, int nrow, int 
     e = row_exponent((int)__reduce_max_sync(0xffffffffu, (unsigned)e));
     if (lane == 0) er[row] = e;
     long long alt = 0;  // in units of 2^8 of the scale
+    int low = 0;        // and of its unit
 #pragma unroll
     for (int i = 0; i < KI; ++i) {
       const int m = lane + 32 * i, h = m ? half : 0;
       uint64_t a = fixed(y[i].x, e + h), b = fixed(y[i].y, e + h);
-      const long long q = (long long)(a - BIAS) >> 8;
-      alt += m ? ((m & 1) ? -2 * q : 2 * q) : q;
+      const long long q = (long long)(a - BIAS);
+      const int w = m ? ((m & 1) ? -2 : 2) : 1;
+      alt += w * (q >> 8);
+      low += w * (int)(q & 0xff);
       pair_exchange(a, b);
       if (S::KP % 32 == 0 || m < S::KP)
         store_digits(dig + (size_t)row * S::YW + (lane & 1) * (S::KP / 2) + (lane >> 1) + 16 * i, plane, a, b);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) alt += __shfl_xor_sync(0xffffffffu, alt, o);
-    if (lane == 0) {
-      double v = (double)alt * __hiloint2double((e - 53) << 20, 0);
-      if (e == ER_ZERO) v = 0.0;
-      if (e == ER_BAD) v = __longlong_as_double(0x7ff8000000000000ll);
-      mid[row] = v;
-    }
+    low = __reduce_add_sync(0xffffffffu, low);
+    // (alt 2^8 + low) 2^(e - 1084), times 2^15 on the scale of e + 1013: rows whose sum could
+    // overflow are NaN, as their tiles' values are
+    if (lane == 0) mid[row] = value(alt >> 9, ((alt & 511) << 23) + (long long)low * (1 << 15), e, 1013);
   }
 }
 
