@@ -866,9 +866,13 @@ def _load_state(eng: Engine, flags: "RunFlags", state0: State, test, t0: int, di
         t = torch.as_tensor(x, device=dev).detach().to(rdt)
         return t if batched else t[None]
 
-    def fo(x):  # (B, J, M+1) -> (M+1, B, J)
+    def fm(x):  # (B, J, M+1), or one member's for all
         t = torch.as_tensor(x, device=dev).detach().to(cdt)
-        return rep((t if batched else t[None]).permute(2, 0, 1))
+        t = t if batched else t[None]
+        return t.expand(member.shape[1] // copies, *t.shape[1:])
+
+    def fo(x):  # (B, J, M+1) -> (M+1, B, J)
+        return rep(fm(x).permute(2, 0, 1))
 
     def rep(x):  # members: axis 1
         return x if copies == 1 else x.repeat(1, copies, *[1] * (x.dim() - 2))
@@ -885,8 +889,7 @@ def _load_state(eng: Engine, flags: "RunFlags", state0: State, test, t0: int, di
     filtered = bool(flags.semi_implicit or flags.raw_filter)
     # the 16 given fields in slot order, in one copy
     by_slot = dict([(slot, name) for name, slot in _STATE_SLOTS] + list(zip(_PREV_SLOTS, _PREV_NAMES)))
-    x = [torch.as_tensor(getattr(state0, by_slot[k]), device=dev).detach().to(cdt) for k in range(len(by_slot))]
-    x = rep(torch.stack(x if batched else [v[None] for v in x]))  # (16, B, J, M+1)
+    x = rep(torch.stack([fm(getattr(state0, by_slot[k])) for k in range(len(by_slot))]))  # (16, B, J, M+1)
     four[:len(by_slot)].copy_(x.permute(0, 3, 1, 2))
     for ps, ms in zip(_PREV_SLOTS, _MID_SLOTS):
         if filtered:  # the Fourier prev carry is the filtered lineage
@@ -917,7 +920,7 @@ def _load_state(eng: Engine, flags: "RunFlags", state0: State, test, t0: int, di
         member[_lib.MS_WMID].copy_(w1)
         member[_lib.MS_UPDATED].copy_(stepped.to(member.dtype))
     dead = torch.as_tensor(state0.dead, device=dev).reshape(1, -1).to(member.dtype)
-    member[_lib.MS_DEAD].copy_(rep(dead)[0].expand(member.shape[1]))
+    member[_lib.MS_DEAD].copy_(rep(dead.expand(1, member.shape[1] // copies))[0])
     # stepped members advance by increments from the first step (fast precision);
     # the semi-implicit scheme takes its lagged remainders from the state
     return t0 - 1 if (flags.semi_implicit or bool(stepped.all())) else t0
