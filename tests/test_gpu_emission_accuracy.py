@@ -1,6 +1,7 @@
 """Accuracy of the emission kernels output by output: the projection onto bases
 of local support, whose coefficients see only a faint part of the map, against
-the FP64 bound of each sum; the digits that the sliced projection keeps."""
+the FP64 bound of each sum; the digits that the sliced projection keeps; the
+Planck intensity relative to its own size."""
 import numpy as np
 import pytest
 import torch
@@ -126,3 +127,26 @@ def test_every_digit_counts(cuda, npix):
     want = pair.sum(axis=2) / rl[:, :1]
     bound = (npix * 2.0**-59 + 24 * U * np.abs(pair).sum(axis=2)) / r[:, :1]
     assert np.all(np.abs(y - want)[:, 1:] <= bound[:, 1:].astype(np.float64))
+
+
+@pytest.mark.parametrize("x_clip", [80.0, 700.0, 0.5])
+def test_planck_intensity_relative_accuracy(cuda, x_clip):
+    """1 / (expm1(x) + tiny) at x = h c / (lambda kB T) from 10^-6 to past 700.  x carries two roundings, each kappa = x e^x / (e^x - 1) times in
+    the intensity; its expm1, sum and reciprocal four ulp."""
+    from my_swampe_gb300.emission import EmissionConfig, temperature_to_intensity
+
+    ld = np.longdouble
+    hck = ld("6.62607015e-34") * ld("299792458.0") / ld("1.380649e-23")
+    x = np.concatenate([10.0 ** np.linspace(-6, np.log10(709.0), 4096), np.linspace(0.002, 0.03, 4096),
+                        np.linspace(695.0, 1100.0, 4096)])
+    T = (hck / (ld(4.5e-6) * x)).astype(np.float64)
+    cfg = EmissionConfig(emission_model="planck", planck_x_clip=x_clip, Tmin_K=1e-3)
+    got = temperature_to_intensity(torch.tensor(T.reshape(96, 128), device="cuda"), cfg).cpu().numpy().reshape(-1)
+    xe = np.minimum(np.maximum(hck / (ld(4.5e-6) * T.astype(ld)), 0), ld(x_clip))
+    with np.errstate(over="ignore"):
+        want = 1 / (np.expm1(xe) + ld(1e-30))
+        kappa = np.abs(xe / (1 - np.exp(-xe)))
+    # beyond 709.7 expm1 overflows in FP64 and the intensity, below 10^-307, is lost
+    small = xe > 709.0
+    assert np.all(np.abs(got / want - 1)[~small] <= ((kappa + 4) * 2 * U)[~small])
+    assert np.all(np.abs(got - want)[small] <= 2e-308)
