@@ -127,14 +127,17 @@ __device__ __forceinline__ double planck_rel(double x, const double* __restrict_
   const double q = fma(e2, t1, e2 - 1.0);
   return 1.0 / (fma(q + 1.0, p, q) + 1.0e-30);
 }
-// v: Phi, or T (c.input 1)
+// v: Phi, or T (c.input 1).  ANY_X: x_clip is outside planck_rel's range
+template <bool ANY_X>
 __device__ __forceinline__ double planck_bands(const EmCfg& c, double v, double Phibar,
                                                const double* __restrict__ tm1) {
   const double p0 = c.input == 0 && c.temp_mode == 0 ? Phibar : c.p0;
   const double u = c.input != 0 ? v : c.folded ? fmax(p0 + v, c.pmin) : temperature(c, v, Phibar);
   double out = 0.0;
-  for (int k = 0; k < c.nbands; ++k)
-    out += c.bw[k] * planck_rel(fmin(fmax(c.pl[k] / u, 0.0), c.x_clip), tm1);
+  for (int k = 0; k < c.nbands; ++k) {
+    const double x = fmin(fmax(c.pl[k] / u, 0.0), c.x_clip);
+    out += c.bw[k] * (ANY_X ? 1.0 / (expm1(x) + 1.0e-30) : planck_rel(x, tm1));
+  }
   return out;
 }
 
@@ -148,6 +151,7 @@ __device__ __forceinline__ double planck_bands(const EmCfg& c, double v, double 
 // FP64-bound (see EM_CL).  The Planck argument takes one division (T itself is
 // not formed), finiteness is tested on the exponent bits, the square root of a
 // weight is taken once per row, with the quotient by the mean folded into it.
+template <bool ANY_X>
 __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS)
     k_emission_map(const double* __restrict__ in, const double* __restrict__ Phibar, int J, int I,
                    const double* __restrict__ w_lat, const __grid_constant__ EmCfg c, int stage,
@@ -194,7 +198,7 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS)
         v = qnan;
       } else if (c.input < 2) {
         if (stage > 0 && c.model == 1) {
-          v = planck_bands(c, v, pb, tm1);
+          v = planck_bands<ANY_X>(c, v, pb, tm1);
         } else {
           if (c.input == 0) v = temperature(c, v, pb);
           if (stage > 0) {
@@ -623,7 +627,7 @@ extern "C" int swp_emission_map(const double* in, const double* Phibar, int B, i
   const double div = cfg->temp_mode == 0 ? cfg->R_d : cfg->phi_to_T_scale;
   c.folded = input == 0 && div >= 1.0;
   const long double scale = c.folded ? div : 1.0L;
-  c.x_clip = cfg->x_clip < 700.0 ? cfg->x_clip : 700.0;
+  c.x_clip = cfg->x_clip;
   c.p0 = c.folded && cfg->temp_mode == 1 ? (double)(cfg->T_ref * scale) : 0.0;
   c.pmin = (double)(cfg->Tmin * scale);
   for (int k = 0; k < SWP_EMISSION_MAX_BANDS; ++k) {
@@ -631,7 +635,8 @@ extern "C" int swp_emission_map(const double* in, const double* Phibar, int B, i
     c.bw[k] = k < c.nbands ? cfg->band_weights[k] : 0.0;
   }
   for (int j = 0; j < EXP_N; ++j) c.tm1[j] = (double)(exp2l((long double)j / EXP_N) - 1.0L);
-  k_emission_map<<<EM_CL * B, EM_THREADS, 0, (cudaStream_t)stream>>>(in, Phibar, J, I, w_lat, c, stage, out, ok);
+  auto kernel = cfg->x_clip >= 0.0 && cfg->x_clip <= 700.0 ? k_emission_map<false> : k_emission_map<true>;
+  kernel<<<EM_CL * B, EM_THREADS, 0, (cudaStream_t)stream>>>(in, Phibar, J, I, w_lat, c, stage, out, ok);
   return em_check(cudaGetLastError());
 }
 

@@ -129,9 +129,10 @@ def test_every_digit_counts(cuda, npix):
     assert np.all(np.abs(y - want)[:, 1:] <= bound[:, 1:].astype(np.float64))
 
 
-@pytest.mark.parametrize("x_clip", [80.0, 700.0, 0.5])
+@pytest.mark.parametrize("x_clip", [80.0, 700.0, 1000.0, 0.5, -1.0, -800.0])
 def test_planck_intensity_relative_accuracy(cuda, x_clip):
-    """1 / (expm1(x) + tiny) at x = h c / (lambda kB T) from 10^-6 to past 700.  x carries two roundings, each kappa = x e^x / (e^x - 1) times in
+    """1 / (expm1(x) + tiny) at x = h c / (lambda kB T) from 10^-6 to past 709, where
+    expm1 overflows.  x carries two roundings, each kappa = x e^x / (e^x - 1) times in
     the intensity; its expm1, sum and reciprocal four ulp."""
     from my_swampe_gb300.emission import EmissionConfig, temperature_to_intensity
 
