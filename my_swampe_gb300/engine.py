@@ -56,16 +56,17 @@ class RunFlagsC:
         )
 
 
-def stack_values(vals: Sequence, device) -> torch.Tensor:
+def stack_values(vals: Sequence, device, n: Optional[int] = None) -> torch.Tensor:
     """Values (floats, 0-d or length-n tensors or sequences) as one float64
-    (len(vals), n) tensor, n = 1 if all are scalars; detached.  The floats cross
-    to the device in one copy."""
+    (len(vals), n) tensor, detached; by default n is their common length, 1 if all
+    are scalars.  The floats cross to the device in one copy."""
     is_float = [isinstance(v, (int, float)) for v in vals]
     floats = iter(torch.tensor([float(v) for v, f in zip(vals, is_float) if f], dtype=torch.float64,
                                device=device).unbind(0)) if any(is_float) else iter(())
     ts = [next(floats) if f else torch.as_tensor(v, dtype=torch.float64, device=device).detach()
           for v, f in zip(vals, is_float)]
-    n = max([t.numel() for t in ts if t.dim()], default=1)
+    if n is None:
+        n = max([t.numel() for t in ts if t.dim()], default=1)
     return torch.stack([t.expand(n) if t.dim() == 0 else t.reshape(n) for t in ts])
 
 
@@ -251,7 +252,7 @@ class Engine:
         gd = self.groups[g]
         # values only: a parameter's gradient or tangent flows through adjoint.integrate
         if len(kw) == len(PARAM_NAMES):  # all of them: one launch instead of one per parameter
-            gd["params"].copy_(stack_values([kw[k] for k in PARAM_NAMES], self.device).expand(-1, gd["B"]))
+            gd["params"].copy_(stack_values([kw[k] for k in PARAM_NAMES], self.device, gd["B"]))
             return
         for name, v in kw.items():
             row = PARAM_NAMES.index(name)

@@ -683,9 +683,9 @@ def _run_split(M, B, precision, device, flags: RunFlagsC, t0: int, T: int, ics: 
     dev = eng.device
     sls = (slice(0, sizes[0]), slice(sizes[0], B))
 
-    rows = stack_values([pvals[k] for k in PARAM_NAMES], dev)
+    rows = stack_values([pvals[k] for k in PARAM_NAMES], dev, B)
     for gd, sl in zip(eng.groups, sls):
-        gd["params"].copy_(rows[:, sl] if rows.shape[1] > 1 else rows.expand(-1, gd["B"]))
+        gd["params"].copy_(rows[:, sl])
     ics_g = [ics[:, sl] for sl in sls]
     eng.init_state([x.detach() for x in ics_g], flags)
     # pass-through carries of the semi-implicit scheme's State fields: F + U / taudrag of the initial state
@@ -1014,8 +1014,8 @@ class _ScanLastFn(torch.autograd.Function):
         else:
             B = ctl["B"]
             eng = _engine_for(eng.groups[0]["M"], copies * B, eng.precision, eng.device, steps=False)
-            vals = stack_values([ctl["vals"][k] for k in PARAM_NAMES], eng.device)
-            eng.groups[0]["params"].copy_(vals.expand(-1, B).repeat(1, copies))
+            vals = stack_values([ctl["vals"][k] for k in PARAM_NAMES], eng.device, B)
+            eng.groups[0]["params"].copy_(vals.repeat(1, copies))
         t_start = _load_state(eng, flags, state0, test, t0, copies=copies)
         fc = _flags_c(flags, test, t_start, diagnostics=False)
         tfour, tresid, _ = eng.new_tangent_buffers()

@@ -1,0 +1,30 @@
+"""The forms of the parameters that build_static and set_params take, and what
+a Static record shares: nothing with the next one."""
+import dataclasses
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+BASE = dict(dt=600.0, a=8.2e7, omega=3.2e-5, g=9.8, Phibar=3.0e5, taurad=36000.0, taudrag=21600.0, DPhieq=1.0e6,
+            K6=1.24e33, K6Phi=None)
+
+
+def _build(**kw):
+    from my_swampe_gb300.model import build_static
+
+    return build_static(M=42, test=None, **dict(BASE, **kw))
+
+
+def test_set_params_refuses_another_length(cuda):
+    from my_swampe_gb300.engine import PARAM_NAMES, Engine
+
+    eng = Engine([(42, 3)], "fp64")
+    kw = {k: 1.0 for k in PARAM_NAMES}
+    for bad in (torch.tensor([1.0]), torch.tensor([1.0, 2.0])):
+        with pytest.raises(RuntimeError):
+            eng.set_params(0, **dict(kw, taurad=bad))
+    eng.set_params(0, **dict(kw, taurad=torch.tensor([1.0, 2.0, 3.0])))
+    assert eng.groups[0]["params"][4].tolist() == [1.0, 2.0, 3.0]
