@@ -217,6 +217,22 @@ def _scalar_tensor(x, dev):
     return torch.as_tensor(x, dtype=torch.float64, device=dev)
 
 
+def _plain_values(vals) -> bool:
+    """Whether parameters are what the table kernel takes: values without a
+    derivative, scalars and vectors of one length."""
+    lengths = set()
+    for x in vals:
+        if _is_python_scalar(x):
+            continue
+        if _tracked(x):
+            return False
+        shape = torch.as_tensor(x).shape
+        if len(shape) > 1:
+            return False
+        lengths.update(shape)
+    return len(lengths) < 2 and 0 not in lengths
+
+
 def build_static(*, M, dt, a, omega, g, Phibar, taurad, taudrag, DPhieq, K6, K6Phi, test, engine: Optional[Engine] = None) -> Static:
     """``model.py:457-557`` on the GPU (FP64).  Scalars may be per-member vectors."""
     eng = engine if engine is not None else _geometry_engine(int(M))
@@ -231,10 +247,10 @@ def build_static(*, M, dt, a, omega, g, Phibar, taurad, taudrag, DPhieq, K6, K6P
                  mJarray=geo["m"][None, :].expand(J, M + 1), narray=geo["nn1"][None, :].expand(M + 1, N + 1), test=test)
     given = dict(dt=dt, a=a, omega=omega, g=g, Phibar=Phibar, taurad=taurad, taudrag=taudrag, DPhieq=DPhieq, K6=K6,
                  K6Phi=K6 if K6Phi is None else K6Phi)
-    if not any(_tracked(v) for v in given.values()):
+    if _plain_values(given.values()):
         v = stack_values(list(given.values()), dev)
         t = eng.static_tables(0, v, test is None)
-        one = not any(torch.is_tensor(x) and x.dim() or np.ndim(x) for x in given.values())
+        one = not any(torch.as_tensor(x).dim() for x in given.values())
         if one:  # scalars: no member axis
             t = {k: x[0] for k, x in t.items()}
         row = lambda x: x[..., None, :].expand(*x.shape[:-1], M + 1, N + 1)  # noqa: E731
@@ -245,7 +261,7 @@ def build_static(*, M, dt, a, omega, g, Phibar, taurad, taudrag, DPhieq, K6, K6P
                       sigma_exp=row(t["sigma_exp"]), sigmaPhi_exp=row(t["sigmaPhi_exp"]),
                       # unforced: zero, without a member axis
                       Phieq=t["Phieq"] if one or test is None else t["Phieq"][0])
-    # tracked parameters: tensor expressions, which carry their derivatives
+    # tensor expressions: they carry the derivatives of tracked parameters, and broadcast
     vals = [_scalar_tensor(v, dev) for v in given.values()]
     if any(v.dim() for v in vals):  # ensemble: broadcast every scalar to the member axis
         Bn = max(v.shape[0] for v in vals if v.dim())

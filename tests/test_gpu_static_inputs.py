@@ -18,6 +18,18 @@ def _build(**kw):
     return build_static(M=42, test=None, **dict(BASE, **kw))
 
 
+def test_one_value_beside_an_ensemble(cuda):
+    """A (1,) parameter broadcasts against (B,) ones, and keeps its shape."""
+    v = torch.tensor([3.0e4, 5.0e4, 9.0e4], dtype=torch.float64, device="cuda")
+    one = torch.tensor([2.0e6], dtype=torch.float64, device="cuda")
+    got, want = _build(taurad=v, DPhieq=one), _build(taurad=v, DPhieq=one.expand(3))
+    assert got.DPhieq.shape == (1,) and got.taurad.shape == (3,)
+    for f in dataclasses.fields(got):
+        x, y = getattr(got, f.name), getattr(want, f.name)
+        if torch.is_tensor(y):
+            assert torch.all((x - y).abs() <= 40 * 2.3e-16 * y.abs()), f.name
+
+
 def test_set_params_refuses_another_length(cuda):
     from my_swampe_gb300.engine import PARAM_NAMES, Engine
 
