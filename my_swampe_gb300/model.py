@@ -253,8 +253,15 @@ def build_static(*, M, dt, a, omega, g, Phibar, taurad, taudrag, DPhieq, K6, K6P
         one = not any(torch.as_tensor(x).dim() for x in given.values())
         if one:  # scalars: no member axis
             t = {k: x[0] for k, x in t.items()}
+
+        def carried(x, r):  # a given tensor is the record's own, also one that requires grad (under no_grad)
+            if not torch.is_tensor(x):
+                return r[0] if one else r
+            x = _scalar_tensor(x, dev)
+            return x if one or x.dim() else x.expand(v.shape[1])
+
         row = lambda x: x[..., None, :].expand(*x.shape[:-1], M + 1, N + 1)  # noqa: E731
-        return Static(**const, **{k: x[0] if one else x for k, x in zip(given, v)}, fmn=t["fmn"],
+        return Static(**const, **{k: carried(x, r) for (k, x), r in zip(given.items(), v)}, fmn=t["fmn"],
                       tstepcoeff=t["tsc"][..., None].expand(*t["tsc"].shape, M + 1),
                       tstepcoeff2=t["tsc2"][..., None].expand(*t["tsc2"].shape[:-1], J, M + 1),
                       tstepcoeffmn=row(t["tc"]), sigma=row(t["sigma"]), sigmaPhi=row(t["sigmaPhi"]),

@@ -30,6 +30,15 @@ def test_one_value_beside_an_ensemble(cuda):
             assert torch.all((x - y).abs() <= 40 * 2.3e-16 * y.abs()), f.name
 
 
+def test_given_tensors_are_carried_as_they_are(cuda):
+    """A tensor parameter is the record's own: also one that requires grad, given under no_grad."""
+    p = torch.tensor([3.0e4, 5.0e4], dtype=torch.float64, device="cuda", requires_grad=True)
+    q = torch.tensor(2.0e4, dtype=torch.float64, device="cuda")
+    with torch.no_grad():
+        s = _build(taurad=p, taudrag=q)
+    assert s.taurad.requires_grad and s.taurad is p and s.taudrag.shape == (2,) and torch.equal(s.taudrag[1], q)
+
+
 def test_set_params_refuses_another_length(cuda):
     from my_swampe_gb300.engine import PARAM_NAMES, Engine
 
