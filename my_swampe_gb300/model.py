@@ -219,12 +219,13 @@ def _scalar_tensor(x, dev):
 
 def _plain_values(vals) -> bool:
     """Whether parameters are what the table kernel takes: values without a
-    derivative, scalars and vectors of one length."""
+    derivative or a function transform's wrapper (torch.func.vmap), scalars and
+    vectors of one length."""
     lengths = set()
     for x in vals:
         if _is_python_scalar(x):
             continue
-        if _tracked(x):
+        if torch.is_tensor(x) and torch._C._functorch.is_functorch_wrapped_tensor(x) or _tracked(x):
             return False
         shape = torch.as_tensor(x).shape
         if len(shape) > 1:

@@ -30,6 +30,15 @@ def test_one_value_beside_an_ensemble(cuda):
             assert torch.all((x - y).abs() <= 40 * 2.3e-16 * y.abs()), f.name
 
 
+def test_under_vmap(cuda):
+    v = torch.tensor([1.0e6, 2.0e6], dtype=torch.float64, device="cuda")
+    Phieq, sigma = torch.func.vmap(lambda DP, K: (lambda s: (s.Phieq, s.sigma_exp))(_build(DPhieq=DP, K6=K)))(v, v * 1e27)
+    for b in range(2):
+        s = _build(DPhieq=v[b], K6=v[b] * 1e27)
+        torch.testing.assert_close(Phieq[b], s.Phieq, rtol=1e-14, atol=0)
+        torch.testing.assert_close(sigma[b], s.sigma_exp, rtol=1e-14, atol=0)
+
+
 def test_given_tensors_are_carried_as_they_are(cuda):
     """A tensor parameter is the record's own: also one that requires grad, given under no_grad."""
     p = torch.tensor([3.0e4, 5.0e4], dtype=torch.float64, device="cuda", requires_grad=True)
