@@ -22,12 +22,12 @@ __global__ void k_static_tables(const double* __restrict__ par, int n, const dou
       const size_t b = t / N1;
       const double k = (double)(t % N1), dt = P(0, b), a = P(1, b);
       if (q == 0) {  // time_stepping.py:491-501
-        v = k > 0.0 ? a / (k * (k + 1.0)) : 0.0;
+        v = k > 0.0 ? a / (k * (k + 1.0)) : a * 0.0;
       } else {  // filters.py:95-213
         const double a3 = a * a * a, K = (q & 1) ? P(8, b) : P(9, b);
         const double nc = ((k * k * k) / a3) * (((k + 1.0) * (k + 1.0) * (k + 1.0)) / a3);
         const double off = (q & 1) ? nc - 8.0 / (a3 * a3) : nc;  // eta, delta; Phi has no offset
-        v = q <= 2 ? 1.0 / (1.0 + 2.0 * dt * K * off) : exp(-2.0 * dt * K * fmax(off, 0.0));
+        v = q <= 2 ? 1.0 / (1.0 + 2.0 * dt * K * off) : exp(-2.0 * dt * K * (off < 0.0 ? 0.0 : off));  // a NaN stays
       }
     } else if ((t -= 5 * nt) < nj) {  // time_stepping.py:516-522
       const size_t b = t / J;

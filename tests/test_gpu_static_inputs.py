@@ -48,6 +48,16 @@ def test_given_tensors_are_carried_as_they_are(cuda):
     assert s.taurad.requires_grad and s.taurad is p and s.taudrag.shape == (2,) and torch.equal(s.taudrag[1], q)
 
 
+def test_non_finite_parameters_stay_visible(cuda):
+    nan = float("nan")
+    for kw in (dict(a=nan), dict(K6=nan), dict(dt=nan), dict(a=math.inf)):
+        got = _build(**kw)
+        want = _build(**kw, g=torch.tensor(9.8, dtype=torch.float64, device="cuda", requires_grad=True))
+        for name in ("tstepcoeffmn", "sigma", "sigmaPhi", "sigma_exp", "sigmaPhi_exp", "tstepcoeff", "tstepcoeff2"):
+            x, y = getattr(got, name), getattr(want, name).detach()
+            assert torch.equal(torch.isnan(x), torch.isnan(y)), (kw, name)
+
+
 def test_set_params_refuses_another_length(cuda):
     from my_swampe_gb300.engine import PARAM_NAMES, Engine
 
