@@ -125,7 +125,7 @@ class Engine:
             # tangents of the residual weights (member rows w_curr, w_mid) of a tangent run
             gd["dweights"] = torch.zeros((2, gd["B"]), dtype=torch.float64, device=dev)
             self.groups.append(gd)
-        self._geo_cache: Dict[int, Dict[str, torch.Tensor]] = {}
+        self._geo_cache: Dict[int, Tuple] = {}
         if autotune:
             self.autotune()
         if concurrent:
@@ -214,9 +214,24 @@ class Engine:
 
     # ------------------------------------------------------------- geometry
     def geometry(self, g: int = 0) -> Dict[str, torch.Tensor]:
-        """FP64 mus, w and dense Pmn, Hmn (J, M+1, N+1) built on the GPU."""
+        """FP64 mus, w and dense Pmn, Hmn (J, M+1, N+1) built on the GPU, kept."""
+        return self._geometry(g)[0]
+
+    def grid_constants(self, g: int = 0) -> Dict[str, torch.Tensor]:
+        """The constants of the grid that model.Static carries beside geometry(): Pmnw,
+        Hmnw, lambdas, m and n (n + 1).  Every call's own, views of one copy."""
+        gd = self.groups[g]
+        J, N1 = gd["J"], gd["M"] + 1
+        shapes = dict(Pmnw=(J, N1, N1), Hmnw=(J, N1, N1), lambdas=(gd["I"],), m=(N1,), nn1=(N1,))
+        buf = self._geometry(g)[1].clone()
+        return {k: x.view(s) for (k, s), x in zip(shapes.items(), buf.split([math.prod(s) for s in shapes.values()]))}
+
+    def _geometry(self, g: int):
         if g in self._geo_cache:
-            return self._geo_cache[g]
+            out, packed, ready, stream = self._geo_cache[g]
+            if self.stream != stream:  # formed on another stream: behind it
+                torch.cuda.current_stream(self.device).wait_event(ready)
+            return out, packed
         gd = self.groups[g]
         J, M = gd["J"], gd["M"]
         mus = torch.empty(J, dtype=torch.float64, device=self.device)
@@ -225,12 +240,14 @@ class Engine:
         H = torch.empty_like(P)
         self._check(self.lib.swp_geometry(self._plan, g, mus.data_ptr(), w.data_ptr(), P.data_ptr(), H.data_ptr(), self.stream), "geometry")
         n = torch.arange(M + 1, dtype=torch.float64, device=self.device)
-        # constants of the grid that Static carries (model.build_static)
-        out = dict(mus=mus, w=w, Pmn=P, Hmn=H, Pmnw=w[:, None, None] * P, Hmnw=w[:, None, None] * H,
-                   lambdas=torch.linspace(-math.pi, math.pi, gd["I"] + 1, dtype=torch.float64, device=self.device)[:-1],
-                   m=n, nn1=n * (n + 1))
-        self._geo_cache[g] = out
-        return out
+        lam = torch.linspace(-math.pi, math.pi, gd["I"] + 1, dtype=torch.float64, device=self.device)[:-1]
+        wj = w[:, None, None]
+        packed = torch.cat([x.reshape(-1) for x in (wj * P, wj * H, lam, n, n * (n + 1))])
+        out = dict(mus=mus, w=w, Pmn=P, Hmn=H)
+        ready = torch.cuda.Event()
+        ready.record(torch.cuda.current_stream(self.device))
+        self._geo_cache[g] = (out, packed, ready, self.stream)
+        return out, packed
 
     def static_tables(self, g: int, vals: torch.Tensor, forced: bool) -> Dict[str, torch.Tensor]:
         """Tables of model.Static that depend on the parameters, in one launch.

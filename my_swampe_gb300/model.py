@@ -242,10 +242,11 @@ def build_static(*, M, dt, a, omega, g, Phibar, taurad, taudrag, DPhieq, K6, K6P
     M = int(M)
     N = M
     J, I, _ = _SUPPORTED_M[M]
-    mus, Pmn, Hmn, lambdas = geo["mus"], geo["Pmn"], geo["Hmn"], geo["lambdas"]
-    const = dict(M=M, N=N, I=I, J=J, lambdas=lambdas, mus=mus, w=geo["w"], Pmn=Pmn, Hmn=Hmn, Pmnw=geo["Pmnw"],
-                 Hmnw=geo["Hmnw"], marray=geo["m"][:, None].expand(M + 1, N + 1),
-                 mJarray=geo["m"][None, :].expand(J, M + 1), narray=geo["nn1"][None, :].expand(M + 1, N + 1), test=test)
+    grid = eng.grid_constants(0)  # this record's own
+    mus, lambdas = geo["mus"], grid["lambdas"]
+    const = dict(M=M, N=N, I=I, J=J, lambdas=lambdas, mus=mus, w=geo["w"], Pmn=geo["Pmn"], Hmn=geo["Hmn"],
+                 Pmnw=grid["Pmnw"], Hmnw=grid["Hmnw"], marray=grid["m"][:, None].expand(M + 1, N + 1),
+                 mJarray=grid["m"][None, :].expand(J, M + 1), narray=grid["nn1"][None, :].expand(M + 1, N + 1), test=test)
     given = dict(dt=dt, a=a, omega=omega, g=g, Phibar=Phibar, taurad=taurad, taudrag=taudrag, DPhieq=DPhieq, K6=K6,
                  K6Phi=K6 if K6Phi is None else K6Phi)
     if _plain_values(given.values()):
@@ -275,7 +276,7 @@ def build_static(*, M, dt, a, omega, g, Phibar, taurad, taudrag, DPhieq, K6, K6P
         Bn = max(v.shape[0] for v in vals if v.dim())
         vals = [v.expand(Bn) if v.dim() == 0 else v for v in vals]
     dt_, a_, om_, g_, Pb_, tr_, td_, DP, K6_, K6P = vals
-    n, den = geo["m"], geo["nn1"].clone()
+    n, den = grid["m"], grid["nn1"].clone()
     den[0] = 1.0
     tcmn = a_[..., None, None] / den if a_.dim() else a_ / den
     tcmn = tcmn * (n > 0)

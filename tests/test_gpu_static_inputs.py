@@ -58,6 +58,21 @@ def test_non_finite_parameters_stay_visible(cuda):
             assert torch.equal(torch.isnan(x), torch.isnan(y)), (kw, name)
 
 
+def test_records_share_nothing_that_was_their_own(cuda):
+    names = ("lambdas", "Pmnw", "Hmnw", "marray", "mJarray", "narray")
+    first = _build()
+    want = {k: getattr(first, k).clone() for k in names}
+    Phieq = _build(DPhieq=torch.tensor(1.0e6, dtype=torch.float64, device="cuda", requires_grad=True)).Phieq.detach()
+    for k in names:
+        torch.as_strided(getattr(first, k), (1,), (1,)).fill_(1.0e3)  # through an expanded view too
+    first.lambdas.fill_(0.25)
+    again = _build()
+    for k in names:
+        assert torch.equal(getattr(again, k), want[k]), k
+    after = _build(DPhieq=torch.tensor(1.0e6, dtype=torch.float64, device="cuda", requires_grad=True)).Phieq.detach()
+    assert torch.equal(Phieq, after)
+
+
 def test_set_params_refuses_another_length(cuda):
     from my_swampe_gb300.engine import PARAM_NAMES, Engine
 
@@ -68,3 +83,18 @@ def test_set_params_refuses_another_length(cuda):
             eng.set_params(0, **dict(kw, taurad=bad))
     eng.set_params(0, **dict(kw, taurad=torch.tensor([1.0, 2.0, 3.0])))
     assert eng.groups[0]["params"][4].tolist() == [1.0, 2.0, 3.0]
+
+
+def test_constants_formed_on_another_stream(cuda):
+    from my_swampe_gb300.engine import Engine
+    from my_swampe_gb300.model import build_static
+
+    want = _build()
+    eng, side = Engine([(42, 1)], "fp64"), torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(100_000_000)
+        eng.geometry(0)
+    got = build_static(M=42, test=None, engine=eng, **BASE)
+    for k in ("mus", "Pmn", "lambdas", "Hmnw", "narray"):
+        assert torch.equal(getattr(got, k), getattr(want, k)), k
+    torch.cuda.synchronize()
