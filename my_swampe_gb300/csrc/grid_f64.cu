@@ -104,8 +104,8 @@ struct Mem {
 
 // Slices of the raw rows [f][m][r] (complex).  Rows of fields f < nhalf have the
 // coefficients of m >= 1 halved (adjoint rows: their weight is 1, the matrix'
-// 2).  mid: the value at longitude I/2, sum_m w_m (-1)^m Re Y_m, in integers
-// from every digit, as the tiles' sums.
+// 2).  mid: the value at longitude I/2, sum_m w_m (-1)^m Re Y_m, summed in
+// integers from every digit and rounded once.
 template <class S, int JB>
 __device__ __forceinline__ void slice_fourier(const double2* raw, int nrow, int nhalf, uint32_t* dig, int plane,
                                               int* er, double* mid) {
@@ -142,9 +142,14 @@ __device__ __forceinline__ void slice_fourier(const double2* raw, int nrow, int 
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) alt += __shfl_xor_sync(0xffffffffu, alt, o);
     low = __reduce_add_sync(0xffffffffu, low);
-    // (alt 2^8 + low) 2^(e - 1084), times 2^15 on the scale of e + 1013: rows whose sum could
-    // overflow are NaN, as their tiles' values are
-    if (lane == 0) mid[row] = value(alt >> 9, ((alt & 511) << 23) + (long long)low * (1 << 15), e, 1013);
+    if (lane == 0) {
+      // (alt 2^8 + low) 2^(e - 1084): alt's upper 50 bits and the rest are exact in FP64, one rounding
+      const double hi = (double)(alt >> 12), lo = (double)(((alt & 0xfff) << 8) + low);
+      double v = fma(hi, 1048576.0, lo) * __hiloint2double((e - 61) << 20, 0);
+      if (e == ER_ZERO) v = 0.0;
+      if (e == ER_BAD) v = __longlong_as_double(0x7ff8000000000000ll);
+      mid[row] = v;
+    }
   }
 }
 
