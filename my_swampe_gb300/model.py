@@ -91,7 +91,7 @@ def _engine_for(M: int, B: int, precision: str, device=None, steps: bool = True)
 # weighs more where that comes earlier: one CTA per SM on the finer grids, the
 # SIMT kernel of the other schemes, the FP64 kernels' smaller tiles.  Microseconds
 # per step, one chain and two: fast M = 63, 16 members 34 / 33 (adjoint 39 / 35), 37
-# members 67 / 58; M = 106, 21 members 118 / 97; semi-implicit M = 42, 24 members 30 /
+# members 67 / 58; M = 106, 10 members 71 / 60 (74 / 68), 21 members 118 / 97; semi-implicit M = 42, 24 members 30 /
 # 31, 28 members 40 / 31, 40 members 40 / 34, M = 63, 16 members 44 / 41, 24 members 63
 # / 46, M = 106, 4 members 49 / 43; FP64 M = 42, 9 members 41 / 40 (adjoint 52 / 53),
 # 10 members 52 / 42 (67 / 56), 16 members 63 / 53 (90 / 68), 32 members 110 / 84; M =
@@ -99,6 +99,29 @@ def _engine_for(M: int, B: int, precision: str, device=None, steps: bool = True)
 _SPLIT_MIN_B = 64
 _SPLIT_WEIGHT = {"fast": {42: 1, 63: 4, 106: 7}, "fp64": {42: 7, 63: 10, 106: 16},
                  "fast other schemes": {42: 2.3, 63: 4, 106: 16}}
+
+
+def _halves(M: int, B: int, precision: str, scheme: int) -> Tuple[int, int]:
+    """The halves of a split ensemble: whole Legendre tiles of members in the first
+    (FP64 by truncation, 8 on the tensor-core kernels, one member on the SIMT kernel,
+    whose tiles follow the count), the fewest in all and then the evenest, the larger
+    half first; even halves where they need no more tiles and whole ones would differ
+    by a factor of two.  Microseconds per step (adjoint): FP64 M = 42, 12 members 4 + 8
+    43, 6 + 6 47, 13 members 8 + 5 45 (61), 6 + 7 48 (67), 28 members 16 + 12 75 (106), 12
+    + 16 80 (106); M = 63, 12 members 6 + 6 85 (114), 8 + 4 90 (113); M = 106, 5 members 2
+    + 3 184 (245), 4 + 1 195 (261), 14 members 7 + 7 461 (598), 8 + 6 466 (600); fast M =
+    63, 20 members 8 + 12 38 (41), 10 + 10 42 (42); M = 106, 10 members 5 + 5 60 (68), 8 +
+    2 61 (73), one chain 71 (74), 12 members 6 + 6 63 (73), 8 + 4 64 (75), 25 members 16 +
+    9 118 (133), 12 + 13 115 (136); other schemes M = 63, 28 members 14 + 14 54, 8 + 20 63."""
+    tile = {42: 4, 63: 2, 106: 1}[M] if precision == "fp64" else 8 if scheme == 0 else 1
+    even = B // 2
+    if tile == 1 or B <= tile:
+        return even, B - even
+    tiles = lambda h: -(-h // tile) + -(-(B - h) // tile)  # noqa: E731
+    half = min(range(tile, B, tile), key=lambda h: (tiles(h), abs(B - 2 * h), -h))
+    if max(half, B - half) >= 2 * min(half, B - half) and tiles(even) <= tiles(half):
+        half = even
+    return half, B - half
 
 
 def _split_engine_for(M: int, sizes: Tuple[int, int], precision: str, device=None) -> Engine:
@@ -698,12 +721,7 @@ def _run_split(M, B, precision, device, flags: RunFlagsC, t0: int, T: int, ics: 
     parameters are scalars or per-member tensors, sliced per half.  Returns the
     physical final fields (5, B, J, I), the differentiable final curr fields
     (or None) and the final State, all joined along the member axis."""
-    # whole tiles of the kernels' members in the first half (FP64, M = 42, 12 members: 4 + 8
-    # 43 us per step, 6 + 6 47); equal halves on the SIMT kernel, whose tiles follow the
-    # member count (M = 63, 28 members: 8 + 20 63, 14 + 14 54)
-    tile = 4 if precision == "fp64" else 8 if flags.scheme == 0 else 1
-    half = tile * ((B + tile - 1) // tile // 2) or B // 2
-    sizes = (half, B - half)
+    sizes = _halves(M, B, precision, flags.scheme)
     eng = _split_engine_for(M, sizes, precision, device)
     dev = eng.device
     sls = (slice(0, sizes[0]), slice(sizes[0], B))
