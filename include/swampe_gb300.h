@@ -56,6 +56,7 @@ extern "C" {
 
 #define SWP_FP64 0
 #define SWP_FAST 1
+#define SWP_GEOMETRY 2 /* an FP64 plan without the step kernels' packed matrices */
 
 #define SWP_NFOURIER 19
 #define SWP_NPAR 12
@@ -120,7 +121,9 @@ typedef struct {
 /* Create a plan for `ngroups` truncations (M[g] in {42, 63, 106}) with B[g]
  * members each; builds Gauss nodes, Legendre bases and FFT twiddles on the
  * device in FP64.  Replaces build_static/_cached_geometry (model.py:62-86,
- * 457-557) and spectral_transform.PmnHmn / gauss_legendre. */
+ * 457-557) and spectral_transform.PmnHmn / gauss_legendre.  SWP_GEOMETRY: for
+ * swp_geometry, swp_static_tables and swp_diagnose_winds (arrays as SWP_FP64);
+ * calls that step, start or output a state fail with SWP_ERR_CUDA. */
 int swp_plan_create(int ngroups, const int* M, const int* B, int precision, swp_plan** out);
 int swp_plan_destroy(swp_plan* plan);
 /* Grid sizes of group g (initial_conditions.spectral_params, initial_conditions.py:50-85). */

@@ -16,6 +16,7 @@ LIB_PATH = _PKG / "libswampe_gb300.so"
 SWP_OK = 0
 SWP_FP64 = 0
 SWP_FAST = 1
+SWP_GEOMETRY = 2
 NFOURIER = 19
 NPAR = 12
 NMEMBER = 4

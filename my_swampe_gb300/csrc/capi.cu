@@ -34,7 +34,8 @@ struct swp_plan {
   float* tcbasis[MAXG] = {};
   float* tcbasis_adj[MAXG] = {};
   // FP64 step kernels on integer slices: packed Legendre basis of the step and of
-  // its transpose (spectral_f64.cu), longitude transforms (grid_f64.cu)
+  // its transpose (spectral_f64.cu), longitude transforms (grid_f64.cu).  Groups of
+  // one truncation share them; a geometry plan has none.
   SliceBasis slices = {}, slices_adj = {}, slices_grid = {};
   void* coefmem[MAXG] = {};              // per-call coefficient tables (CoefTables) of each group
   int* d_err = nullptr;                  // device error word set by bounded waits that ran out
@@ -292,6 +293,8 @@ cudaError_t launch_step_spec(const swp_plan* p, const SpecLaunch<T>& LS, int nbs
       if (e == cudaSuccess && nb > 0) e = launch_spec<T>(LR, nb, p->spec_smem, s);
       return e;
     }
+  } else if (!p->slices.p[0]) {
+    return cudaErrorNotSupported;
   } else if (LS.mode == 0 && !LS.cfg.tl_filter) {
     return launch_spec_f64(LS, p->slices, false, s);
   }
@@ -314,6 +317,7 @@ cudaError_t launch_step_spec_adj(const swp_plan* p, const SpecLaunch<T>& LS, int
     }
     return launch_spec_adj<T>(LS, nbs, p->spec_adj_smem, s);
   } else {
+    if (!p->slices_adj.p[0]) return cudaErrorNotSupported;
     return launch_spec_f64(LS, p->slices_adj, true, s);
   }
 }
@@ -324,6 +328,7 @@ cudaError_t launch_step_spec_adj(const swp_plan* p, const SpecLaunch<T>& LS, int
 template <typename T>
 cudaError_t launch_any_grid(const swp_plan* p, const GridLaunch<T>& LG, int nbg, cudaStream_t s) {
   if constexpr (std::is_same<T, double>::value) {
+    if (!p->slices_grid.p[0]) return cudaErrorNotSupported;
     if (LG.mode == GM_STEP || LG.mode == GM_ADJ_STEP || LG.mode == GM_OUTPUT)
       return launch_grid_f64(LG, p->slices_grid, s);
     cudaError_t e = launch_grid<T>(LG, nbg, p->grid_smem[LG.mode], s);
@@ -1115,7 +1120,9 @@ int swp_plan_create(int ngroups, const int* M, const int* B, int precision, swp_
   if (!out) return SWP_ERR_ARG;
   *out = nullptr;
   if (ngroups < 1 || ngroups > MAXG || !M || !B) return SWP_ERR_ARG;
-  if (precision != SWP_FP64 && precision != SWP_FAST) return SWP_ERR_ARG;
+  if (precision != SWP_FP64 && precision != SWP_FAST && precision != SWP_GEOMETRY) return SWP_ERR_ARG;
+  const bool steps = precision != SWP_GEOMETRY;
+  if (!steps) precision = SWP_FP64;
   swp_plan* p = new (std::nothrow) swp_plan();
   if (!p) return SWP_ERR_ARG;
   p->precision = precision;
@@ -1202,8 +1209,16 @@ int swp_plan_create(int ngroups, const int* M, const int* B, int precision, swp_
     }
     p->use_tc = true;
   }
-  if (precision == SWP_FP64) {
+  if (precision == SWP_FP64 && steps) {
     for (int g = 0; g < ngroups; ++g) {
+      int h = 0;
+      while (M[h] != M[g]) ++h;
+      if (h < g) {  // the truncation's first group has them
+        p->slices.p[g] = p->slices.p[h];
+        p->slices_adj.p[g] = p->slices_adj.p[h];
+        p->slices_grid.p[g] = p->slices_grid.p[h];
+        continue;
+      }
       void *fwd = nullptr, *adj = nullptr, *grid = nullptr;
       cudaError_t e = cudaMalloc(&fwd, spec_f64_basis_bytes(M[g]));
       p->slices.p[g] = fwd;
@@ -1241,9 +1256,11 @@ int swp_plan_destroy(swp_plan* p) {
     if (p->geom[g].mem) cudaFree(p->geom[g].mem);
     if (p->tcbasis[g]) cudaFree(p->tcbasis[g]);
     if (p->tcbasis_adj[g]) cudaFree(p->tcbasis_adj[g]);
-    if (p->slices.p[g]) cudaFree(const_cast<void*>(p->slices.p[g]));
-    if (p->slices_adj.p[g]) cudaFree(const_cast<void*>(p->slices_adj.p[g]));
-    if (p->slices_grid.p[g]) cudaFree(const_cast<void*>(p->slices_grid.p[g]));
+    int h = 0;
+    while (p->M[h] != p->M[g]) ++h;
+    if (h == g)  // shared by the groups of a truncation
+      for (const SliceBasis* b : {&p->slices, &p->slices_adj, &p->slices_grid})
+        if (b->p[g]) cudaFree(const_cast<void*>(b->p[g]));
     if (p->coefmem[g]) cudaFree(p->coefmem[g]);
   }
   if (p->d_err) cudaFree(p->d_err);

@@ -83,9 +83,13 @@ class Engine:
     """One plan + device state for a list of ``(M, B)`` groups."""
 
     def __init__(self, groups: Sequence[Tuple[int, int]], precision: str = "fp64", device=None,
-                 autotune: bool = False, concurrent: bool = False):
+                 autotune: bool = False, concurrent: bool = False, steps: bool = True):
+        """steps=False (FP64): for geometry, static tables and winds only, without the
+        matrices that the step kernels keep packed (140 MB at M = 106)."""
         if precision not in PRECISIONS:
             raise ValueError(f"precision must be one of {sorted(PRECISIONS)}, got {precision!r}")
+        if not steps and precision != "fp64":
+            raise ValueError("an engine without steps is FP64")
         for M, _ in groups:
             if int(M) not in (42, 63, 106):
                 raise ValueError(f"Unsupported value of M={M}. Only 42, 63, and 106 are supported.")
@@ -101,7 +105,8 @@ class Engine:
         Bs = (ctypes.c_int * ng)(*[int(b) for _, b in groups])
         self._plan = ctypes.c_void_p()
         with torch.cuda.device(self.device):
-            rc = self.lib.swp_plan_create(ng, Ms, Bs, PRECISIONS[precision], ctypes.byref(self._plan))
+            rc = self.lib.swp_plan_create(ng, Ms, Bs, PRECISIONS[precision] if steps else _lib.SWP_GEOMETRY,
+                                          ctypes.byref(self._plan))
         if rc != _lib.SWP_OK:
             msg = self.lib.swp_last_error(self._plan).decode() if self._plan.value else ""
             if self._plan.value:

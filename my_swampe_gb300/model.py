@@ -49,7 +49,7 @@ _GEO_ENGINES: Dict[int, Engine] = {}
 
 def _geometry_engine(M: int) -> Engine:
     if M not in _GEO_ENGINES:
-        _GEO_ENGINES[M] = Engine([(M, 1)], "fp64")
+        _GEO_ENGINES[M] = Engine([(M, 1)], "fp64", steps=False)
     return _GEO_ENGINES[M]
 
 
