@@ -39,8 +39,8 @@ constexpr int NL = 8;                       // levels kept
 constexpr uint64_t BIAS = 0x8080808080808080ull;  // 128 in each digit
 constexpr float ACC0 = 12582912.0f;         // 1.5 * 2^23
 constexpr int ACC0_BITS = 0x4B400000;
-constexpr int ER_BAD = 4000;                // row exponent of a row with an infinity or a NaN
 constexpr int ER_ZERO = -8000;              // row exponent of a zero row
+constexpr int ER_BAD = 20000;               // of a row with an infinity or a NaN: NaN times a zero row too
 constexpr int KFLUSH = 2;                   // mma k-steps (of 16) per flush of the accumulators
 
 __device__ __forceinline__ int expo(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
