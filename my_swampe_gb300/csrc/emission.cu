@@ -277,6 +277,7 @@ struct ProjectSmem {
       double part[2][PR_COEF][PR_MEMB + 1];
       float mag[2][PR_COEF][PR_MEMB + 1];  // sums of the top digits' magnitudes
       int ec[2][PR_COEF];                  // coefficient scales
+      int2 ms[PR_COEF][PR_MEMB + 1];       // both halves' magnitudes (FP32 bits) and their scale
     };
   };
   uint32_t dig[slices::ND][PR_MEMB][PR_ROW];
@@ -432,28 +433,33 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS, 2)
     S.ec[half][mt * 16 + g] = ea[0];
     S.ec[half][mt * 16 + g + 8] = ea[1];
   }
+  __syncthreads();
+  // the halves together: sums, and the magnitudes on the larger of their scales
+  for (int i = threadIdx.x; i < PR_COEF * PR_MEMB; i += EM_THREADS) {
+    const int c = i / PR_MEMB, r = i % PR_MEMB, e0 = S.ec[0][c], e1 = S.ec[1][c], e = max(e0, e1);
+    S.part[0][c][r] += S.part[1][c][r];
+    S.ms[c][r] = make_int2(
+        __float_as_int(S.mag[0][c][r] * pow2_down(e - e0) + S.mag[1][c][r] * pow2_down(e - e1)), S.er[0][r] + e);
+  }
   cl.sync();
-  // every eighth coefficient per rank: the sum over ranks and halves, in order
+  // every eighth coefficient per rank: the sum over ranks, in order
   static_assert(PR_COEF * PR_MEMB / EM_CL <= EM_THREADS, "an output per thread");
   bool again = false;
-  int c = 0, r = 0;
+  const int c = rank + EM_CL * (threadIdx.x / PR_MEMB), r = threadIdx.x % PR_MEMB;
   if (threadIdx.x < PR_COEF * PR_MEMB / EM_CL) {
-    c = rank + EM_CL * (threadIdx.x % (PR_COEF / EM_CL));
-    r = threadIdx.x / (PR_COEF / EM_CL);
     double s = 0.0;
-    float m = 0.0f, mq[EM_CL];
-    int top = 0, sq[EM_CL];
+    int2 ms[EM_CL];
+    int top = 0;
+    float m = 0.0f;
 #pragma unroll
     for (int q = 0; q < EM_CL; ++q) {
       const Smem* p = cl.map_shared_rank(&S, q);
-      s += p->part[0][c][r] + p->part[1][c][r];
-      const int e0 = p->ec[0][c], e1 = p->ec[1][c], e = max(e0, e1);
-      sq[q] = p->er[0][r] + e;
-      mq[q] = p->mag[0][c][r] * pow2_down(e - e0) + p->mag[1][c][r] * pow2_down(e - e1);
-      top = max(top, sq[q]);
+      s += p->part[0][c][r];
+      ms[q] = p->ms[c][r];
+      top = max(top, ms[q].y);
     }
 #pragma unroll
-    for (int q = 0; q < EM_CL; ++q) m += mq[q] * pow2_down(top - sq[q]);
+    for (int q = 0; q < EM_CL; ++q) m += __int_as_float(ms[q].x) * pow2_down(top - ms[q].y);
     const bool out = c0 + c < ncoef && r < nm;
     // scales within 2^1200 and 2^3000: no partial sum was cut off at either end (value())
     again = out && !(m >= PR_GUARD && top >= 1200 && top <= 3000);
