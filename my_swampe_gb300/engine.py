@@ -56,17 +56,14 @@ class RunFlagsC:
         )
 
 
-def stack_values(vals: Sequence, device, n: Optional[int] = None) -> torch.Tensor:
+def stack_values(vals: Sequence, device, n: int) -> torch.Tensor:
     """Values (floats, 0-d or length-n tensors or sequences) as one float64
-    (len(vals), n) tensor, detached; by default n is their common length, 1 if all
-    are scalars.  The floats cross to the device in one copy."""
+    (len(vals), n) tensor, detached.  The floats cross to the device in one copy."""
     is_float = [isinstance(v, (int, float)) for v in vals]
     floats = iter(torch.tensor([float(v) for v, f in zip(vals, is_float) if f], dtype=torch.float64,
                                device=device).unbind(0)) if any(is_float) else iter(())
     ts = [next(floats) if f else torch.as_tensor(v, dtype=torch.float64, device=device).detach()
           for v, f in zip(vals, is_float)]
-    if n is None:
-        n = max([t.numel() for t in ts if t.dim()], default=1)
     return torch.stack([t.expand(n) if t.dim() == 0 else t.reshape(n) for t in ts])
 
 
@@ -151,7 +148,9 @@ class Engine:
 
     @property
     def stream(self) -> int:
-        return torch.cuda.current_stream(self.device).cuda_stream
+        """Handle of torch's current stream (read without forming a Stream: 10 us of host time a call)."""
+        dev = self.device.index
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if dev is None else dev)
 
     def _states(self, fourier=None, hist=None, diag=None) -> ctypes.Array:
         arr = (_lib.GroupState * len(self.groups))()
@@ -222,14 +221,14 @@ class Engine:
         """FP64 mus, w and dense Pmn, Hmn (J, M+1, N+1) built on the GPU, kept."""
         return self._geometry(g)[0]
 
-    def grid_constants(self, g: int = 0) -> Dict[str, torch.Tensor]:
-        """The constants of the grid that model.Static carries beside geometry(): Pmnw,
-        Hmnw, lambdas, m and n (n + 1).  Every call's own, views of one copy."""
+    def grid(self, g: int = 0):
+        """geometry(), and the constants of the grid that model.Static carries beside it
+        (Pmnw, Hmnw, lambdas, m, n (n + 1)): the latter every call's own, views of one copy."""
         gd = self.groups[g]
         J, N1 = gd["J"], gd["M"] + 1
-        shapes = dict(Pmnw=(J, N1, N1), Hmnw=(J, N1, N1), lambdas=(gd["I"],), m=(N1,), nn1=(N1,))
-        buf = self._geometry(g)[1].clone()
-        return {k: x.view(s) for (k, s), x in zip(shapes.items(), buf.split([math.prod(s) for s in shapes.values()]))}
+        geo, packed = self._geometry(g)
+        Pw, Hw, lam, m, nn1 = packed.clone().split_with_sizes((J * N1 * N1, J * N1 * N1, gd["I"], N1, N1))
+        return geo, dict(Pmnw=Pw.view(J, N1, N1), Hmnw=Hw.view(J, N1, N1), lambdas=lam, m=m, nn1=nn1)
 
     def _geometry(self, g: int):
         if g in self._geo_cache:

@@ -18,6 +18,7 @@ import math
 import warnings
 from collections import OrderedDict
 from dataclasses import dataclass, replace as _dc_replace
+from functools import lru_cache
 from typing import Any, Dict, NamedTuple, Optional, Tuple
 
 import numpy as np
@@ -101,6 +102,7 @@ _SPLIT_WEIGHT = {"fast": {42: 1, 63: 4, 106: 7}, "fp64": {42: 7, 63: 10, 106: 16
                  "fast other schemes": {42: 2.3, 63: 4, 106: 16}}
 
 
+@lru_cache(maxsize=256)
 def _halves(M: int, B: int, precision: str, scheme: int) -> Tuple[int, int]:
     """The halves of a split ensemble: whole Legendre tiles of members in the first
     (FP64 by truncation, 8 on the tensor-core kernels, one member on the SIMT kernel,
@@ -240,42 +242,45 @@ def _scalar_tensor(x, dev):
     return torch.as_tensor(x, dtype=torch.float64, device=dev)
 
 
-def _plain_values(vals) -> bool:
-    """Whether parameters are what the table kernel takes: values without a
-    derivative or a function transform's wrapper (torch.func.vmap), scalars and
-    vectors of one length."""
-    lengths = set()
+def _plain_length(vals) -> Optional[int]:
+    """The common length of parameters that the table kernel takes (0 if all are
+    scalars): values without a derivative or a function transform's wrapper
+    (torch.func.vmap), scalars and vectors of one length; else None."""
+    n = 0
     for x in vals:
         if _is_python_scalar(x):
             continue
-        if torch.is_tensor(x) and torch._C._functorch.is_functorch_wrapped_tensor(x) or _tracked(x):
-            return False
-        shape = torch.as_tensor(x).shape
-        if len(shape) > 1:
-            return False
-        lengths.update(shape)
-    return len(lengths) < 2 and 0 not in lengths
+        if not torch.is_tensor(x):
+            x = torch.as_tensor(x)
+        elif torch._C._functorch.is_functorch_wrapped_tensor(x) or _tracked(x):
+            return None
+        if x.dim() == 0:
+            continue
+        if x.dim() > 1 or x.numel() == 0 or n not in (0, x.numel()):
+            return None
+        n = x.numel()
+    return n
 
 
 def build_static(*, M, dt, a, omega, g, Phibar, taurad, taudrag, DPhieq, K6, K6Phi, test, engine: Optional[Engine] = None) -> Static:
     """``model.py:457-557`` on the GPU (FP64).  Scalars may be per-member vectors."""
     eng = engine if engine is not None else _geometry_engine(int(M))
-    geo = eng.geometry(0)
+    geo, grid = eng.grid(0)  # kept with the engine, and this record's own
     dev = eng.device
     M = int(M)
     N = M
     J, I, _ = _SUPPORTED_M[M]
-    grid = eng.grid_constants(0)  # this record's own
     mus, lambdas = geo["mus"], grid["lambdas"]
     const = dict(M=M, N=N, I=I, J=J, lambdas=lambdas, mus=mus, w=geo["w"], Pmn=geo["Pmn"], Hmn=geo["Hmn"],
                  Pmnw=grid["Pmnw"], Hmnw=grid["Hmnw"], marray=grid["m"][:, None].expand(M + 1, N + 1),
                  mJarray=grid["m"][None, :].expand(J, M + 1), narray=grid["nn1"][None, :].expand(M + 1, N + 1), test=test)
     given = dict(dt=dt, a=a, omega=omega, g=g, Phibar=Phibar, taurad=taurad, taudrag=taudrag, DPhieq=DPhieq, K6=K6,
                  K6Phi=K6 if K6Phi is None else K6Phi)
-    if _plain_values(given.values()):
-        v = stack_values(list(given.values()), dev)
+    n = _plain_length(given.values())
+    if n is not None:
+        v = stack_values(list(given.values()), dev, max(n, 1))
         t = eng.static_tables(0, v, test is None)
-        one = not any(torch.as_tensor(x).dim() for x in given.values())
+        one = n == 0
         if one:  # scalars: no member axis
             t = {k: x[0] for k, x in t.items()}
 
@@ -283,7 +288,7 @@ def build_static(*, M, dt, a, omega, g, Phibar, taurad, taudrag, DPhieq, K6, K6P
             if not torch.is_tensor(x):
                 return r[0] if one else r
             x = _scalar_tensor(x, dev)
-            return x if one or x.dim() else x.expand(v.shape[1])
+            return x if one or x.dim() else x.expand(n)
 
         row = lambda x: x[..., None, :].expand(*x.shape[:-1], M + 1, N + 1)  # noqa: E731
         return Static(**const, **{k: carried(x, r) for (k, x), r in zip(given.items(), v)}, fmn=t["fmn"],
