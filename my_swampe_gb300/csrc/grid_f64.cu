@@ -576,10 +576,14 @@ __global__ void __launch_bounds__(256, 2) k_grid_out_f64(const __grid_constant__
 
 // Rows per CTA: at most as many as leave two CTAs per SM their shared memory.  Few
 // rows for few members: two from 1.5 CTAs of one row per SM on (the two then share
-// the SM's FP64 pipe), four from 1.5 rounds of two.  Step, M = 42, us with 1 / 2 /
-// 4 rows (before the conversions moved to integers): 2 members 17 / 19 / 29, 4
-// members 21 / 19 / 29, 8 members 33 / 27 / 29, 12 members 45 / 39 / 41, 16 members
-// 55 / 45 / 41.
+// the SM's FP64 pipe), four from 1.5 rounds of two.  Step (adjoint, at most two), M =
+// 42, us with 1 / 2 / 4 rows: 1 member 15 / 17 / 25 (18 / 23), 4 members 18 / 18 / 25
+// (23 / 23), 6 members 25 / 25 / 25 (35 / 31), 8 members 29 / 24 / 25 (41 / 32), 12
+// members 39 / 35 / 37 (55 / 47), 14 members 39 / 35 / 37 (57 / 47), 16 members 47 / 41 /
+// 37 (68 / 53), 20 members 57 / 51 / 54 (84 / 70), 24 members 66 / 55 / 54 (97 / 76), 48
+// members 120 / 97 / 89 (181 / 137), 256 members 596 / 438 / 379 (934 / 648); M = 63 with
+// 1 / 2: 2 members 23 / 23 (33 / 32), 5 members 39 / 35 (55 / 47), 32 members 181 / 150
+// (267 / 209).
 enum Kind { STEP, ADJ, OUT };
 template <int M_, Kind K>
 constexpr int max_rows() { return K == OUT ? 1 : K == ADJ ? (M_ == 106 ? 1 : 2) : M_ == 42 ? 4 : M_ == 63 ? 2 : 1; }

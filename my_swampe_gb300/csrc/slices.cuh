@@ -25,8 +25,14 @@
 // The result's error is that of the inputs on the row's scale and one final
 // rounding; a chain of FP64 FMAs rounds K times.  (With 7 digits, 2^-54 of the
 // maximum, rows that fall by orders of magnitude lost bits: meridional winds were
-// up to 9 times further off the oracle than with FMAs.)  A row that holds an infinity or
-// a NaN gives NaN.
+// up to 9 times further off the oracle than with FMAs.)  So the error is a part, K
+// 2^-59 at most, of the product of the two rows' maxima, as an FFT's is of its row's,
+// and not of each sum's own terms: rows that meet only where both are faint need more.
+// The Legendre bases are levelled over the latitudes for that (spectral_f64.cu), the
+// emission projection takes such sums again with FMAs (emission.cu).
+// A row that holds an infinity or a NaN gives NaN, against a zero row too.  A row
+// below 2^-959 counts as zero; rows whose maxima's product is below 2^-1006 give zero,
+// beyond 2^1006 NaN.
 #pragma once
 #include <cuda_fp16.h>
 #include <stdint.h>

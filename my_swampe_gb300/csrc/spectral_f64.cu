@@ -721,11 +721,13 @@ __global__ void __launch_bounds__(256, 2) k_spectral_adj_f64(const __grid_consta
 
 // Members per unit.  One round of CTAs (two per SM) at one member each, then two;
 // four (M = 42 only: the unit's shared memory has to fit twice in an SM) once
-// those are most of a round themselves.  Step, M = 42, us with 1 / 2 / 4 members:
-// 6 members 23 / 24 / 36, 8 members 36 / 30 / 37, 16 members 51 / 42 / 46, 24
-// members 67 / 50 / 47 (before the conversion of the sums moved to integers; since
-// then 8 members 25, 16 members 34, 256 members 297, their transpose 294; the FMA
-// kernels 880 / 840 us there and 98 / 80 us for one member, now 17 / 18).
+// those are most of a round themselves.  Step (transpose), M = 42, us with 1 / 2 / 4
+// members: 7 members 21 / 25 / 32 (21 / 27 / 32), 8 members 28 / 25 / 32 (31 / 27 /
+// 32), 16 members 43 / 34 / 40 (47 / 41 / 42), 20 members 45 / 40 / 40 (49 / 44 / 43),
+// 24 members 53 / 42 / 40 (61 / 46 / 43), 32 members 67 / 54 / 55 (76 / 63 / 56), 256
+// members 459 / 317 / 296 (544 / 381 / 292); M = 63 with 1 / 2: 4 members 28 / 29 (28 /
+// 27), 5 members 44 / 35 (41 / 35), 32 members 153 / 119 (158 / 115).  The FMA kernels
+// took 880 / 840 us for 256 members and 98 / 80 us for one, now 17 / 18.
 template <int M_>
 int tile_for(const SpecLaunch<double>& L) {
   auto units = [&](int mt) {
