@@ -105,12 +105,15 @@ struct Mem {
 // Slices of the raw rows [f][m][r] (complex).  Rows of fields f < nhalf have the
 // coefficients of m >= 1 halved (adjoint rows: their weight is 1, the matrix'
 // 2).  mid: the value at longitude I/2, sum_m w_m (-1)^m Re Y_m, summed in
-// integers from every digit and rounded once.
+// integers from every digit and rounded once; a lane converts a row of the warp's, so
+// that the FP64 instructions serve them all.
 template <class S, int JB>
 __device__ __forceinline__ void slice_fourier(const double2* raw, int nrow, int nhalf, uint32_t* dig, int plane,
                                               int* er, double* mid) {
   constexpr int KI = (S::KP + 31) / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  long long row_alt = 0;  // of row warp + 8 lane
+  int row_low = 0, row_e = ER_ZERO;
   for (int row = warp; row < nrow; row += 8) {
     const int f = row / JB, r = row % JB, half = f < nhalf ? 1 : 0;
     double2 y[KI];
@@ -125,31 +128,41 @@ __device__ __forceinline__ void slice_fourier(const double2* raw, int nrow, int 
     }
     e = row_exponent((int)__reduce_max_sync(0xffffffffu, (unsigned)e));
     if (lane == 0) er[row] = e;
-    long long alt = 0;  // in units of 2^8 of the scale
+    long long alt = 0;  // in units of 2^8 of the scale (a lane's m are of one parity)
     int low = 0;        // and of its unit
 #pragma unroll
     for (int i = 0; i < KI; ++i) {
       const int m = lane + 32 * i, h = m ? half : 0;
       uint64_t a = fixed(y[i].x, e + h), b = fixed(y[i].y, e + h);
       const long long q = (long long)(a - BIAS);
-      const int w = m ? ((m & 1) ? -2 : 2) : 1;
-      alt += w * (q >> 8);
-      low += w * (int)(q & 0xff);
+      const long long qh = q >> 8;
+      const int ql = (int)q & 0xff;
+      alt += m ? 2 * qh : qh;
+      low += m ? 2 * ql : ql;
       pair_exchange(a, b);
       if (S::KP % 32 == 0 || m < S::KP)
         store_digits(dig + (size_t)row * S::YW + (lane & 1) * (S::KP / 2) + (lane >> 1) + 16 * i, plane, a, b);
     }
+    if (lane & 1) {
+      alt = -alt;
+      low = -low;
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) alt += __shfl_xor_sync(0xffffffffu, alt, o);
     low = __reduce_add_sync(0xffffffffu, low);
-    if (lane == 0) {
-      // (alt 2^8 + low) 2^(e - 1084): alt's upper 50 bits and the rest are exact in FP64, one rounding
-      const double hi = (double)(alt >> 12), lo = (double)(((alt & 0xfff) << 8) + low);
-      double v = fma(hi, 1048576.0, lo) * __hiloint2double((e - 61) << 20, 0);
-      if (e == ER_ZERO) v = 0.0;
-      if (e == ER_BAD) v = __longlong_as_double(0x7ff8000000000000ll);
-      mid[row] = v;
+    if (lane == row >> 3) {
+      row_alt = alt;
+      row_low = low;
+      row_e = e;
     }
+  }
+  if (warp + 8 * lane < nrow) {
+    // (alt 2^8 + low) 2^(e - 1084): alt's upper 50 bits and the rest are exact in FP64, one rounding
+    const double hi = (double)(row_alt >> 12), lo = (double)(int)(((int)(row_alt & 0xfff) << 8) + row_low);
+    double v = fma(hi, 1048576.0, lo) * __hiloint2double((row_e - 61) << 20, 0);
+    if (row_e == ER_ZERO) v = 0.0;
+    if (row_e == ER_BAD) v = __longlong_as_double(0x7ff8000000000000ll);
+    mid[warp + 8 * lane] = v;
   }
 }
 
