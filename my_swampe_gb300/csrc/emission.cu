@@ -109,9 +109,10 @@ __device__ __forceinline__ double temperature(const EmCfg& c, double phi, double
 // 1989): x = n ln2 / 64 + r, 2^(n/64) = 2^e (1 + tm1[j]),
 //   expm1(x) = 2^e (1 + tm1) p + (2^e tm1 + (2^e - 1)),  p = expm1(r), |r| <= ln2 / 128,
 // with p's Taylor polynomial to r^6, whose next term is below 2^-57 p (for x below
-// ln2 / 128, n = 0, p is the result itself).  13 FP64 instructions, where the
-// library call took about 40 of the map's 100 a pixel.
-__device__ __forceinline__ double planck_rel(double x, const double* __restrict__ tm1) {
+// ln2 / 128, n = 0, p is the result itself).  The table holds tm1 and 1 + tm1, whose
+// exponent is raised in integers.  12 FP64 instructions, where the library call took
+// about 40 of the map's 100 a pixel.
+__device__ __forceinline__ double planck_rel(double x, const double2* __restrict__ tab) {
   const double magic = 6755399441055744.0;  // 1.5 * 2^52: rounds to an integer in the low word
   const double t = fma(x, 92.332482616893656877, magic);  // 64 / ln 2
   const int n = __double2loint(t);
@@ -123,20 +124,21 @@ __device__ __forceinline__ double planck_rel(double x, const double* __restrict_
   double p = fma(fma(r, 1.0 / 720.0, 1.0 / 120.0), r2, fma(r, 1.0 / 24.0, 1.0 / 6.0));
   p = fma(fma(p, r, 0.5), r2, r);
   const double e2 = __hiloint2double((1023 + (n >> 6)) << 20, 0);
-  const double t1 = tm1[n & (EXP_N - 1)];
-  const double q = fma(e2, t1, e2 - 1.0);
-  return 1.0 / (fma(q + 1.0, p, q) + 1.0e-30);
+  const double2 t1 = tab[n & (EXP_N - 1)];
+  const double q = fma(e2, t1.x, e2 - 1.0);
+  const double s = __hiloint2double(__double2hiint(t1.y) + ((n >> 6) << 20), __double2loint(t1.y));
+  return 1.0 / (fma(s, p, q) + 1.0e-30);
 }
 // v: Phi, or T (c.input 1).  ANY_X: x_clip is outside planck_rel's range
 template <bool ANY_X>
 __device__ __forceinline__ double planck_bands(const EmCfg& c, double v, double Phibar,
-                                               const double* __restrict__ tm1) {
+                                               const double2* __restrict__ tab) {
   const double p0 = c.input == 0 && c.temp_mode == 0 ? Phibar : c.p0;
   const double u = c.input != 0 ? v : c.folded ? fmax(p0 + v, c.pmin) : temperature(c, v, Phibar);
   double out = 0.0;
   for (int k = 0; k < c.nbands; ++k) {
     const double x = fmin(fmax(c.pl[k] / u, 0.0), c.x_clip);
-    out += c.bw[k] * (ANY_X ? 1.0 / (expm1(x) + 1.0e-30) : planck_rel(x, tm1));
+    out += c.bw[k] * (ANY_X ? 1.0 / (expm1(x) + 1.0e-30) : planck_rel(x, tab));
   }
   return out;
 }
@@ -157,7 +159,7 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS)
                    const double* __restrict__ w_lat, const __grid_constant__ EmCfg c, int stage,
                    double* __restrict__ out, int* __restrict__ ok) {
   __shared__ double slots[2][3 * EM_WARPS];
-  __shared__ double tm1[EXP_N];
+  __shared__ double2 tab[EXP_N];
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank(), b = blockIdx.x / EM_CL;
   const int lane = threadIdx.x & 31;
@@ -168,7 +170,7 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS)
   double* y = out + (size_t)b * npix;
   const double pb = Phibar ? Phibar[b] : 0.0;
   const double qnan = __longlong_as_double(0x7ff8000000000000ll);
-  if (threadIdx.x < EXP_N) tm1[threadIdx.x] = c.tm1[threadIdx.x];
+  if (threadIdx.x < EXP_N) tab[threadIdx.x] = make_double2(c.tm1[threadIdx.x], 1.0 + c.tm1[threadIdx.x]);
   // pass 1: all of the input finite (Phi -> T guard) and, with the Planck
   // model, all of T finite
   bool nan_map = false;
@@ -183,7 +185,7 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS)
       }
     nan_map = !cluster_sum(0.0, 0.0, fin, slots[0]).all;
   } else {
-    cl.sync();  // tm1, and every rank running before the remote reads below
+    cl.sync();  // the table, and every rank running before the remote reads below
   }
   // pass 2: T, or the intensity and, for stage 2, its weighted mean over the
   // finite pixels (pipeline.py:821-837)
@@ -198,7 +200,7 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS)
         v = qnan;
       } else if (c.input < 2) {
         if (stage > 0 && c.model == 1) {
-          v = planck_bands<ANY_X>(c, v, pb, tm1);
+          v = planck_bands<ANY_X>(c, v, pb, tab);
         } else {
           if (c.input == 0) v = temperature(c, v, pb);
           if (stage > 0) {
