@@ -280,6 +280,7 @@ struct ProjectSmem {
       float mag[2][PR_COEF][PR_MEMB + 1];  // sums of the top digits' magnitudes
       int ec[2][PR_COEF];                  // coefficient scales
       int2 ms[PR_COEF][PR_MEMB + 1];       // both halves' magnitudes (FP32 bits) and their scale
+      int again[PR_COEF * PR_MEMB / EM_CL], nagain;  // outputs below the guard (static memory for them: 2 us more)
     };
   };
   uint32_t dig[slices::ND][PR_MEMB][PR_ROW];
@@ -468,13 +469,12 @@ __global__ void __cluster_dims__(EM_CL, 1, 1) __launch_bounds__(EM_THREADS, 2)
     if (out && !again) yraw[(size_t)(b0 + r) * ncoef + c0 + c] = s;
   }
   // the outputs below the guard, spread over the CTA's warps
-  __shared__ int s_again[PR_COEF * PR_MEMB / EM_CL], s_nagain;
-  if (threadIdx.x == 0) s_nagain = 0;
+  if (threadIdx.x == 0) S.nagain = 0;
   __syncthreads();
-  if (again) s_again[atomicAdd(&s_nagain, 1)] = (c0 + c) * PR_MEMB + r;
+  if (again) S.again[atomicAdd(&S.nagain, 1)] = (c0 + c) * PR_MEMB + r;
   __syncthreads();
-  for (int i = warp; i < s_nagain; i += EM_WARPS) {
-    const int cc = s_again[i] / PR_MEMB, bb = b0 + s_again[i] % PR_MEMB;
+  for (int i = warp; i < S.nagain; i += EM_WARPS) {
+    const int cc = S.again[i] / PR_MEMB, bb = b0 + S.again[i] % PR_MEMB;
     const double *x = rhs + (size_t)bb * npix, *w = P + (size_t)cc * npix;
     double s = 0.0;
 #pragma unroll 8
