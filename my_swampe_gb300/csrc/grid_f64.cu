@@ -147,9 +147,12 @@ __device__ __forceinline__ void slice_fourier(const double2* raw, int nrow, int 
       alt = -alt;
       low = -low;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) alt += __shfl_xor_sync(0xffffffffu, alt, o);
+    // the warp's sums, 24 bits of alt at a time: four independent reductions
+    const int a0 = __reduce_add_sync(0xffffffffu, (int)(alt & 0xffffff));
+    const int a1 = __reduce_add_sync(0xffffffffu, (int)((alt >> 24) & 0xffffff));
+    const int a2 = __reduce_add_sync(0xffffffffu, (int)(alt >> 48));
     low = __reduce_add_sync(0xffffffffu, low);
+    alt = (long long)a0 + ((long long)a1 << 24) + (long long)a2 * (1ll << 48);
     if (lane == row >> 3) {
       row_alt = alt;
       row_low = low;
