@@ -664,8 +664,8 @@ extern "C" int swp_emission_project(const double* rhs, const int* ok, int B, int
   };
   // 32 coefficients per CTA while those CTAs fit two per SM at once: a small ensemble's
   // chain per chunk is shorter by half the MMAs and the slicing.  121 coefficients, M = 42,
-  // us with 64 / 32: 1 member 90 / 62, 16 members 105 / 72 (FP64 FMAs 82 and 86), 48
-  // members 105 / 72, 64 members 106 / 99, 128 members 150 / 104, 256 members 155 / 194;
+  // us with 64 / 32: 1 member 90 / 59, 16 members 105 / 71 (FP64 FMAs 82 and 86), 48
+  // members 105 / 72, 64 members 106 / 98, 128 members 150 / 102, 256 members 148 / 194;
   // 36 coefficients, 256 members 141 / 98.
   const long long small = (long long)EM_CL * ((ncoef + 31) / 32) * ((B + PR_MEMB - 1) / PR_MEMB);
   auto by_coef = [&](auto vk) {

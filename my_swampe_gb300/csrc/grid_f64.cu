@@ -7,7 +7,7 @@
 // 24,000 were the 12 transforms.  A transform of truncated Fourier rows is a
 // product with a static cosine and sine matrix of M + 1 by I / 2; on slices it
 // costs no FP64 instruction, and the physics' 4,000 remain.  M = 42, step / adjoint:
-// 256 members 806 / 1174 -> 394 / 638 us, one member 39 / 55 -> 14 / 18 us.  FP64
+// 256 members 806 / 1174 -> 371 / 622 us, one member 39 / 55 -> 14 / 18 us.  FP64
 // pipe, tensor cores and integer issue each account for about a third of that; the
 // phases between barriers overlap only across the two CTAs of an SM (128 registers).
 //
@@ -597,9 +597,9 @@ __global__ void __launch_bounds__(256, 2) k_grid_out_f64(const __grid_constant__
 // (23 / 23), 6 members 25 / 25 / 25 (35 / 31), 8 members 29 / 24 / 25 (41 / 32), 12
 // members 39 / 35 / 37 (55 / 47), 14 members 39 / 35 / 37 (57 / 47), 16 members 47 / 41 /
 // 37 (68 / 53), 20 members 57 / 51 / 54 (84 / 70), 24 members 66 / 55 / 54 (97 / 76), 48
-// members 120 / 97 / 89 (181 / 137), 256 members 596 / 438 / 379 (934 / 648); M = 63 with
+// members 120 / 97 / 89 (181 / 137), 256 members 596 / 438 / 371 (934 / 622); M = 63 with
 // 1 / 2: 2 members 23 / 23 (33 / 32), 5 members 39 / 35 (55 / 47), 32 members 181 / 150
-// (267 / 209).
+// (267 / 209).  (The forms not taken: before the row sums of I/2 were reduced together.)
 enum Kind { STEP, ADJ, OUT };
 template <int M_, Kind K>
 constexpr int max_rows() { return K == OUT ? 1 : K == ADJ ? (M_ == 106 ? 1 : 2) : M_ == 42 ? 4 : M_ == 63 ? 2 : 1; }
