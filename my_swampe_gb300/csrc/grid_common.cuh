@@ -150,7 +150,7 @@ struct StepDiag {
       unsigned long long m = s.spin[0];
       for (int w = 1; w < 8; ++w) m = min(m, s.spin[w]);
       const double v = __longlong_as_double((long long)m);
-      if (v < 1e300) atomic_min_d(&dn[D_SPIN * B + b], sqrt(v));
+      if (m < 0x7ff0000000000000ull) atomic_min_d(&dn[D_SPIN * B + b], sqrt(v));  // the least square is finite
     } else if (q == 2 && dc) {
       K m = s.lo[0];
       for (int w = 1; w < 8; ++w) m = min(m, s.lo[w]);
